@@ -34,6 +34,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "conv_tc.h"
@@ -76,11 +77,6 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t &r0, uint32_t 
                                           uint32_t &r2, uint32_t &r3) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-               : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x2_t(uint32_t addr, uint32_t &r0, uint32_t &r1) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
-               : "=r"(r0), "=r"(r1)
                : "r"(addr));
 }
 __device__ __forceinline__ void mma_bf16(float *d, uint32_t a0, uint32_t a1, uint32_t a2,
@@ -189,90 +185,134 @@ __global__ void __launch_bounds__(CTHREADS, 1)
     }
 }
 
-/* Weight gradient of one tap over one chunk of cells:
+/* Weight gradient of the three taps (dz, dy, -1..1) over one chunk of cells:
  * part[chunk][tap][ci][co] = sum_{v in chunk} X[v + off(tap)][ci] dZ[v][co],
- * and for the centre tap the bias gradient part_b[chunk][co] = sum dZ[v][co].
+ * and for the centre taps the bias gradient part_b[chunk][co] = sum dZ[v][co].
  * GEMM with M = ci, N = co, K = cells: A = X^T and B = dZ come from shared
- * memory through transposing ldmatrix. Each warp owns 16x8 output tiles
- * w, w+8, ... */
-__global__ void __launch_bounds__(CTHREADS)
-    k_wgrad(int n, int cin, int cout, int cps, int ch, const bf16 *__restrict__ X,
-            const bf16 *__restrict__ dZ, float *__restrict__ part, float *__restrict__ part_b) {
+ * memory through transposing ldmatrix, 16 cells per MMA in cell order, so
+ * each sum has one fixed order whatever the block shape.
+ *
+ * A block stages 64 cells of dZ and the 66 cells of X around them once for
+ * its three taps: tap dx reads the staged rows one slot apart, and a lane
+ * whose neighbour lies across a line's end reads the zero row instead. Warp w
+ * holds the 16 x COUT tile of tap w % 3 and 16-channel group w / 3; the warps
+ * after them sum the bias. The copies run two steps ahead (cp.async, three
+ * stages). One block per tap that staged synchronously, with the tiles dealt
+ * to eight warps (two of which had work in the 16 x 16 layers), was bound by
+ * the staging latency: the 14 layers of 16 systems of 32^3 cells took 7.33 ms
+ * of a training step's 9.12 ms; with this the step takes 2.53 ms. */
+__device__ __forceinline__ void wg_copy(uint32_t dst, const void *src, bool ok) {
+  const int bytes = ok ? 16 : 0; /* 0: the 16 bytes are zero-filled */
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes)
+               : "memory");
+}
+
+constexpr int WG_ROWS = WG_SUB + 2, WG_STAGES = 3;
+
+template <int CIN, int COUT> struct WgShape {
+  static constexpr int MWARPS = 3 * (CIN / 16), BWARPS = (COUT + 31) / 32;
+  static constexpr int THREADS = 32 * (MWARPS + BWARPS);
+  static constexpr int XS = CIN + 8, ZS = COUT + 8; /* padded rows: conflict-free ldmatrix */
+  static constexpr int STAGE = (WG_ROWS * XS + WG_SUB * ZS) * (int)sizeof(bf16);
+  static constexpr int SMEM = 16 + WG_STAGES * (STAGE + WG_SUB);
+};
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(WgShape<CIN, COUT>::THREADS)
+    k_wgrad(int n, int cps, int ch, const bf16 *__restrict__ X, const bf16 *__restrict__ dZ,
+            float *__restrict__ part, float *__restrict__ part_b) {
+  typedef WgShape<CIN, COUT> S;
+  constexpr int NT = COUT / 8;
   extern __shared__ __align__(16) unsigned char smraw[];
-  const int xs = cin + 8, zs = cout + 8;
-  bf16 *sx = reinterpret_cast<bf16 *>(smraw);
-  bf16 *sz = sx + WG_SUB * xs;
-  const int tap = blockIdx.y;
-  const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-  const size_t n3 = (size_t)n * n * n;
+  unsigned char *flags = smraw + 16 + WG_STAGES * S::STAGE; /* [stage][cell]: bit dx+1 = tap dx reads a cell */
+  const uint32_t zero = smem_u32(smraw), stage0 = zero + 16;
+  const int dz = (int)blockIdx.y / 3 - 1, dy = (int)blockIdx.y % 3 - 1;
+  const int n3 = n * n * n;
   /* chunk blockIdx.x: sample s, cells [cb, cb + chunk_cells) of that sample */
-  const size_t s = blockIdx.x / cps;
-  const size_t cb = (size_t)(blockIdx.x % cps) * ch;
-  const int chunk_cells = (int)((cb + ch <= n3) ? ch : n3 - cb);
-  const size_t c0 = s * n3 + cb; /* flat cell over the batch */
+  const int s = (int)blockIdx.x / cps, cb = ((int)blockIdx.x % cps) * ch;
+  const int chunk_cells = min(ch, n3 - cb);
+  const bf16 *Xs = X + (size_t)s * n3 * CIN, *Zs = dZ + ((size_t)s * n3 + cb) * COUT;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int mt_n = cin / 16, nt_n = cout / 8, tiles = mt_n * nt_n;
-  constexpr int MAXT = 7; /* 112/16 x 64/8 = 56 tiles over 8 warps */
-  float acc[MAXT][4];
+  if (threadIdx.x < 4) reinterpret_cast<uint32_t *>(smraw)[threadIdx.x] = 0u;
+  const int subs = (chunk_cells + WG_SUB - 1) / WG_SUB;
+
+  auto fill = [&](int it) {
+    if (it < subs) {
+      const int st = it % WG_STAGES, sub = it * WG_SUB;
+      const uint32_t sx = stage0 + st * S::STAGE, sz = sx + WG_ROWS * S::XS * 2;
+      for (int idx = threadIdx.x; idx < WG_ROWS * (CIN / 8); idx += S::THREADS) {
+        const int slot = idx / (CIN / 8), q = idx % (CIN / 8);
+        const int v = cb + sub + slot - 1; /* the cell whose (dz, dy) neighbour the slot holds */
+        const unsigned row = (unsigned)v / (unsigned)n;
+        const int i = (int)(row / (unsigned)n) + dz, j = (int)(row % (unsigned)n) + dy;
+        const bool ok = v >= 0 && v < n3 && i >= 0 && i < n && j >= 0 && j < n;
+        const int src = ok ? v + (dz * n + dy) * n : 0;
+        wg_copy(sx + (slot * S::XS + q * 8) * 2, Xs + (size_t)src * CIN + q * 8, ok);
+      }
+      for (int idx = threadIdx.x; idx < WG_SUB * (COUT / 8); idx += S::THREADS) {
+        const int r = idx / (COUT / 8), q = idx % (COUT / 8);
+        const bool ok = sub + r < chunk_cells;
+        wg_copy(sz + (r * S::ZS + q * 8) * 2, Zs + (size_t)(ok ? sub + r : 0) * COUT + q * 8, ok);
+      }
+      if (threadIdx.x < WG_SUB) {
+        const int r = threadIdx.x, k = (cb + sub + r) % n;
+        const int f = (k > 0 ? 1 : 0) | 2 | (k < n - 1 ? 4 : 0);
+        flags[st * WG_SUB + r] = (unsigned char)(sub + r < chunk_cells ? f : 0);
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+
+  float acc[NT][4];
 #pragma unroll
-  for (int q = 0; q < MAXT; q++) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.0f;
+  for (int q = 0; q < NT; q++) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.0f;
   float bsum = 0.0f;
-  const bool centre = tap == 13;
-  for (int sub = 0; sub < chunk_cells; sub += WG_SUB) {
-    __syncthreads();
-    /* stage X at the shifted cells and dZ at the cells */
-    for (int idx = threadIdx.x; idx < WG_SUB * (cin / 8); idx += CTHREADS) {
-      const int r = idx / (cin / 8), q = idx % (cin / 8);
-      uint4 val = make_uint4(0, 0, 0, 0);
-      if (sub + r < chunk_cells) {
-        const size_t v = (c0 + sub + r) - s * n3;
-        const int i = (int)(v / ((size_t)n * n)) + dz, j = (int)((v / n) % n) + dy,
-                  k = (int)(v % n) + dx;
-        if (i >= 0 && i < n && j >= 0 && j < n && k >= 0 && k < n)
-          val = *reinterpret_cast<const uint4 *>(
-              X + (s * n3 + ((size_t)i * n + j) * n + k) * cin + q * 8);
-      }
-      *reinterpret_cast<uint4 *>(sx + r * xs + q * 8) = val;
-    }
-    for (int idx = threadIdx.x; idx < WG_SUB * (cout / 8); idx += CTHREADS) {
-      const int r = idx / (cout / 8), q = idx % (cout / 8);
-      uint4 val = make_uint4(0, 0, 0, 0);
-      if (sub + r < chunk_cells)
-        val = *reinterpret_cast<const uint4 *>(dZ + (c0 + sub + r) * cout + q * 8);
-      *reinterpret_cast<uint4 *>(sz + r * zs + q * 8) = val;
-    }
-    __syncthreads();
-    if (centre && threadIdx.x < cout)
-      for (int r = 0; r < WG_SUB; r++) bsum += __bfloat162float(sz[r * zs + threadIdx.x]);
-    for (int kk = 0; kk < WG_SUB; kk += 16) {
+  const bool mma_warp = warp < S::MWARPS;
+  const int dx = warp % 3, mi = warp / 3;              /* tap dx - 1, channels 16 mi.. */
+  const int bc = (warp - S::MWARPS) * 32 + lane;       /* bias warps: output channel */
+  const bool bias = !mma_warp && blockIdx.y == 4 && bc < COUT;
+  const int vr = (lane & 7) + (lane >> 4) * 8, cio = mi * 16 + ((lane >> 3) & 1) * 8;
+  const int vb = (lane & 7) + ((lane >> 3) & 1) * 8, nb = (lane >> 4) * 8;
 #pragma unroll
-      for (int q = 0; q < MAXT; q++) {
-        const int tile = warp + q * 8;
-        if (tile >= tiles) break;
-        const int mi = tile / nt_n, ni = tile % nt_n;
-        uint32_t a0, a1, a2, a3, b0, b1;
-        const int vr = (lane & 7) + (lane >> 4) * 8, cio = ((lane >> 3) & 1) * 8;
-        ldsm_x4_t(smem_u32(sx + (kk + vr) * xs + mi * 16 + cio), a0, a1, a2, a3);
-        const int vb = (lane & 7) + ((lane >> 3) & 1) * 8;
-        ldsm_x2_t(smem_u32(sz + (kk + vb) * zs + ni * 8), b0, b1);
-        mma_bf16(acc[q], a0, a1, a2, a3, b0, b1);
+  for (int it = 0; it < WG_STAGES - 1; it++) fill(it);
+  for (int it = 0; it < subs; it++) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(WG_STAGES - 2) : "memory");
+    __syncthreads(); /* stage it has landed; stage it - 1 has been read */
+    fill(it + WG_STAGES - 1);
+    const int st = it % WG_STAGES;
+    const uint32_t sx = stage0 + st * S::STAGE, sz = sx + WG_ROWS * S::XS * 2;
+    if (mma_warp) {
+#pragma unroll
+      for (int kk = 0; kk < WG_SUB; kk += 16) {
+        uint32_t b[NT][2], a0, a1, a2, a3;
+#pragma unroll
+        for (int q = 0; q < NT; q += 2)
+          ldsm_x4_t(sz + ((kk + vb) * S::ZS + q * 8 + nb) * 2, b[q][0], b[q][1], b[q + 1][0],
+                    b[q + 1][1]);
+        const int r = kk + vr;
+        const bool in = (flags[st * WG_SUB + r] >> dx) & 1;
+        ldsm_x4_t(in ? sx + ((r + dx) * S::XS + cio) * 2 : zero, a0, a1, a2, a3);
+#pragma unroll
+        for (int q = 0; q < NT; q++) mma_bf16(acc[q], a0, a1, a2, a3, b[q][0], b[q][1]);
       }
+    } else if (bias) {
+      const bf16 *z = reinterpret_cast<const bf16 *>(smraw + 16 + st * S::STAGE) + WG_ROWS * S::XS;
+#pragma unroll 16
+      for (int r = 0; r < WG_SUB; r++) bsum += __bfloat162float(z[r * S::ZS + bc]);
     }
   }
-  const int g = lane >> 2, t = lane & 3;
-  float *dst = part + ((size_t)blockIdx.x * 27 + tap) * cin * cout;
+  if (mma_warp) {
+    const int g = lane >> 2, t = lane & 3, ci = mi * 16 + g;
+    float *dst = part + ((size_t)blockIdx.x * 27 + blockIdx.y * 3 + dx) * CIN * COUT;
 #pragma unroll
-  for (int q = 0; q < MAXT; q++) {
-    const int tile = warp + q * 8;
-    if (tile >= tiles) break;
-    const int mi = tile / nt_n, ni = tile % nt_n;
-    const int ci = mi * 16 + g, co = ni * 8 + 2 * t;
-    dst[ci * cout + co] = acc[q][0];
-    dst[ci * cout + co + 1] = acc[q][1];
-    dst[(ci + 8) * cout + co] = acc[q][2];
-    dst[(ci + 8) * cout + co + 1] = acc[q][3];
+    for (int q = 0; q < NT; q++) {
+      const int co = q * 8 + 2 * t;
+      *reinterpret_cast<float2 *>(dst + ci * COUT + co) = make_float2(acc[q][0], acc[q][1]);
+      *reinterpret_cast<float2 *>(dst + (ci + 8) * COUT + co) = make_float2(acc[q][2], acc[q][3]);
+    }
+  } else if (bias) {
+    part_b[(size_t)blockIdx.x * COUT + bc] = bsum;
   }
-  if (centre && threadIdx.x < cout) part_b[(size_t)blockIdx.x * cout + threadIdx.x] = bsum;
 }
 
 /* grad W[tap][ci][co] = sum over chunks in order; grad b likewise */
@@ -537,12 +577,18 @@ __global__ void k_loss_head_bwd(size_t n3, int batch, const uint8_t *__restrict_
   if (threadIdx.x < 18) part[(size_t)blockIdx.x * 18 + threadIdx.x] = sh[0][threadIdx.x];
 }
 
+/* sums of the 18 columns of part (loss, head weights, head bias): one warp a
+ * column, its lanes 32 rows apart, then a fixed tree. One thread a column
+ * waited for each row's load in turn (172 us for 2,048 rows). */
 __global__ void k_head_reduce(int nblocks, const double *__restrict__ part, float *__restrict__ gh,
                               double *__restrict__ loss) {
-  const int c = threadIdx.x;
+  const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (c >= 18) return;
   double s = 0.0;
-  for (int b = 0; b < nblocks; b++) s += part[(size_t)b * 18 + c];
+#pragma unroll 8
+  for (int b = lane; b < nblocks; b += 32) s += part[(size_t)b * 18 + c];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane != 0) return;
   if (c == 0) *loss = s;
   else gh[c - 1] = (float)s;
 }
@@ -837,8 +883,23 @@ template <class T> cudaError_t ualloc(T *&p, size_t n) {
 }
 
 size_t conv_smem(int cin) { return (size_t)HV * (cin + 8) * sizeof(bf16); }
-size_t wgrad_smem(int cin, int cout) {
-  return (size_t)WG_SUB * ((cin + 8) + (cout + 8)) * sizeof(bf16);
+
+/* k_wgrad for the channel counts of one layer: f(kernel, threads, shared bytes) */
+template <class F> bool with_wgrad(int cin, int cout, F f) {
+  bool hit = false;
+  auto one = [&](auto ci, auto co) {
+    constexpr int CI = decltype(ci)::value, CO = decltype(co)::value;
+    if (cin != CI || cout != CO) return;
+    typedef WgShape<CI, CO> S;
+    f(&k_wgrad<CI, CO>, S::THREADS, S::SMEM);
+    hit = true;
+  };
+  using std::integral_constant;
+#define WG_PAIR(a, b) one(integral_constant<int, a>{}, integral_constant<int, b>{})
+  WG_PAIR(16, 16); WG_PAIR(16, 32); WG_PAIR(32, 32); WG_PAIR(32, 48); WG_PAIR(48, 48);
+  WG_PAIR(48, 64); WG_PAIR(64, 64); WG_PAIR(112, 48); WG_PAIR(80, 32); WG_PAIR(48, 16);
+#undef WG_PAIR
+  return hit;
 }
 
 int unet_init_device() {
@@ -853,6 +914,15 @@ int unet_init_device() {
       cudaFuncSetAttribute(k_conv3<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) ||
       conv_tc_init_device() != 0)
     return -1;
+  for (int l = 0; l < NCONV; l++) {
+    bool ok = true;
+    if (!with_wgrad(kConv[l].cin, kConv[l].cout, [&](auto kern, int, int smem) {
+          ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
+               cudaSuccess;
+        }) ||
+        !ok)
+      return -1;
+  }
   done[dev] = true;
   return 0;
 }
@@ -1032,8 +1102,10 @@ int wgrad(FlipUNet *u, int l, int n, int batch, const bf16 *X, const bf16 *dZ) {
   const int cps = (int)((V + 4095) / 4096);
   const int ch = (int)((V + cps - 1) / cps);
   const size_t chunks = (size_t)cps * batch;
-  k_wgrad<<<dim3((unsigned)chunks, 27), CTHREADS, wgrad_smem(cin, cout), u->stream>>>(
-      n, cin, cout, cps, ch, X, dZ, u->part, u->part_b);
+  with_wgrad(cin, cout, [&](auto kern, int threads, int smem) {
+    kern<<<dim3((unsigned)chunks, 9), threads, smem, u->stream>>>(n, cps, ch, X, dZ, u->part,
+                                                                  u->part_b);
+  });
   const int wc = 27 * cin * cout;
   k_wgrad_reduce<<<(wc + cout + EBLK - 1) / EBLK, EBLK, 0, u->stream>>>(
       (int)chunks, wc, cout, u->part, u->part_b, u->G + u->woff[l], u->G + u->boff[l]);
@@ -1070,7 +1142,7 @@ int backward(FlipUNet *u, int n, int batch, const uint8_t *A, const float *x, co
   const unsigned hb = eg(V0 * B);
   k_loss_head_bwd<<<hb, EBLK, 0, u->stream>>>(V0, B, A, x, x0, u->scale, inv, u->O, u->D0,
                                               u->P + u->hoff, u->G1, u->hpart);
-  k_head_reduce<<<1, 32, 0, u->stream>>>((int)hb, u->hpart, u->G + u->hoff, u->loss);
+  k_head_reduce<<<1, 18 * 32, 0, u->stream>>>((int)hb, u->hpart, u->G + u->hoff, u->loss);
   UCK(cudaGetLastError());
   /* decoder, level 0 */
   if ((r = conv_bwd(u, 13, n, B, u->G1, u->B0, u->D0, u->G3))) return r;
