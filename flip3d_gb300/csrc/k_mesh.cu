@@ -86,6 +86,7 @@ __constant__ signed char c_ring[3][4][4] = {
 struct FieldConst {
   int n, mg;
   float fn, wall_r, wall_thr2;
+  float near2; /* (0.3 cells)^2 */
   double h, phi0, wall_val;
   const uint32_t *slab; /* [axis][lo/hi][n] order-preserving keys */
 };
@@ -99,6 +100,7 @@ FieldConst field_const(const FlipGpu *h) {
   f.slab = nullptr;
   f.wall_r = c.density / (float)c.n;           /* density/gn, FLOAT */
   f.wall_thr2 = f.wall_r * f.wall_r * 1.000244140625f;
+  f.near2 = 0.09f / (f.fn * f.fn);
   f.h = 1.0 / (double)(f.mg - 1);
   f.phi0 = 8.0 * (double)c.density / c.n;
   f.wall_val = 4.5 * (double)c.density / c.n;
@@ -115,31 +117,56 @@ __device__ __forceinline__ float key_float(uint32_t k) {
 }
 
 /* per axis a and slab s (cells with that coordinate): the smallest and
- * largest current coordinate of the particles listed there */
-__global__ void k_slab_bounds(int n, const uint32_t *__restrict__ cs,
-                              const float4 *__restrict__ spos, uint32_t *__restrict__ slab) {
+ * largest current coordinate of the particles listed there. Minima and
+ * maxima do not depend on the order. Each block keeps all 6 n bounds in
+ * shared memory over its share of the cells and writes the ones that improve
+ * the global bounds at its end; a bound is read before its atomic, which most
+ * cells then skip. With six global atomics a cell the n^3 cells queued on 6 n
+ * words (264 us at n = 100). */
+constexpr int SLAB_GRID = 152 * 2;
+
+__global__ void __launch_bounds__(MBLK) k_slab_bounds(int n, const uint32_t *__restrict__ cs,
+                                                      const float4 *__restrict__ spos,
+                                                      uint32_t *__restrict__ slab) {
+  extern __shared__ uint32_t sb[]; /* [axis][lo/hi][n] as slab */
+  for (int i = threadIdx.x; i < 6 * n; i += MBLK) sb[i] = (i / n) & 1 ? 0u : 0xffffffffu;
+  __syncthreads();
   const size_t nc = (size_t)n * n * n;
-  const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nc) return;
-  const uint32_t s = cs[c], e = cs[c + 1];
-  if (s == e) return;
-  float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-  bool any[3] = {false, false, false};
-  for (uint32_t q = s; q < e; q++) {
-    const float4 Q = spos[q];
-    const float v[3] = {Q.x, Q.y, Q.z};
-    for (int a = 0; a < 3; a++)
-      if (v[a] == v[a]) {
-        lo[a] = fminf(lo[a], v[a]);
-        hi[a] = fmaxf(hi[a], v[a]);
-        any[a] = true;
-      }
+  for (size_t c = (size_t)blockIdx.x * MBLK + threadIdx.x; c < nc; c += (size_t)gridDim.x * MBLK) {
+    const uint32_t s = cs[c], e = cs[c + 1];
+    if (s == e) continue;
+    float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+    bool any[3] = {false, false, false};
+    for (uint32_t q = s; q < e; q++) {
+      const float4 Q = spos[q];
+      const float v[3] = {Q.x, Q.y, Q.z};
+#pragma unroll
+      for (int a = 0; a < 3; a++)
+        if (v[a] == v[a]) {
+          lo[a] = fminf(lo[a], v[a]);
+          hi[a] = fmaxf(hi[a], v[a]);
+          any[a] = true;
+        }
+    }
+    int cell[3];
+    decode_index(c, n, n, cell[0], cell[1], cell[2]);
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      if (!any[a]) continue;
+      uint32_t *l = sb + (2 * a) * n + cell[a], *u = sb + (2 * a + 1) * n + cell[a];
+      const uint32_t kl = ord_key(lo[a]), kh = ord_key(hi[a]);
+      if (kl < *(volatile uint32_t *)l) atomicMin(l, kl);
+      if (kh > *(volatile uint32_t *)u) atomicMax(u, kh);
+    }
   }
-  const int cell[3] = {(int)(c / ((size_t)n * n)), (int)((c / n) % n), (int)(c % n)};
-  for (int a = 0; a < 3; a++) {
-    if (!any[a]) continue;
-    atomicMin(slab + (2 * a) * n + cell[a], ord_key(lo[a]));
-    atomicMax(slab + (2 * a + 1) * n + cell[a], ord_key(hi[a]));
+  __syncthreads();
+  for (int i = threadIdx.x; i < 6 * n; i += MBLK) {
+    const uint32_t v = sb[i], g = __ldcg(slab + i);
+    if ((i / n) & 1) {
+      if (v > g) atomicMax(slab + i, v);
+    } else if (v < g) {
+      atomicMin(slab + i, v);
+    }
   }
 }
 
@@ -154,7 +181,12 @@ __device__ __forceinline__ float axis_gap(const FieldConst &f, int a, int s, flo
 /* implicit_func (src/implicit.cpp:14-38) at p. Fluid candidates whose
  * squared distance exceeds the current minimum by a margin far above the
  * rounding of hypot (2^-12 relative) cannot lower it; only the others get
- * the reference's hypotf(hypotf()) distance. */
+ * the reference's hypotf(hypotf()) distance. The value is a minimum (or the
+ * wall value, when any wall particle is near), so the order of the cells
+ * cannot change it: pass 0 takes the cells whose bound lies within 0.3 cells
+ * of p, usually the eight around a node, which leaves a minimum that rules
+ * nearly all the others out in pass 1. A row of five cells is skipped by its
+ * two bounds alone, or when its run of slots is empty. */
 __device__ double implicit_value(const FieldConst &f, const uint32_t *__restrict__ cs,
                                  const float4 *__restrict__ spos, float px, float py,
                                  float pz) {
@@ -164,28 +196,28 @@ __device__ double implicit_value(const FieldConst &f, const uint32_t *__restrict
   const int i0 = max(ci - 2, 0), i1 = min(ci + 2, n - 1);
   const int j0 = max(cj - 2, 0), j1 = min(cj + 2, n - 1);
   const int k0 = max(ck - 2, 0), k1 = min(ck + 2, n - 1);
-  float gx[5], gy[5], gz[5];
+  float gz[5];
 #pragma unroll
   for (int a = 0; a < 5; a++) {
-    gx[a] = (i0 + a <= i1) ? axis_gap(f, 0, i0 + a, px) : FLT_MAX;
-    gy[a] = (j0 + a <= j1) ? axis_gap(f, 1, j0 + a, py) : FLT_MAX;
     gz[a] = (k0 + a <= k1) ? axis_gap(f, 2, k0 + a, pz) : FLT_MAX;
-    gx[a] *= gx[a];
-    gy[a] *= gy[a];
     gz[a] *= gz[a];
   }
   double phi = f.phi0;
   float best2 = (float)(phi * phi) * 1.000244140625f;
-  /* pass 0: cells at zero distance; pass 1: the rest, nearest bound first
-   * is not needed for exactness, only the skip test */
+  const float near2 = f.near2;
   for (int pass = 0; pass < 2; pass++) {
-    for (int a = 0; a <= i1 - i0; a++)
-      for (int b = 0; b <= j1 - j0; b++) {
-        const float gab = gx[a] + gy[b];
-        const size_t row = ((size_t)(i0 + a) * n + (j0 + b)) * n;
-        for (int c = 0; c <= k1 - k0; c++) {
+    for (int i = i0; i <= i1; i++) {
+      const float gx = axis_gap(f, 0, i, px), gx2 = gx * gx;
+      if ((pass == 0 && !(gx2 <= near2)) || gx2 * 0.99998f >= fmaxf(best2, f.wall_thr2)) continue;
+      for (int j = j0; j <= j1; j++) {
+        const float gy = axis_gap(f, 1, j, py), gab = gx2 + gy * gy;
+        if ((pass == 0 && !(gab <= near2)) || gab * 0.99998f >= fmaxf(best2, f.wall_thr2)) continue;
+        const size_t row = ((size_t)i * n + j) * n;
+        if (__ldg(cs + row + k0) == __ldg(cs + row + k1 + 1)) continue;
+#pragma unroll
+        for (int c = 0; c < 5; c++) {
           const float lb2 = gab + gz[c];
-          if ((lb2 == 0.0f) != (pass == 0)) continue;
+          if (k0 + c > k1 || (lb2 <= near2) != (pass == 0)) continue;
           if (lb2 * 0.99998f >= fmaxf(best2, f.wall_thr2)) continue;
           const uint32_t s = __ldg(cs + row + k0 + c), e = __ldg(cs + row + k0 + c + 1);
           for (uint32_t q = s; q < e; q++) {
@@ -204,24 +236,30 @@ __device__ double implicit_value(const FieldConst &f, const uint32_t *__restrict
           }
         }
       }
+    }
   }
   return phi - (double)f.wall_r;
 }
 
 /* density field (src/mesher.cpp:142-153): node (x,y,z) at x*h, boundary
- * nodes raised to at least 0.01, stored negated */
+ * nodes raised to at least 0.01, stored negated. Consecutive threads take
+ * consecutive z: their cells are neighbours in the lists (k fastest), so a
+ * warp's loads share lines; the field's own order (x fastest) put a warp's
+ * cells n^2 apart and cost n = 100 0.98 ms. The 4-byte stores are scattered
+ * instead and merge in L2. */
 __global__ void k_mesh_field(FieldConst f, const uint32_t *__restrict__ cs,
                              const float4 *__restrict__ spos, float *__restrict__ phi) {
   const size_t nn = (size_t)f.mg * f.mg * f.mg;
-  const size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nn) return;
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nn) return;
   const int mg = f.mg;
-  const int x = (int)(v % mg), y = (int)((v / mg) % mg), z = (int)(v / ((size_t)mg * mg));
+  int x, y, z;
+  decode_index(t, mg, mg, x, y, z);
   const float px = (float)(x * f.h), py = (float)(y * f.h), pz = (float)(z * f.h);
   double value = implicit_value(f, cs, spos, px, py, pz);
   if (x == 0 || x == mg - 1 || y == 0 || y == mg - 1 || z == 0 || z == mg - 1)
     value = fmax(value, 0.01);
-  phi[v] = (float)(-value);
+  phi[((size_t)z * mg + y) * mg + x] = (float)(-value);
 }
 
 __global__ void k_implicit_points(FieldConst f, int m, const float *__restrict__ pts,
@@ -454,9 +492,11 @@ __global__ void k_mesh_faces(size_t nt, const int32_t *__restrict__ T,
   F[3 * f + 2] = T[3 * t + 2];
 }
 
+/* isnormal() from the exponent field: FP64 compares run at 1/64 of the rate
+ * (two smoothing passes at n = 100: 131 us with them) */
 __device__ __forceinline__ bool is_normal(double x) {
-  const double a = fabs(x);
-  return a >= DBL_MIN && a <= DBL_MAX;
+  const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+  return e != 0u && e != 0x7ffu;
 }
 
 /* one pass of smoothMesh (src/mesher.cpp:21-71): unit weights, a vertex or
@@ -548,7 +588,7 @@ cudaError_t field_prepare(FlipGpu *h, FieldConst &f) {
   MeshBufs *m = h->mesh;
   const int n = h->n;
   if (!m->slab) MCK(dalloc_n(m->slab, 6 * (size_t)n));
-  MCK(launch_payload(h, 0));
+  MCK(launch_payload(h, 0, 0)); /* the field reads positions alone */
   for (int a = 0; a < 3; a++) {
     MCK(cudaMemsetAsync(m->slab + (2 * a) * (size_t)n, 0xff, (size_t)n * sizeof(uint32_t),
                         h->stream));
@@ -556,7 +596,9 @@ cudaError_t field_prepare(FlipGpu *h, FieldConst &f) {
                         h->stream));
   }
   const size_t nc = (size_t)n * n * n;
-  k_slab_bounds<<<grid_for(nc, MBLK), MBLK, 0, h->stream>>>(n, h->cell_start, h->spos, m->slab);
+  const unsigned g = grid_for(nc, MBLK);
+  k_slab_bounds<<<g < SLAB_GRID ? g : SLAB_GRID, MBLK, 6 * (size_t)n * sizeof(uint32_t),
+                  h->stream>>>(n, h->cell_start, h->spos, m->slab);
   FG_LAUNCHED(h, 1);
   MCK(cudaGetLastError());
   f = field_const(h);
