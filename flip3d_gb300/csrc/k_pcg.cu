@@ -1376,11 +1376,6 @@ template <int BLOCK> __global__ void __launch_bounds__(BLOCK, 1) k_cg_cg1(CgArgs
 constexpr int MGU = 4;            /* cells per thread and round, loads first */
 constexpr unsigned MG_BLOCK_CELLS = 4096; /* levels this small run in block 0 */
 
-template <bool GLOBAL> __device__ __forceinline__ float mg_ld(const float *p) {
-  if (GLOBAL) return __ldcg(p);
-  return *p;
-}
-
 __device__ __forceinline__ void mg_decode(unsigned c, unsigned m, int &i, int &j, int &k) {
   const unsigned row = c / m;
   k = (int)(c - row * m);
@@ -1400,174 +1395,178 @@ __device__ __forceinline__ void mg_decode(unsigned c, unsigned m, int lg, int &i
   }
 }
 
-template <bool GLOBAL>
+/* The middle levels' passes: a thread's MGU cells read their flags first
+ * (constant during the solve, so mostly in L1) and request nothing for the
+ * cells that have no work, which outnumber the liquid ones. */
 __device__ __forceinline__ float mg_nbsum(const float *x, int m, int i, int j, int k, unsigned c) {
   const unsigned mm = (unsigned)m * m;
   float s = 0.0f;
-  if (i > 0) s += mg_ld<GLOBAL>(x + c - mm);
-  if (i + 1 < m) s += mg_ld<GLOBAL>(x + c + mm);
-  if (j > 0) s += mg_ld<GLOBAL>(x + c - m);
-  if (j + 1 < m) s += mg_ld<GLOBAL>(x + c + m);
-  if (k > 0) s += mg_ld<GLOBAL>(x + c - 1);
-  if (k + 1 < m) s += mg_ld<GLOBAL>(x + c + 1);
+  if (i > 0) s += __ldcg(x + c - mm);
+  if (i + 1 < m) s += __ldcg(x + c + mm);
+  if (j > 0) s += __ldcg(x + c - m);
+  if (j + 1 < m) s += __ldcg(x + c + m);
+  if (k > 0) s += __ldcg(x + c - 1);
+  if (k + 1 < m) s += __ldcg(x + c + 1);
   return s;
 }
 
 /* red-black half sweep: liquid cells of `color` take
- * x = (b / hs + sum of the neighbours' x) / diag */
-template <bool GLOBAL>
-__device__ void mg_gs(const MgLevel &L, int color, unsigned start, unsigned stride) {
-  const unsigned m = (unsigned)L.m, tot = m * m * m;
-  if (L.lgm >= 1) {
-    /* m = 2^lg: enumerate the cells of the colour only (k = 2 kk + parity) */
-    const int lg = L.lgm;
-    const unsigned half = tot >> 1, hm = m >> 1;
-    for (unsigned h0 = start; h0 < half; h0 += stride * MGU) {
-      float nbs[MGU], bv[MGU], dv[MGU];
-      unsigned cc[MGU];
-      bool upd[MGU];
-#pragma unroll
-      for (int u = 0; u < MGU; u++) {
-        const unsigned h = h0 + (unsigned)u * stride;
-        upd[u] = false;
-        nbs[u] = bv[u] = 0.0f;
-        dv[u] = 1.0f;
-        cc[u] = 0;
-        if (h < half) {
-          const unsigned row = h >> (lg - 1);
-          const int j = (int)(row & (m - 1)), i = (int)(row >> lg);
-          const int k = 2 * (int)(h & (hm - 1)) + ((i + j + color) & 1);
-          const unsigned c = (row << lg) + (unsigned)k;
-          cc[u] = c;
-          upd[u] = L.flags[c] == CELL_FLUID;
-          bv[u] = mg_ld<GLOBAL>(L.b + c);
-          dv[u] = L.diag[c];
-          nbs[u] = mg_nbsum<GLOBAL>(L.x, (int)m, i, j, k, c);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < MGU; u++)
-        if (upd[u]) L.x[cc[u]] = __fdividef(bv[u] * L.ihs + nbs[u], dv[u]);
-    }
-    return;
-  }
-  for (unsigned c0 = start; c0 < tot; c0 += stride * MGU) {
-    float nbs[MGU], bv[MGU], dv[MGU];
+ * x = (b / hs + sum of the neighbours' x) / diag. The pairs of cells
+ * (2 kk, 2 kk + 1) of a line are enumerated, each with its cell of the colour. */
+__device__ __noinline__ void mg_gs(const MgLevel L, int color, unsigned start, unsigned stride) {
+  const unsigned m = (unsigned)L.m, hm = (m + 1) >> 1, tot = m * m * hm;
+  for (unsigned h0 = start; h0 < tot; h0 += stride * MGU) {
+    unsigned cc[MGU];
+    int ii[MGU], jj[MGU], kk[MGU];
     bool upd[MGU];
 #pragma unroll
     for (int u = 0; u < MGU; u++) {
-      const unsigned c = c0 + (unsigned)u * stride;
+      const unsigned h = h0 + (unsigned)u * stride;
       upd[u] = false;
-      nbs[u] = bv[u] = 0.0f;
-      dv[u] = 1.0f;
-      if (c < tot) {
-        int i, j, k;
-        mg_decode(c, m, L.lgm, i, j, k);
-        if (((i + j + k) & 1) == color) {
-          upd[u] = L.flags[c] == CELL_FLUID;
-          bv[u] = mg_ld<GLOBAL>(L.b + c);
-          dv[u] = L.diag[c];
-          nbs[u] = mg_nbsum<GLOBAL>(L.x, (int)m, i, j, k, c);
+      if (h < tot) {
+        unsigned row;
+        if (L.lgm >= 1) {
+          row = h >> (L.lgm - 1);
+          jj[u] = (int)(row & (m - 1));
+          ii[u] = (int)(row >> L.lgm);
+        } else {
+          row = h / hm;
+          ii[u] = (int)(row / m);
+          jj[u] = (int)(row - (unsigned)ii[u] * m);
         }
+        kk[u] = 2 * (int)(h - row * hm) + ((ii[u] + jj[u] + color) & 1);
+        cc[u] = row * m + (unsigned)kk[u];
+        upd[u] = kk[u] < (int)m && __ldg(L.flags + cc[u]) == CELL_FLUID;
       }
     }
+    float nbs[MGU], bv[MGU], dv[MGU];
 #pragma unroll
     for (int u = 0; u < MGU; u++)
-      if (upd[u]) L.x[c0 + (unsigned)u * stride] = __fdividef(bv[u] * L.ihs + nbs[u], dv[u]);
-  }
-}
-
-/* res = b - A x on the liquid, 0 elsewhere */
-template <bool GLOBAL>
-__device__ void mg_residual(const MgLevel &L, unsigned start, unsigned stride) {
-  const unsigned m = (unsigned)L.m, tot = m * m * m;
-  for (unsigned c0 = start; c0 < tot; c0 += stride * MGU) {
-    float nbs[MGU], bv[MGU], dv[MGU], xv[MGU];
-    bool fl_[MGU];
-#pragma unroll
-    for (int u = 0; u < MGU; u++) {
-      const unsigned c = c0 + (unsigned)u * stride;
-      fl_[u] = false;
-      nbs[u] = bv[u] = dv[u] = xv[u] = 0.0f;
-      if (c < tot) {
-        int i, j, k;
-        mg_decode(c, m, L.lgm, i, j, k);
-        fl_[u] = L.flags[c] == CELL_FLUID;
-        bv[u] = mg_ld<GLOBAL>(L.b + c);
-        dv[u] = L.diag[c];
-        xv[u] = mg_ld<GLOBAL>(L.x + c);
-        nbs[u] = mg_nbsum<GLOBAL>(L.x, (int)m, i, j, k, c);
+      if (upd[u]) {
+        bv[u] = __ldcg(L.b + cc[u]);
+        dv[u] = __ldg(L.diag + cc[u]);
+        nbs[u] = mg_nbsum(L.x, (int)m, ii[u], jj[u], kk[u], cc[u]);
       }
-    }
 #pragma unroll
-    for (int u = 0; u < MGU; u++) {
-      const unsigned c = c0 + (unsigned)u * stride;
-      if (c < tot) L.res[c] = fl_[u] ? bv[u] - L.hs * (dv[u] * xv[u] - nbs[u]) : 0.0f;
-    }
+    for (int u = 0; u < MGU; u++)
+      if (upd[u]) L.x[cc[u]] = __fdividef(bv[u] * L.ihs + nbs[u], dv[u]);
   }
 }
 
-/* coarse b = mean of the 8 children's residuals; coarse x = its first red
+/* coarse b = mean of the 8 children's residuals, coarse x = its first red
  * half sweep from zero (b / (hs diag) on red liquid cells, 0 elsewhere) */
-template <bool GF, bool GC>
-__device__ void mg_restrict(const MgLevel &F, const MgLevel &Cl, unsigned start, unsigned stride) {
+__device__ __forceinline__ void mg_coarse_start(const MgLevel &Cl, unsigned c, bool red, float sum) {
+  const float bc = sum * 0.125f;
+  Cl.b[c] = bc;
+  Cl.x[c] = red ? __fdividef(bc * Cl.ihs, __ldg(Cl.diag + c)) : 0.0f;
+}
+
+/* from the residual that the level-0 pass stored (n is even) */
+__device__ __noinline__ void mg_restrict(const MgLevel F, const MgLevel Cl, unsigned start,
+                                         unsigned stride) {
   const unsigned mc = (unsigned)Cl.m, totc = mc * mc * mc, mf = (unsigned)F.m;
   for (unsigned c0 = start; c0 < totc; c0 += stride * MGU) {
     float sum[MGU];
-    bool red[MGU], fl_[MGU];
-    float dv[MGU];
+    bool red[MGU];
 #pragma unroll
     for (int u = 0; u < MGU; u++) {
       const unsigned c = c0 + (unsigned)u * stride;
       sum[u] = 0.0f;
-      red[u] = fl_[u] = false;
-      dv[u] = 1.0f;
-      if (c < totc) {
+      red[u] = false;
+      if (c < totc && __ldg(Cl.flags + c) == CELL_FLUID) {
         int I, J, K;
         mg_decode(c, mc, Cl.lgm, I, J, K);
         red[u] = ((I + J + K) & 1) == 0;
-        fl_[u] = Cl.flags[c] == CELL_FLUID;
-        dv[u] = Cl.diag[c];
-        if ((mf & 1u) == 0) { /* the k pair as one aligned float2 */
+        /* the k pair as one aligned float2 */
 #pragma unroll
-          for (int a = 0; a < 2; a++)
+        for (int a = 0; a < 2; a++)
 #pragma unroll
-            for (int b = 0; b < 2; b++) {
-              const unsigned i = 2u * I + a, j = 2u * J + b;
-              const float2 *pp =
-                  reinterpret_cast<const float2 *>(F.res + (i * mf + j) * mf + 2u * K);
-              const float2 v = GF ? __ldcg(pp) : *pp;
-              sum[u] += v.x;
-              sum[u] += v.y;
-            }
-        } else {
-#pragma unroll
-          for (int a = 0; a < 2; a++)
-#pragma unroll
-            for (int b = 0; b < 2; b++)
-#pragma unroll
-              for (int d = 0; d < 2; d++) {
-                const unsigned i = 2u * I + a, j = 2u * J + b, k = 2u * K + d;
-                if (i < mf && j < mf && k < mf)
-                  sum[u] += mg_ld<GF>(F.res + (i * mf + j) * mf + k);
-              }
-        }
+          for (int b = 0; b < 2; b++) {
+            const unsigned i = 2u * I + a, j = 2u * J + b;
+            const float2 v = __ldcg(
+                reinterpret_cast<const float2 *>(F.res + (i * mf + j) * mf + 2u * K));
+            sum[u] += v.x;
+            sum[u] += v.y;
+          }
       }
     }
 #pragma unroll
     for (int u = 0; u < MGU; u++) {
       const unsigned c = c0 + (unsigned)u * stride;
-      if (c >= totc) continue;
-      const float bc = sum[u] * 0.125f;
-      Cl.b[c] = bc;
-      Cl.x[c] = (red[u] && fl_[u]) ? __fdividef(bc * Cl.ihs, dv[u]) : 0.0f;
+      if (c < totc) mg_coarse_start(Cl, c, red[u], sum[u]);
     }
   }
 }
 
+/* residual b - A x and restriction of a middle level in one pass: a thread
+ * per coarse cell computes its 8 children's residuals (two lines of two
+ * cells in i and j, and the cells around them), which saves writing and
+ * rereading them and a grid barrier */
+__device__ __noinline__ void mg_residual_restrict(const MgLevel F, const MgLevel Cl,
+                                                  unsigned start, unsigned stride) {
+  const int mc = Cl.m, m = F.m;
+  const unsigned totc = (unsigned)mc * mc * mc;
+  const unsigned mm = (unsigned)m * m;
+  for (unsigned c = start; c < totc; c += stride) {
+    float sum = 0.0f;
+    bool red = false;
+    if (__ldg(Cl.flags + c) == CELL_FLUID) {
+      int I, J, K;
+      mg_decode(c, (unsigned)mc, Cl.lgm, I, J, K);
+      red = ((I + J + K) & 1) == 0;
+      const int i0 = 2 * I, j0 = 2 * J, k0 = 2 * K;
+      const unsigned base = ((unsigned)i0 * m + j0) * m + k0;
+      /* x of lines i0 - 1 .. i0 + 2, j0 - 1 .. j0 + 2 without the corners:
+       * xv[a][b][d], cell (i0 + a - 1, j0 + b - 1, k0 + d - 1), 0 outside */
+      float xv[4][4][4], bv[2][2][2], dv[2][2][2];
+      bool in[2][2][2];
+#pragma unroll
+      for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+          const bool ai = a == 1 || a == 2, bi = b == 1 || b == 2;
+          if (!ai && !bi) continue;
+          const int i = i0 + a - 1, j = j0 + b - 1;
+          const bool line = i >= 0 && i < m && j >= 0 && j < m;
+          const float *x = F.x + ((long)base + (a - 1) * (long)mm + (b - 1) * m);
+#pragma unroll
+          for (int d = 0; d < 4; d++) {
+            if ((d == 0 || d == 3) && !(ai && bi)) continue;
+            const int k = k0 + d - 1;
+            xv[a][b][d] = line && k >= 0 && k < m ? __ldcg(x + d - 1) : 0.0f;
+          }
+        }
+#pragma unroll
+      for (int a = 0; a < 2; a++)
+#pragma unroll
+        for (int b = 0; b < 2; b++)
+#pragma unroll
+          for (int d = 0; d < 2; d++) {
+            const unsigned f = base + a * mm + b * m + d;
+            const bool ok = i0 + a < m && j0 + b < m && k0 + d < m;
+            in[a][b][d] = ok && __ldg(F.flags + f) == CELL_FLUID;
+            bv[a][b][d] = ok ? __ldcg(F.b + f) : 0.0f;
+            dv[a][b][d] = ok ? __ldg(F.diag + f) : 0.0f;
+          }
+#pragma unroll
+      for (int a = 0; a < 2; a++)
+#pragma unroll
+        for (int b = 0; b < 2; b++)
+#pragma unroll
+          for (int d = 0; d < 2; d++) {
+            const int p = a + 1, q = b + 1, r = d + 1;
+            const float nbs = ((((xv[p - 1][q][r] + xv[p + 1][q][r]) + xv[p][q - 1][r]) +
+                                xv[p][q + 1][r]) + xv[p][q][r - 1]) + xv[p][q][r + 1];
+            sum += in[a][b][d] ? bv[a][b][d] - F.hs * (dv[a][b][d] * xv[p][q][r] - nbs) : 0.0f;
+          }
+    }
+    mg_coarse_start(Cl, c, red, sum);
+  }
+}
+
 /* x += the parent's correction on the liquid */
-template <bool GF, bool GC>
-__device__ void mg_prolong(const MgLevel &F, const MgLevel &Cl, unsigned start, unsigned stride) {
+__device__ __noinline__ void mg_prolong(const MgLevel F, const MgLevel Cl, unsigned start,
+                                        unsigned stride) {
   const unsigned mf = (unsigned)F.m, tot = mf * mf * mf, mc = (unsigned)Cl.m;
   for (unsigned c0 = start; c0 < tot; c0 += stride * MGU) {
     float xv[MGU], ev[MGU];
@@ -1575,100 +1574,235 @@ __device__ void mg_prolong(const MgLevel &F, const MgLevel &Cl, unsigned start, 
 #pragma unroll
     for (int u = 0; u < MGU; u++) {
       const unsigned c = c0 + (unsigned)u * stride;
-      fl_[u] = false;
-      xv[u] = ev[u] = 0.0f;
-      if (c < tot) {
+      fl_[u] = c < tot && __ldg(F.flags + c) == CELL_FLUID;
+    }
+#pragma unroll
+    for (int u = 0; u < MGU; u++)
+      if (fl_[u]) {
+        const unsigned c = c0 + (unsigned)u * stride;
         int i, j, k;
         mg_decode(c, mf, F.lgm, i, j, k);
         const unsigned pc =
             (((unsigned)i >> 1) * mc + ((unsigned)j >> 1)) * mc + ((unsigned)k >> 1);
-        fl_[u] = F.flags[c] == CELL_FLUID;
-        xv[u] = mg_ld<GF>(F.x + c);
-        ev[u] = mg_ld<GC>(Cl.x + pc);
+        xv[u] = __ldcg(F.x + c);
+        ev[u] = __ldcg(Cl.x + pc);
       }
-    }
 #pragma unroll
     for (int u = 0; u < MGU; u++)
       if (fl_[u]) F.x[c0 + (unsigned)u * stride] = xv[u] + ev[u];
   }
 }
 
-/* The levels lb.. in block 0's shared memory: V-cycle from level lb's b and
- * first half sweep (in global memory, from the restriction) to level lb's
- * corrected x (written back to global memory). */
-__device__ void mg_block_levels(const MgArgs &mg, MgLevel *sl) {
-  const unsigned t = threadIdx.x, S = blockDim.x;
-  const int lb = mg.lb, last = mg.nlev - 1;
-  const MgLevel &G = mg.lv[lb];
-  const unsigned m0 = (unsigned)G.m, tot0 = m0 * m0 * m0;
-  for (unsigned c0 = t; c0 < tot0; c0 += S * 8) {
-    float bv[8], xv[8];
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const unsigned c = c0 + (unsigned)u * S;
-      bv[u] = c < tot0 ? __ldcg(G.b + c) : 0.0f;
-      xv[u] = c < tot0 ? __ldcg(G.x + c) : 0.0f;
-    }
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const unsigned c = c0 + (unsigned)u * S;
-      if (c < tot0) {
-        sl[lb].b[c] = bv[u];
-        sl[lb].x[c] = xv[u];
-      }
-    }
-  }
-  __syncthreads();
-  for (int l = lb; l < last; l++) {
-    mg_gs<false>(sl[l], 1, t, S);
-    __syncthreads();
-    for (int sw = 1; sw < mg.nu; sw++) {
-      mg_gs<false>(sl[l], 0, t, S);
-      __syncthreads();
-      mg_gs<false>(sl[l], 1, t, S);
-      __syncthreads();
-    }
-    mg_residual<false>(sl[l], t, S);
-    __syncthreads();
-    mg_restrict<false, false>(sl[l], sl[l + 1], t, S);
-    __syncthreads();
-  }
-  /* coarsest: the restriction did the first red half sweep */
-  mg_gs<false>(sl[last], 1, t, S);
-  __syncthreads();
-  for (int it = 1; it < mg.coarse_sweeps; it++) {
-    mg_gs<false>(sl[last], 0, t, S);
-    __syncthreads();
-    mg_gs<false>(sl[last], 1, t, S);
-    __syncthreads();
-  }
-  for (int it = 0; it < mg.coarse_sweeps; it++) {
-    mg_gs<false>(sl[last], 1, t, S);
-    __syncthreads();
-    mg_gs<false>(sl[last], 0, t, S);
-    __syncthreads();
-  }
-  for (int l = last - 1; l >= lb; l--) {
-    mg_prolong<false, false>(sl[l], sl[l + 1], t, S);
-    __syncthreads();
-    for (int sw = 0; sw < mg.nu; sw++) {
-      mg_gs<false>(sl[l], 1, t, S);
-      __syncthreads();
-      mg_gs<false>(sl[l], 0, t, S);
-      __syncthreads();
-    }
-  }
-  for (unsigned c = t; c < tot0; c += S) G.x[c] = sl[lb].x[c];
+/* One of block 0's levels in shared memory. x and res are padded by a zero
+ * layer, so that neighbours need no tests. The cells are listed by colour
+ * (red, i + j + k even, first; within a colour in cell order): at[] holds a
+ * listed cell's padded index, d[] its diagonal, infinite off the liquid, where
+ * x = (b / hs + neighbours) / d then stays 0, and b[] its right-hand side. */
+struct MgBlockLevel {
+  int m, pm;             /* cells per axis; m + 2 */
+  int nred, ncell;
+  float hs, ihs;
+  float *x, *res, *b, *d;
+  unsigned short *at, *slot; /* slot: cell -> its place in the lists */
+};
+constexpr int MG_BLOCK_LEVELS = 3; /* at most 16, 8 and 4 cells per axis */
+
+/* place of cell (i, j, k) of m^3 in the lists: the red cells before row (i, j)
+ * are counted from the rows that start red, ceil(m / 2) of them in lines of
+ * even i, floor(m / 2) in the others */
+__host__ __device__ inline int mg_list_slot(int m, int i, int j, int k) {
+  const int up = (m + 1) / 2, dn = m / 2;
+  const int z = (i + 1) / 2 * up + i / 2 * dn + (i & 1 ? j / 2 : (j + 1) / 2);
+  const int rows = i * m + j, red = z * up + (rows - z) * dn;
+  const int all = (m * m * m + 1) / 2;
+  return ((i + j + k) & 1) == 0 ? red + k / 2 : all + rows * m - red + k / 2;
 }
 
-/* Shared-memory bytes of block 0's levels (flags, diag, x, b, res). */
+/* Shared-memory bytes of block 0's levels. */
+__host__ __device__ inline size_t mg_level_bytes(int m) {
+  const size_t c = (size_t)m * m * m, pc = (size_t)(m + 2) * (m + 2) * (m + 2);
+  return (4 * (2 * pc + 2 * c) + 2 * 2 * c + 15) / 16 * 16;
+}
 __host__ __device__ inline size_t mg_block_bytes(const int *m, int lb, int nlev) {
   size_t b = 0;
-  for (int l = lb; l < nlev; l++) {
-    const size_t c = (size_t)m[l] * m[l] * m[l];
-    b += (c + 15) / 16 * 16 + 4 * 4 * c;
-  }
+  for (int l = lb; l < nlev; l++) b += mg_level_bytes(m[l]);
   return b;
+}
+
+/* the block's level l (lb ..), its arrays at their place in shared memory */
+__device__ __forceinline__ MgBlockLevel mg_block_level(const MgArgs &mg, unsigned char *smem,
+                                                       int l) {
+  for (int q = mg.lb; q < l; q++) smem += mg_level_bytes(mg.lv[q].m);
+  MgBlockLevel B;
+  const int m = mg.lv[l].m, c = m * m * m, pm = m + 2, pc = pm * pm * pm;
+  B.m = m;
+  B.pm = pm;
+  B.ncell = c;
+  B.nred = (c + 1) / 2;
+  B.hs = mg.lv[l].hs;
+  B.ihs = mg.lv[l].ihs;
+  B.x = reinterpret_cast<float *>(smem);
+  B.res = B.x + pc;
+  B.b = B.res + pc;
+  B.d = B.b + c;
+  B.at = reinterpret_cast<unsigned short *>(B.d + c);
+  B.slot = B.at + c;
+  return B;
+}
+
+__device__ __forceinline__ void mg_block_init(const MgArgs &mg, unsigned char *smem) {
+  for (int l = mg.lb; l < mg.nlev; l++) {
+    const MgLevel &G = mg.lv[l];
+    const MgBlockLevel B = mg_block_level(mg, smem, l);
+    const int m = B.m, pm = B.pm;
+    for (int e = threadIdx.x; e < 2 * pm * pm * pm; e += blockDim.x) B.x[e] = 0.0f;
+    for (int e = threadIdx.x; e < B.ncell; e += blockDim.x) {
+      int i, j, k;
+      mg_decode((unsigned)e, (unsigned)m, i, j, k);
+      const int w = mg_list_slot(m, i, j, k);
+      B.slot[e] = (unsigned short)w;
+      B.at[w] = (unsigned short)(((i + 1) * pm + j + 1) * pm + k + 1);
+      B.d[w] = G.flags[e] == CELL_FLUID ? G.diag[e] : INFINITY;
+    }
+  }
+}
+
+__device__ __forceinline__ float mg_block_nbsum(const float *x, int p, int pm) {
+  const int pp = pm * pm;
+  return ((((x[p - pp] + x[p + pp]) + x[p - pm]) + x[p + pm]) + x[p - 1]) + x[p + 1];
+}
+
+/* half sweep of one colour over the lists, the block's threads from t in
+ * steps of S */
+__device__ __forceinline__ void mg_block_gs(const MgBlockLevel &L, int color, int t, int S) {
+  const int end = color ? L.ncell : L.nred;
+#pragma unroll 4
+  for (int w = (color ? L.nred : 0) + t; w < end; w += S) {
+    const int p = L.at[w];
+    L.x[p] = __fdividef(L.b[w] * L.ihs + mg_block_nbsum(L.x, p, L.pm), L.d[w]);
+  }
+}
+
+__device__ __forceinline__ void mg_block_residual(const MgBlockLevel &L, int t, int S) {
+#pragma unroll 4
+  for (int w = t; w < L.ncell; w += S) {
+    const int p = L.at[w];
+    const float d = L.d[w];
+    const float r = L.b[w] - L.hs * (d * L.x[p] - mg_block_nbsum(L.x, p, L.pm));
+    L.res[p] = d < INFINITY ? r : 0.0f;
+  }
+}
+
+/* the coarser level's b and first red half sweep from the finer residual */
+__device__ __forceinline__ void mg_block_restrict(const MgBlockLevel &F, const MgBlockLevel &C,
+                                                  int t, int S) {
+  for (int e = t; e < C.ncell; e += S) {
+    int I, J, K;
+    mg_decode((unsigned)e, (unsigned)C.m, I, J, K);
+    float sum = 0.0f;
+#pragma unroll
+    for (int a = 0; a < 2; a++)
+#pragma unroll
+      for (int b = 0; b < 2; b++) {
+        const float *r = F.res + ((2 * I + a + 1) * F.pm + 2 * J + b + 1) * F.pm + 2 * K + 1;
+        sum += r[0];
+        sum += r[1];
+      }
+    const float bc = sum * 0.125f;
+    const int w = C.slot[e];
+    C.b[w] = bc;
+    C.x[C.at[w]] = w < C.nred ? __fdividef(bc * C.ihs, C.d[w]) : 0.0f;
+  }
+}
+
+__device__ __forceinline__ void mg_block_prolong(const MgBlockLevel &F, const MgBlockLevel &C,
+                                                 int t, int S) {
+  for (int e = t; e < F.ncell; e += S) {
+    int i, j, k;
+    mg_decode((unsigned)e, (unsigned)F.m, i, j, k);
+    const int w = F.slot[e], p = F.at[w];
+    const float v = C.x[((i / 2 + 1) * C.pm + j / 2 + 1) * C.pm + k / 2 + 1];
+    if (F.d[w] < INFINITY) F.x[p] += v;
+  }
+}
+
+/* The levels lb.. in block 0's shared memory: V-cycle from level lb's b (in
+ * global memory, from the restriction) to level lb's corrected x (written
+ * back to global memory). Block 0 is alone with these levels, so their
+ * latency is the whole grid's: with the flags, tests and index divisions of
+ * the grid-wide passes they took 20 us a V-cycle of one sweep (n = 128). The
+ * coarsest level (at most 32 cells a colour) runs in one warp. With the middle
+ * levels' fused residual and restriction, flags read first and level 0's loads
+ * requested together, a refined solve at n = 192 went from 8.3 to 6.5 ms, bit
+ * for bit the same. */
+__device__ __forceinline__ void mg_block_levels(const MgArgs &mg, unsigned char *smem) {
+  const int t = threadIdx.x, S = blockDim.x;
+  const int last = mg.nlev - 1;
+  const MgLevel &G = mg.lv[mg.lb];
+  const MgBlockLevel T = mg_block_level(mg, smem, mg.lb);
+  for (int e0 = t; e0 < T.ncell; e0 += S * 8) {
+    float bv[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) bv[u] = e0 + u * S < T.ncell ? __ldcg(G.b + e0 + u * S) : 0.0f;
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const int e = e0 + u * S;
+      if (e >= T.ncell) continue;
+      const int w = T.slot[e];
+      T.b[w] = bv[u];
+      T.x[T.at[w]] = w < T.nred ? __fdividef(bv[u] * T.ihs, T.d[w]) : 0.0f;
+    }
+  }
+  __syncthreads();
+  for (int l = mg.lb; l < last; l++) {
+    const MgBlockLevel L = mg_block_level(mg, smem, l);
+    mg_block_gs(L, 1, t, S);
+    __syncthreads();
+    for (int sw = 1; sw < mg.nu; sw++) {
+      mg_block_gs(L, 0, t, S);
+      __syncthreads();
+      mg_block_gs(L, 1, t, S);
+      __syncthreads();
+    }
+    mg_block_residual(L, t, S);
+    __syncthreads();
+    mg_block_restrict(L, mg_block_level(mg, smem, l + 1), t, S);
+    __syncthreads();
+  }
+  /* coarsest: the first red half sweep is done; the black half sweep that
+   * ends the forward sweeps also starts the backward ones */
+  if (t < 32) {
+    const MgBlockLevel L = mg_block_level(mg, smem, last);
+    mg_block_gs(L, 1, t, 32);
+    __syncwarp();
+    for (int it = 1; it < mg.coarse_sweeps; it++) {
+      mg_block_gs(L, 0, t, 32);
+      __syncwarp();
+      mg_block_gs(L, 1, t, 32);
+      __syncwarp();
+    }
+    for (int it = 0; it < mg.coarse_sweeps; it++) {
+      if (it > 0) {
+        mg_block_gs(L, 1, t, 32);
+        __syncwarp();
+      }
+      mg_block_gs(L, 0, t, 32);
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  for (int l = last - 1; l >= mg.lb; l--) {
+    const MgBlockLevel L = mg_block_level(mg, smem, l);
+    mg_block_prolong(L, mg_block_level(mg, smem, l + 1), t, S);
+    __syncthreads();
+    for (int sw = 0; sw < mg.nu; sw++) {
+      mg_block_gs(L, 1, t, S);
+      __syncthreads();
+      mg_block_gs(L, 0, t, S);
+      __syncthreads();
+    }
+  }
+  for (int e = t; e < T.ncell; e += S) G.x[e] = T.x[T.at[T.slot[e]]];
 }
 
 /* Level-0 phases on quads of the liquid chunks. */
@@ -1719,6 +1853,17 @@ __device__ __forceinline__ void mg_quads(const CgArgs &a, float alpha, float bet
     const long off[4] = {(long)qplane, -(long)qplane, (long)qrow, -(long)qrow};
     const bool ed = (lane == 0 && k0 > 0) || (lane == 31 && k0 + 4 < n);
     const size_t ce = lane == 0 ? c0 - 1 : c0 + 4;
+    /* everything the phase reads is requested here, before the first use:
+     * loads left behind the flag test or the shuffles would cost the chunk a
+     * second round trip to L2 */
+    const float4 dg = __ldg(d4p + qs);
+    float4 r4 = zero, x4 = zero, p4u = zero, q4 = zero;
+    if (PH != MG_MATVEC) r4 = __ldcg(reinterpret_cast<const float4 *>(rf) + qs);
+    if (PH == MG_UPDATE) {
+      x4 = __ldcg(reinterpret_cast<const float4 *>(a.x) + qs);
+      p4u = __ldcg(reinterpret_cast<const float4 *>(pnew) + qs);
+      q4 = __ldcg(reinterpret_cast<const float4 *>(a.q) + qs);
+    }
     if (PH == MG_MATVEC) {
       const float4 z4 = __ldcg(reinterpret_cast<const float4 *>(zf) + qs);
       const float4 p4 = __ldcg(reinterpret_cast<const float4 *>(pold) + qs);
@@ -1792,7 +1937,6 @@ __device__ __forceinline__ void mg_quads(const CgArgs &a, float alpha, float bet
       for (int u = 0; u < 4; u++) nbs[u] = ((((n0[u] + n1[u]) + n2[u]) + n3[u]) + kl[u]) + kr[u];
     }
     if (PH == MG_MATVEC) {
-      const float4 dg = __ldg(d4p + qs);
       const float dv[4] = {dg.x, dg.y, dg.z, dg.w};
       float qv[4], pv[4];
 #pragma unroll
@@ -1805,13 +1949,8 @@ __device__ __forceinline__ void mg_quads(const CgArgs &a, float alpha, float bet
       reinterpret_cast<float4 *>(a.q)[q] = make_float4(qv[0], qv[1], qv[2], qv[3]);
     } else if (PH == MG_UPDATE) {
       /* x += alpha p', r -= alpha q; r.r; z: first red half sweep from 0 */
-      const float4 x4 = __ldcg(reinterpret_cast<const float4 *>(a.x) + q);
-      const float4 r4 = __ldcg(reinterpret_cast<const float4 *>(rf) + q);
-      const float4 p4 = __ldcg(reinterpret_cast<const float4 *>(pnew) + q);
-      const float4 q4 = __ldcg(reinterpret_cast<const float4 *>(a.q) + q);
-      const float4 dg = __ldg(d4p + qs);
       const float xv[4] = {x4.x, x4.y, x4.z, x4.w}, rv[4] = {r4.x, r4.y, r4.z, r4.w};
-      const float pv[4] = {p4.x, p4.y, p4.z, p4.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
+      const float pv[4] = {p4u.x, p4u.y, p4u.z, p4u.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
       const float dv[4] = {dg.x, dg.y, dg.z, dg.w};
       float xn[4], rn[4], zn[4];
 #pragma unroll
@@ -1830,8 +1969,6 @@ __device__ __forceinline__ void mg_quads(const CgArgs &a, float alpha, float bet
       reinterpret_cast<float4 *>(rf)[q] = make_float4(rn[0], rn[1], rn[2], rn[3]);
       reinterpret_cast<float4 *>(zf)[q] = make_float4(zn[0], zn[1], zn[2], zn[3]);
     } else if (PH == MG_RES) {
-      const float4 r4 = __ldcg(reinterpret_cast<const float4 *>(rf) + q);
-      const float4 dg = __ldg(d4p + qs);
       const float rv[4] = {r4.x, r4.y, r4.z, r4.w}, dv[4] = {dg.x, dg.y, dg.z, dg.w};
       float res[4];
 #pragma unroll
@@ -1839,8 +1976,6 @@ __device__ __forceinline__ void mg_quads(const CgArgs &a, float alpha, float bet
       reinterpret_cast<float4 *>(L0.res)[q] = make_float4(res[0], res[1], res[2], res[3]);
     } else { /* MG_BLACK, MG_BLACK_PROLONG, MG_RED, MG_RED_DOT: half sweep of one colour */
       const int color = (PH == MG_RED_DOT || PH == MG_RED) ? 0 : 1;
-      const float4 r4 = __ldcg(reinterpret_cast<const float4 *>(rf) + q);
-      const float4 dg = __ldg(d4p + qs);
       const float rv[4] = {r4.x, r4.y, r4.z, r4.w}, dv[4] = {dg.x, dg.y, dg.z, dg.w};
       const float o0[4] = {own0.x, own0.y, own0.z, own0.w};
       float zn[4];
@@ -1874,29 +2009,9 @@ template <int BLOCK> __global__ void __launch_bounds__(BLOCK, 1) k_cg_mg(CgArgs 
   __shared__ int s_done;
   extern __shared__ __align__(16) unsigned char mg_smem[];
 
-  /* block 0: its levels' flags and diagonals into shared memory (fixed
+  /* block 0: its levels' lists and diagonals into shared memory (fixed
    * during the solve) */
-  MgLevel sl[MG_MAX_LEVELS];
-  if (blockIdx.x == 0) {
-    unsigned char *pp = mg_smem;
-    for (int l = mg.lb; l < mg.nlev; l++) {
-      const unsigned m = (unsigned)mg.lv[l].m, c = m * m * m;
-      sl[l] = mg.lv[l];
-      uint8_t *fl8 = pp;
-      pp += (c + 15) / 16 * 16;
-      float *dg = reinterpret_cast<float *>(pp);
-      sl[l].x = dg + c;
-      sl[l].b = dg + 2 * c;
-      sl[l].res = dg + 3 * c;
-      pp += 4 * 4 * (size_t)c;
-      for (unsigned e = threadIdx.x; e < c; e += BLOCK) {
-        fl8[e] = mg.lv[l].flags[e];
-        dg[e] = mg.lv[l].diag[e];
-      }
-      sl[l].flags = fl8;
-      sl[l].diag = dg;
-    }
-  }
+  if (blockIdx.x == 0) mg_block_init(mg, mg_smem);
 
   /* phase 0: r = b - A x on the liquid (x zeroed elsewhere); b.b, r.r */
   FF pbb = ff_zero(), prr = ff_zero();
@@ -1969,35 +2084,33 @@ template <int BLOCK> __global__ void __launch_bounds__(BLOCK, 1) k_cg_mg(CgArgs 
     }
     mg_quads<MG_RES, BLOCK>(a, 0.0f, 0.0f, nullptr, nullptr, none);
     if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-    mg_restrict<true, true>(mg.lv[0], mg.lv[1], gt, gs);
+    mg_restrict(mg.lv[0], mg.lv[1], gt, gs);
     if (!count_barrier(a.bar, epoch, a.iflags)) return false;
     for (int l = 1; l < mg.lb; l++) {
-      mg_gs<true>(mg.lv[l], 1, gt, gs);
+      mg_gs(mg.lv[l], 1, gt, gs);
       if (!count_barrier(a.bar, epoch, a.iflags)) return false;
       for (int sw = 1; sw < mg.nu; sw++) {
-        mg_gs<true>(mg.lv[l], 0, gt, gs);
+        mg_gs(mg.lv[l], 0, gt, gs);
         if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-        mg_gs<true>(mg.lv[l], 1, gt, gs);
+        mg_gs(mg.lv[l], 1, gt, gs);
         if (!count_barrier(a.bar, epoch, a.iflags)) return false;
       }
-      mg_residual<true>(mg.lv[l], gt, gs);
-      if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-      mg_restrict<true, true>(mg.lv[l], mg.lv[l + 1], gt, gs);
+      mg_residual_restrict(mg.lv[l], mg.lv[l + 1], gt, gs);
       if (!count_barrier(a.bar, epoch, a.iflags)) return false;
     }
-    if (blockIdx.x == 0) mg_block_levels(mg, sl);
+    if (blockIdx.x == 0) mg_block_levels(mg, mg_smem);
     if (!count_barrier(a.bar, epoch, a.iflags)) return false;
     for (int l = mg.lb - 1; l >= 1; l--) {
-      mg_prolong<true, true>(mg.lv[l], mg.lv[l + 1], gt, gs);
+      mg_prolong(mg.lv[l], mg.lv[l + 1], gt, gs);
       if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-      mg_gs<true>(mg.lv[l], 1, gt, gs);
+      mg_gs(mg.lv[l], 1, gt, gs);
       if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-      mg_gs<true>(mg.lv[l], 0, gt, gs);
+      mg_gs(mg.lv[l], 0, gt, gs);
       if (!count_barrier(a.bar, epoch, a.iflags)) return false;
       for (int sw = 1; sw < mg.nu; sw++) {
-        mg_gs<true>(mg.lv[l], 1, gt, gs);
+        mg_gs(mg.lv[l], 1, gt, gs);
         if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-        mg_gs<true>(mg.lv[l], 0, gt, gs);
+        mg_gs(mg.lv[l], 0, gt, gs);
         if (!count_barrier(a.bar, epoch, a.iflags)) return false;
       }
     }
@@ -3097,7 +3210,7 @@ constexpr int MG_COARSE_SWEEPS = 2; /* the iteration count does not depend on it
 constexpr int MG_SWEEPS_DEFAULT = 2; /* measured: 1 -> 2 sweeps cut the solve 11 % at
                                           n=128 and 35 % at n=256; 3 gain nothing */
 constexpr int CG_MG_BLOCK = 512;
-constexpr size_t MG_SMEM_MAX = 96 * 1024; /* block 0's levels: <= 16^3 + 8^3 + 4^3 cells */
+constexpr size_t MG_SMEM_MAX = 128 * 1024; /* block 0's levels: <= 16^3 + 8^3 + 4^3 cells */
 
 /* threads per block of a persistent CG kernel */
 static int cg_block_of(const void *kern) {
@@ -3123,7 +3236,8 @@ int mg_alloc(FlipGpu *h) {
   if (nlev < 2 || lv[nlev - 1] > 4) return FLIPGPU_EINVAL;
   int lb = 1;
   while (lb < nlev - 1 && (size_t)lv[lb] * lv[lb] * lv[lb] > MG_BLOCK_CELLS) lb++;
-  if (mg_block_bytes(lv, lb, nlev) > MG_SMEM_MAX) return FLIPGPU_EINVAL;
+  if (nlev - lb > MG_BLOCK_LEVELS || mg_block_bytes(lv, lb, nlev) > MG_SMEM_MAX)
+    return FLIPGPU_EINVAL;
   const size_t nc = h->nc;
   bool ok = cudaMalloc(&h->mg_res[0], nc * sizeof(float)) == cudaSuccess &&
             cudaMalloc(&h->mg_p2, nc * sizeof(float)) == cudaSuccess &&
