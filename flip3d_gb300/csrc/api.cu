@@ -395,7 +395,7 @@ int flipgpu_create(const FlipGpuParams *p, FlipGpu **out) {
   AL(h->A, nc) AL(h->L, nc) AL(h->press, nc) AL(h->div, nc) AL(h->r, nc) AL(h->z, nc)
   AL(h->press_lo, nc) AL(h->ir_b, nc) AL(h->ir_e, nc)
   AL(h->s, nc) AL(h->s1, nc) AL(h->w, nc) AL(h->w1, nc) AL(h->pdir, nc) AL(h->chunk_off, nc / 128 + 2) AL(h->chunk_list, nc / 128 + 1) AL(h->P, 2 * nc) AL(h->Pf, nc) AL(h->diag, nc)
-  AL(h->partial, 8192) AL(h->bar, 2)
+  AL(h->partial, 8192) AL(h->bar, BAR_WORDS)
   AL(h->scal, SC_COUNT) AL(h->iflags, IF_COUNT) AL(h->flag, cap) AL(h->scan_a, scan_n)
   AL(h->scan_b, scan_n) AL(h->scan_tmp, h->scan_cap) AL(h->stuck_idx, cap)
   AL(h->water_idx, nc) AL(h->stage, 3 * cap)

@@ -64,6 +64,7 @@ struct SimConst {
   const int64_t *dstep; /* the step counter in device memory (graph replays advance it) */
 };
 
+constexpr int BAR_WORDS = 12;
 constexpr int CG_VARIANTS = 6; /* persistent CG kernels (k_pcg.cu cg_grid_size) */
 
 struct FlipGpu {
@@ -128,7 +129,9 @@ struct FlipGpu {
   /* MG preconditioner (k_pcg.cu mg_alloc): levels 1.. and level-0 scratch */
   int mg_nlev, mg_lb, mg_m[10];
   uint8_t *mg_flags[10];
-  float *mg_diag[10], *mg_x[10], *mg_b[10], *mg_res[10];
+  float *mg_diag[10], *mg_x[10], *mg_b[10];
+  float *mg_y[10];        /* middle levels: the correction after the post-smoothing */
+  unsigned *mg_tiles[10]; /* the tiles of a level that hold liquid */
   float *mg_p2, *mg_q;
   unsigned *chunk_off;  /* single-reduction CG: liquid flags of the 32-quad chunks, scanned */
   unsigned *chunk_list; /* ... and the indices of the chunks that hold liquid */
@@ -138,7 +141,8 @@ struct FlipGpu {
   double *partial;    /* per-block reduction partials */
   double *scal;       /* device scalars of the CG recurrence */
   int *iflags;        /* device flags/counters */
-  unsigned *bar;      /* grid barrier of the persistent CG: count, generation */
+  unsigned *bar;      /* BAR_WORDS: grid barrier of the persistent CG (count, generation),
+                         then the number of tiles in each level's mg_tiles */
   int cg_grid[CG_VARIANTS]; /* cooperative CG grids (0 = none): REF, FAST, FAST single-
                                reduction (small blocks), FAST IC, single-reduction (large),
                                FAST MG */

@@ -454,9 +454,11 @@ struct MgLevel {
   int m;                 /* cells per axis */
   const uint8_t *flags;  /* CELL_FLUID / CELL_AIR / CELL_WALL */
   const float *diag;     /* level 0: the operator's diagonal; coarser: non-wall neighbours */
-  float *x, *b, *res;    /* correction, right-hand side, residual */
+  float *x, *b;          /* correction, right-hand side */
+  float *out;            /* the level's final correction: x, or a tiled level's second buffer */
   float hs, ihs;         /* 1 / h^2 of the level and its inverse */
   int lgm;               /* log2(m) when m is a power of two, else -1 */
+  unsigned *tiles, *ntiles; /* middle levels: the tiles holding liquid, their number */
 };
 struct MgArgs {
   MgLevel lv[MG_MAX_LEVELS];
@@ -552,9 +554,9 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, int *iflags,
 
 /* A counting grid barrier: bar[0] counts the arrivals of the whole launch
  * (zeroed before it), so the epoch-th barrier is complete when it reaches
- * epoch x gridDim.x. Thread 0 arrives with a release add after the block's
- * __syncthreads and polls with acquire loads: two L2 round trips, no reset
- * and no generation word. The wait gives up after 2 s of %globaltimer,
+ * epoch x gridDim.x. Thread 0 arrives with an acquire-release add after the
+ * block's __syncthreads (the last block to arrive reads no more) and polls
+ * with acquire loads: two L2 round trips, no reset and no generation word. The wait gives up after 2 s of %globaltimer,
  * flags FLIPGPU_ETIMEOUT and returns false in that block (the others give up
  * at their next barrier). */
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -570,7 +572,7 @@ __device__ __forceinline__ bool count_barrier(unsigned *bar, unsigned &epoch, in
     epoch++;
     const unsigned target = epoch * gridDim.x;
     unsigned v;
-    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(bar) : "memory");
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(bar) : "memory");
     v += 1;
     bool good = true;
     unsigned long long t0 = 0;
@@ -1413,7 +1415,7 @@ __device__ __forceinline__ float mg_nbsum(const float *x, int m, int i, int j, i
 /* red-black half sweep: liquid cells of `color` take
  * x = (b / hs + sum of the neighbours' x) / diag. The pairs of cells
  * (2 kk, 2 kk + 1) of a line are enumerated, each with its cell of the colour. */
-__device__ __noinline__ void mg_gs(const MgLevel L, int color, unsigned start, unsigned stride) {
+__device__ __forceinline__ void mg_gs(const MgLevel &L, int color, unsigned start, unsigned stride) {
   const unsigned m = (unsigned)L.m, hm = (m + 1) >> 1, tot = m * m * hm;
   for (unsigned h0 = start; h0 < tot; h0 += stride * MGU) {
     unsigned cc[MGU];
@@ -1461,49 +1463,12 @@ __device__ __forceinline__ void mg_coarse_start(const MgLevel &Cl, unsigned c, b
   Cl.x[c] = red ? __fdividef(bc * Cl.ihs, __ldg(Cl.diag + c)) : 0.0f;
 }
 
-/* from the residual that the level-0 pass stored (n is even) */
-__device__ __noinline__ void mg_restrict(const MgLevel F, const MgLevel Cl, unsigned start,
-                                         unsigned stride) {
-  const unsigned mc = (unsigned)Cl.m, totc = mc * mc * mc, mf = (unsigned)F.m;
-  for (unsigned c0 = start; c0 < totc; c0 += stride * MGU) {
-    float sum[MGU];
-    bool red[MGU];
-#pragma unroll
-    for (int u = 0; u < MGU; u++) {
-      const unsigned c = c0 + (unsigned)u * stride;
-      sum[u] = 0.0f;
-      red[u] = false;
-      if (c < totc && __ldg(Cl.flags + c) == CELL_FLUID) {
-        int I, J, K;
-        mg_decode(c, mc, Cl.lgm, I, J, K);
-        red[u] = ((I + J + K) & 1) == 0;
-        /* the k pair as one aligned float2 */
-#pragma unroll
-        for (int a = 0; a < 2; a++)
-#pragma unroll
-          for (int b = 0; b < 2; b++) {
-            const unsigned i = 2u * I + a, j = 2u * J + b;
-            const float2 v = __ldcg(
-                reinterpret_cast<const float2 *>(F.res + (i * mf + j) * mf + 2u * K));
-            sum[u] += v.x;
-            sum[u] += v.y;
-          }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < MGU; u++) {
-      const unsigned c = c0 + (unsigned)u * stride;
-      if (c < totc) mg_coarse_start(Cl, c, red[u], sum[u]);
-    }
-  }
-}
-
 /* residual b - A x and restriction of a middle level in one pass: a thread
  * per coarse cell computes its 8 children's residuals (two lines of two
  * cells in i and j, and the cells around them), which saves writing and
  * rereading them and a grid barrier */
-__device__ __noinline__ void mg_residual_restrict(const MgLevel F, const MgLevel Cl,
-                                                  unsigned start, unsigned stride) {
+__device__ __forceinline__ void mg_residual_restrict(const MgLevel &F, const MgLevel &Cl,
+                                                     unsigned start, unsigned stride) {
   const int mc = Cl.m, m = F.m;
   const unsigned totc = (unsigned)mc * mc * mc;
   const unsigned mm = (unsigned)m * m;
@@ -1565,8 +1530,8 @@ __device__ __noinline__ void mg_residual_restrict(const MgLevel F, const MgLevel
 }
 
 /* x += the parent's correction on the liquid */
-__device__ __noinline__ void mg_prolong(const MgLevel F, const MgLevel Cl, unsigned start,
-                                        unsigned stride) {
+__device__ __forceinline__ void mg_prolong(const MgLevel &F, const MgLevel &Cl, unsigned start,
+                                           unsigned stride) {
   const unsigned mf = (unsigned)F.m, tot = mf * mf * mf, mc = (unsigned)Cl.m;
   for (unsigned c0 = start; c0 < tot; c0 += stride * MGU) {
     float xv[MGU], ev[MGU];
@@ -1585,7 +1550,7 @@ __device__ __noinline__ void mg_prolong(const MgLevel F, const MgLevel Cl, unsig
         const unsigned pc =
             (((unsigned)i >> 1) * mc + ((unsigned)j >> 1)) * mc + ((unsigned)k >> 1);
         xv[u] = __ldcg(F.x + c);
-        ev[u] = __ldcg(Cl.x + pc);
+        ev[u] = __ldcg(Cl.out + pc);
       }
 #pragma unroll
     for (int u = 0; u < MGU; u++)
@@ -1593,35 +1558,28 @@ __device__ __noinline__ void mg_prolong(const MgLevel F, const MgLevel Cl, unsig
   }
 }
 
-/* One of block 0's levels in shared memory. x and res are padded by a zero
- * layer, so that neighbours need no tests. The cells are listed by colour
- * (red, i + j + k even, first; within a colour in cell order): at[] holds a
- * listed cell's padded index, d[] its diagonal, infinite off the liquid, where
- * x = (b / hs + neighbours) / d then stays 0, and b[] its right-hand side. */
+/* One of block 0's levels (at most 16 cells an axis) in shared memory. A
+ * thread owns a segment, cells k = 8 seg .. 8 seg + 7 of one line (i, j): four
+ * of each colour (red: i + j + k even). The colours are stored apart, as float4s
+ * of the cells k / 2 = 4 seg .. 4 seg + 3: the four neighbouring lines' other
+ * colour then lies at the same place of their segments, and the neighbours in k
+ * are the thread's own values but one. x has a layer of zero lines around it;
+ * off the liquid and past the line's end the diagonal is infinite, so that
+ * x = (b / hs + neighbours) / d stays 0. No test, no division and, a half
+ * sweep, four 16-byte loads and one store a thread. */
 struct MgBlockLevel {
-  int m, pm;             /* cells per axis; m + 2 */
-  int nred, ncell;
+  int m, ns, segs;   /* cells per axis; segments of a line (1 or 2) and in all */
+  int act, id;       /* threads: segs rounded up to whole warps; their barrier */
   float hs, ihs;
-  float *x, *res, *b, *d;
-  unsigned short *at, *slot; /* slot: cell -> its place in the lists */
+  float4 *x[2];      /* colour 0 (red), 1: [(m + 2)^2 lines][ns] */
+  float4 *b[2], *d[2], *r[2]; /* [m^2 lines][ns]; r: the residuals of even and odd k */
 };
-constexpr int MG_BLOCK_LEVELS = 3; /* at most 16, 8 and 4 cells per axis */
-
-/* place of cell (i, j, k) of m^3 in the lists: the red cells before row (i, j)
- * are counted from the rows that start red, ceil(m / 2) of them in lines of
- * even i, floor(m / 2) in the others */
-__host__ __device__ inline int mg_list_slot(int m, int i, int j, int k) {
-  const int up = (m + 1) / 2, dn = m / 2;
-  const int z = (i + 1) / 2 * up + i / 2 * dn + (i & 1 ? j / 2 : (j + 1) / 2);
-  const int rows = i * m + j, red = z * up + (rows - z) * dn;
-  const int all = (m * m * m + 1) / 2;
-  return ((i + j + k) & 1) == 0 ? red + k / 2 : all + rows * m - red + k / 2;
-}
+constexpr int MG_BLOCK_MAX = 16; /* cells per axis */
 
 /* Shared-memory bytes of block 0's levels. */
 __host__ __device__ inline size_t mg_level_bytes(int m) {
-  const size_t c = (size_t)m * m * m, pc = (size_t)(m + 2) * (m + 2) * (m + 2);
-  return (4 * (2 * pc + 2 * c) + 2 * 2 * c + 15) / 16 * 16;
+  const size_t ns = m > 8 ? 2 : 1, pm = (size_t)m + 2;
+  return 16 * ns * 2 * (pm * pm + 3 * (size_t)m * m);
 }
 __host__ __device__ inline size_t mg_block_bytes(const int *m, int lb, int nlev) {
   size_t b = 0;
@@ -1629,193 +1587,511 @@ __host__ __device__ inline size_t mg_block_bytes(const int *m, int lb, int nlev)
   return b;
 }
 
-/* the block's level l (lb ..), its arrays at their place in shared memory */
-__device__ __forceinline__ MgBlockLevel mg_block_level(const MgArgs &mg, unsigned char *smem,
-                                                       int l) {
-  for (int q = mg.lb; q < l; q++) smem += mg_level_bytes(mg.lv[q].m);
+/* a middle level's tile (mg_tile_level) comes first */
+constexpr int MG_TILE = 8, MG_HALO = 4, MG_REGION = 16, MG_TILE_NU = 2;
+constexpr int MG_TILE_LINES = MG_REGION * MG_REGION * 2; /* segments: one a thread */
+constexpr int MG_TILE_PLINES = (MG_REGION + 2) * (MG_REGION + 2) * 2;
+constexpr size_t MG_TILE_BYTES = 16 * 2 * (size_t)(MG_TILE_PLINES + MG_TILE_LINES);
+
+extern __shared__ __align__(16) float4 mg_smem[];
+
+/* the block's level l (lb ..) */
+__device__ __forceinline__ MgBlockLevel mg_block_level(const MgArgs &mg, int l) {
+  float4 *at = mg_smem + MG_TILE_BYTES / 16; /* after the tile's */
+  for (int q = mg.lb; q < l; q++) at += mg_level_bytes(mg.lv[q].m) / 16;
   MgBlockLevel B;
-  const int m = mg.lv[l].m, c = m * m * m, pm = m + 2, pc = pm * pm * pm;
-  B.m = m;
-  B.pm = pm;
-  B.ncell = c;
-  B.nred = (c + 1) / 2;
+  B.m = mg.lv[l].m;
   B.hs = mg.lv[l].hs;
   B.ihs = mg.lv[l].ihs;
-  B.x = reinterpret_cast<float *>(smem);
-  B.res = B.x + pc;
-  B.b = B.res + pc;
-  B.d = B.b + c;
-  B.at = reinterpret_cast<unsigned short *>(B.d + c);
-  B.slot = B.at + c;
+  B.ns = B.m > 8 ? 2 : 1;
+  const int lines = B.m * B.m * B.ns, plines = (B.m + 2) * (B.m + 2) * B.ns;
+  B.segs = lines;
+  B.act = (lines + 31) / 32 * 32;
+  B.id = 1 + l - mg.lb;
+  B.x[0] = at;
+  B.x[1] = at + plines;
+  B.b[0] = at + 2 * plines;
+  B.b[1] = B.b[0] + lines;
+  B.d[0] = B.b[1] + lines;
+  B.d[1] = B.d[0] + lines;
+  B.r[0] = B.d[1] + lines;
+  B.r[1] = B.r[0] + lines;
   return B;
 }
 
-__device__ __forceinline__ void mg_block_init(const MgArgs &mg, unsigned char *smem) {
+/* the segment of thread t (< segs) */
+struct MgSeg {
+  int i, j, seg, par; /* par: (i + j) & 1, the parity of its red cells' k */
+  int at;             /* its place in x */
+};
+__device__ __forceinline__ MgSeg mg_seg(const MgBlockLevel &L, int t) {
+  MgSeg s;
+  const int line = L.ns == 2 ? t >> 1 : t;
+  s.seg = L.ns == 2 ? t & 1 : 0;
+  s.i = line / L.m;
+  s.j = line - s.i * L.m;
+  s.par = (s.i + s.j) & 1;
+  s.at = ((s.i + 1) * (L.m + 2) + s.j + 1) * L.ns + s.seg;
+  return s;
+}
+
+/* barrier of a level's threads: each level has its own, since the threads
+ * that skip the coarser levels wait at theirs meanwhile */
+__device__ __forceinline__ void mg_bar(const MgBlockLevel &L) {
+  asm volatile("bar.sync %0, %1;" ::"r"(L.id), "r"(L.act) : "memory");
+}
+
+__device__ __forceinline__ void mg_block_init(const MgArgs &mg) {
   for (int l = mg.lb; l < mg.nlev; l++) {
     const MgLevel &G = mg.lv[l];
-    const MgBlockLevel B = mg_block_level(mg, smem, l);
-    const int m = B.m, pm = B.pm;
-    for (int e = threadIdx.x; e < 2 * pm * pm * pm; e += blockDim.x) B.x[e] = 0.0f;
-    for (int e = threadIdx.x; e < B.ncell; e += blockDim.x) {
-      int i, j, k;
-      mg_decode((unsigned)e, (unsigned)m, i, j, k);
-      const int w = mg_list_slot(m, i, j, k);
-      B.slot[e] = (unsigned short)w;
-      B.at[w] = (unsigned short)(((i + 1) * pm + j + 1) * pm + k + 1);
-      B.d[w] = G.flags[e] == CELL_FLUID ? G.diag[e] : INFINITY;
+    const MgBlockLevel B = mg_block_level(mg, l);
+    const int m = B.m, n4 = (int)(mg_level_bytes(m) / 16);
+    for (int e = threadIdx.x; e < n4; e += blockDim.x) B.x[0][e] = make_float4(0, 0, 0, 0);
+    __syncthreads();
+    if ((int)threadIdx.x < B.segs) {
+      const MgSeg s = mg_seg(B, threadIdx.x);
+      float dv[2][4]; /* even and odd k */
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int k = 8 * s.seg + u;
+        const unsigned c = ((unsigned)s.i * m + s.j) * m + k;
+        dv[u & 1][u >> 1] = k < m && G.flags[c] == CELL_FLUID ? G.diag[c] : INFINITY;
+      }
+      const float4 e = make_float4(dv[0][0], dv[0][1], dv[0][2], dv[0][3]),
+                   o = make_float4(dv[1][0], dv[1][1], dv[1][2], dv[1][3]);
+      B.d[0][threadIdx.x] = s.par ? o : e;
+      B.d[1][threadIdx.x] = s.par ? e : o;
     }
   }
 }
 
-__device__ __forceinline__ float mg_block_nbsum(const float *x, int p, int pm) {
-  const int pp = pm * pm;
-  return ((((x[p - pp] + x[p + pp]) + x[p - pm]) + x[p + pm]) + x[p - 1]) + x[p + 1];
+__device__ __forceinline__ float4 mg_add4(float4 a, float4 b) {
+  return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
 }
 
-/* half sweep of one colour over the lists, the block's threads from t in
- * steps of S */
-__device__ __forceinline__ void mg_block_gs(const MgBlockLevel &L, int color, int t, int S) {
-  const int end = color ? L.ncell : L.nred;
-#pragma unroll 4
-  for (int w = (color ? L.nred : 0) + t; w < end; w += S) {
-    const int p = L.at[w];
-    L.x[p] = __fdividef(L.b[w] * L.ihs + mg_block_nbsum(L.x, p, L.pm), L.d[w]);
-  }
+/* the sum of the neighbours of the segment's cells of one colour: o, the other
+ * colour in shared memory; mine, the segment's own cells of that other colour;
+ * odd: whether the cells summed for have odd k */
+__device__ __forceinline__ float4 mg_block_nbs(const MgBlockLevel &L, const MgSeg &s,
+                                               const float4 *o, float4 mine, bool odd) {
+  const int ii = (L.m + 2) * L.ns, jj = L.ns;
+  const float4 v = mg_add4(mg_add4(mg_add4(o[s.at - ii], o[s.at + ii]), o[s.at - jj]),
+                           o[s.at + jj]);
+  /* the neighbour across the segment's end: after it for odd k, before it for even */
+  const bool have = odd ? s.seg + 1 < L.ns : s.seg > 0;
+  const float e =
+      have ? reinterpret_cast<const float *>(o + s.at)[odd ? 4 : -1] : 0.0f;
+  const float4 lo = odd ? mine : make_float4(e, mine.x, mine.y, mine.z);
+  const float4 hi = odd ? make_float4(mine.y, mine.z, mine.w, e) : mine;
+  return mg_add4(mg_add4(v, lo), hi);
 }
 
-__device__ __forceinline__ void mg_block_residual(const MgBlockLevel &L, int t, int S) {
-#pragma unroll 4
-  for (int w = t; w < L.ncell; w += S) {
-    const int p = L.at[w];
-    const float d = L.d[w];
-    const float r = L.b[w] - L.hs * (d * L.x[p] - mg_block_nbsum(L.x, p, L.pm));
-    L.res[p] = d < INFINITY ? r : 0.0f;
-  }
+/* half sweep of colour C by the segment's thread; own[]: its cells */
+template <int C>
+__device__ __forceinline__ void mg_block_half(const MgBlockLevel &L, const MgSeg &s, float4 b,
+                                              float4 d, float4 (&own)[2]) {
+  const float4 v = mg_block_nbs(L, s, L.x[C ^ 1], own[C ^ 1], s.par ? C == 0 : C == 1);
+  own[C] = make_float4(
+      __fdividef(b.x * L.ihs + v.x, d.x), __fdividef(b.y * L.ihs + v.y, d.y),
+      __fdividef(b.z * L.ihs + v.z, d.z), __fdividef(b.w * L.ihs + v.w, d.w));
+  L.x[C][s.at] = own[C];
 }
 
-/* the coarser level's b and first red half sweep from the finer residual */
-__device__ __forceinline__ void mg_block_restrict(const MgBlockLevel &F, const MgBlockLevel &C,
-                                                  int t, int S) {
-  for (int e = t; e < C.ncell; e += S) {
-    int I, J, K;
-    mg_decode((unsigned)e, (unsigned)C.m, I, J, K);
-    float sum = 0.0f;
-#pragma unroll
-    for (int a = 0; a < 2; a++)
-#pragma unroll
-      for (int b = 0; b < 2; b++) {
-        const float *r = F.res + ((2 * I + a + 1) * F.pm + 2 * J + b + 1) * F.pm + 2 * K + 1;
-        sum += r[0];
-        sum += r[1];
-      }
-    const float bc = sum * 0.125f;
-    const int w = C.slot[e];
-    C.b[w] = bc;
-    C.x[C.at[w]] = w < C.nred ? __fdividef(bc * C.ihs, C.d[w]) : 0.0f;
-  }
+__device__ __forceinline__ float mg_block_res(float b, float hs, float d, float x, float nbs) {
+  return d < INFINITY ? b - hs * (d * x - nbs) : 0.0f;
 }
 
-__device__ __forceinline__ void mg_block_prolong(const MgBlockLevel &F, const MgBlockLevel &C,
-                                                 int t, int S) {
-  for (int e = t; e < F.ncell; e += S) {
-    int i, j, k;
-    mg_decode((unsigned)e, (unsigned)F.m, i, j, k);
-    const int w = F.slot[e], p = F.at[w];
-    const float v = C.x[((i / 2 + 1) * C.pm + j / 2 + 1) * C.pm + k / 2 + 1];
-    if (F.d[w] < INFINITY) F.x[p] += v;
-  }
+/* the segment's residuals, by the parity of k */
+__device__ __forceinline__ void mg_block_residuals(const MgBlockLevel &L, const MgSeg &s, int t,
+                                                   const float4 (&b)[2], const float4 (&d)[2],
+                                                   const float4 (&own)[2]) {
+  const float4 n0 = mg_block_nbs(L, s, L.x[1], own[1], s.par),
+               n1 = mg_block_nbs(L, s, L.x[0], own[0], !s.par);
+  const float hs = L.hs;
+  const float4 r0 = make_float4(mg_block_res(b[0].x, hs, d[0].x, own[0].x, n0.x),
+                                mg_block_res(b[0].y, hs, d[0].y, own[0].y, n0.y),
+                                mg_block_res(b[0].z, hs, d[0].z, own[0].z, n0.z),
+                                mg_block_res(b[0].w, hs, d[0].w, own[0].w, n0.w));
+  const float4 r1 = make_float4(mg_block_res(b[1].x, hs, d[1].x, own[1].x, n1.x),
+                                mg_block_res(b[1].y, hs, d[1].y, own[1].y, n1.y),
+                                mg_block_res(b[1].z, hs, d[1].z, own[1].z, n1.z),
+                                mg_block_res(b[1].w, hs, d[1].w, own[1].w, n1.w));
+  L.r[0][t] = s.par ? r1 : r0;
+  L.r[1][t] = s.par ? r0 : r1;
 }
 
 /* The levels lb.. in block 0's shared memory: V-cycle from level lb's b (in
  * global memory, from the restriction) to level lb's corrected x (written
- * back to global memory). Block 0 is alone with these levels, so their
- * latency is the whole grid's: with the flags, tests and index divisions of
- * the grid-wide passes they took 20 us a V-cycle of one sweep (n = 128). The
- * coarsest level (at most 32 cells a colour) runs in one warp. With the middle
- * levels' fused residual and restriction, flags read first and level 0's loads
- * requested together, a refined solve at n = 192 went from 8.3 to 6.5 ms, bit
- * for bit the same. */
-__device__ __forceinline__ void mg_block_levels(const MgArgs &mg, unsigned char *smem) {
-  const int t = threadIdx.x, S = blockDim.x;
-  const int last = mg.nlev - 1;
+ * back to global memory). Block 0 is alone with these levels while the grid
+ * waits, so their latency counts whole. Cell by cell, with flags, tests and
+ * index divisions, they took 35 to 45 us of a V-cycle of two sweeps at n =
+ * 128; on lists of cells 17 us. A level has at most 512 segments; the threads
+ * past its last warp skip it, and its barriers count the others alone. */
+__device__ __forceinline__ void mg_block_levels(const MgArgs &mg) {
+  const int t = threadIdx.x, last = mg.nlev - 1;
   const MgLevel &G = mg.lv[mg.lb];
-  const MgBlockLevel T = mg_block_level(mg, smem, mg.lb);
-  for (int e0 = t; e0 < T.ncell; e0 += S * 8) {
-    float bv[8];
+  /* down: the right-hand side and the first red half sweep, 2 nu - 1 more half
+   * sweeps (black first), residuals; the coarsest level's forward and backward
+   * sweeps: 4 coarse_sweeps - 2 alternating half sweeps, black first (the one
+   * that ends the former also starts the latter) */
+  for (int l = mg.lb; l <= last; l++) {
+    const MgBlockLevel L = mg_block_level(mg, l);
+    if (t >= L.act) continue;
+    const bool in = t < L.segs;
+    const MgSeg s = mg_seg(L, in ? t : 0);
+    float4 own[2], b[2], d[2];
+    if (in) {
+      float v[2][4]; /* b of even and odd k */
+      if (l == mg.lb) {
 #pragma unroll
-    for (int u = 0; u < 8; u++) bv[u] = e0 + u * S < T.ncell ? __ldcg(G.b + e0 + u * S) : 0.0f;
+        for (int u = 0; u < 8; u++) {
+          const int k = 8 * s.seg + u;
+          v[u & 1][u >> 1] = k < L.m ? __ldcg(G.b + ((unsigned)s.i * L.m + s.j) * L.m + k) : 0.0f;
+        }
+      } else {
+        /* the mean of the 8 children's residuals, lines in i, then j, then k */
+        const MgBlockLevel F = mg_block_level(mg, l - 1);
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u & 1][u >> 1] = 0.0f;
+        for (int c = 0; c < 4; c++) {
+          const int i = 2 * s.i + (c >> 1), j = 2 * s.j + (c & 1);
+          if (i >= F.m || j >= F.m) continue;
+#pragma unroll
+          for (int h = 0; h < 2; h++) { /* children of cells 4 h .. 4 h + 3 */
+            if (h >= F.ns) continue;
+            const int at = (i * F.m + j) * F.ns + h;
+            const float4 e = F.r[0][at], o = F.r[1][at];
+            const float ev[4] = {e.x, e.y, e.z, e.w}, ov[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+              float &sum = v[q & 1][2 * h + (q >> 1)];
+              sum += ev[q];
+              sum += ov[q];
+            }
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u & 1][u >> 1] *= 0.125f;
+      }
+      const float4 ve = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]),
+                   vo = make_float4(v[1][0], v[1][1], v[1][2], v[1][3]);
+      b[0] = s.par ? vo : ve;
+      b[1] = s.par ? ve : vo;
+      d[0] = L.d[0][t];
+      d[1] = L.d[1][t];
+      L.b[0][t] = b[0];
+      L.b[1][t] = b[1];
+      own[0] = make_float4(__fdividef(b[0].x * L.ihs, d[0].x), __fdividef(b[0].y * L.ihs, d[0].y),
+                           __fdividef(b[0].z * L.ihs, d[0].z), __fdividef(b[0].w * L.ihs, d[0].w));
+      own[1] = make_float4(0, 0, 0, 0);
+      L.x[0][s.at] = own[0];
+      L.x[1][s.at] = own[1];
+    }
+    mg_bar(L);
+    const int halves = l == last ? 4 * mg.coarse_sweeps - 2 : 2 * mg.nu - 1;
+    for (int h = 0; h < halves; h++) {
+      if (in) {
+        if (h & 1)
+          mg_block_half<0>(L, s, b[0], d[0], own);
+        else
+          mg_block_half<1>(L, s, b[1], d[1], own);
+      }
+      mg_bar(L);
+    }
+    if (l == last) break;
+    if (in) mg_block_residuals(L, s, t, b, d, own);
+    mg_bar(L);
+  }
+  /* up: the parents' corrections, then 2 nu half sweeps, black first */
+  for (int l = last - 1; l >= mg.lb; l--) {
+    const MgBlockLevel L = mg_block_level(mg, l);
+    if (t >= L.act) continue;
+    mg_bar(L); /* the coarser level is done */
+    const bool in = t < L.segs;
+    const MgSeg s = mg_seg(L, in ? t : 0);
+    float4 own[2], b[2], d[2];
+    if (in) {
+      const MgBlockLevel C = mg_block_level(mg, l + 1);
+      const int ci = s.i / 2, cj = s.j / 2;
+      /* cells K = 4 seg .. 4 seg + 3 of the parents' line: two of each colour */
+      const int at = 2 * ((((ci + 1) * (C.m + 2) + cj + 1) * C.ns) * 2 + s.seg);
+      const float2 cr = *reinterpret_cast<const float2 *>(
+          reinterpret_cast<const float *>(C.x[0]) + at);
+      const float2 cb = *reinterpret_cast<const float2 *>(
+          reinterpret_cast<const float *>(C.x[1]) + at);
+      const bool cp = (ci + cj) & 1;
+      const float2 ce = cp ? cb : cr, co = cp ? cr : cb; /* even and odd K */
+      const float4 add = make_float4(ce.x, co.x, ce.y, co.y);
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        b[q] = L.b[q][t];
+        d[q] = L.d[q][t];
+        float4 x = L.x[q][s.at];
+        x.x += d[q].x < INFINITY ? add.x : 0.0f;
+        x.y += d[q].y < INFINITY ? add.y : 0.0f;
+        x.z += d[q].z < INFINITY ? add.z : 0.0f;
+        x.w += d[q].w < INFINITY ? add.w : 0.0f;
+        L.x[q][s.at] = own[q] = x;
+      }
+    }
+    mg_bar(L);
+    for (int h = 0; h < 2 * mg.nu; h++) {
+      if (in) {
+        if (h & 1)
+          mg_block_half<0>(L, s, b[0], d[0], own);
+        else
+          mg_block_half<1>(L, s, b[1], d[1], own);
+      }
+      mg_bar(L);
+    }
+  }
+  const MgBlockLevel T = mg_block_level(mg, mg.lb);
+  if (t < T.segs) {
+    const MgSeg s = mg_seg(T, t);
+    const float4 x0 = T.x[s.par][s.at], x1 = T.x[s.par ^ 1][s.at]; /* even and odd k */
+    const float v[8] = {x0.x, x1.x, x0.y, x1.y, x0.z, x1.z, x0.w, x1.w};
 #pragma unroll
     for (int u = 0; u < 8; u++) {
-      const int e = e0 + u * S;
-      if (e >= T.ncell) continue;
-      const int w = T.slot[e];
-      T.b[w] = bv[u];
-      T.x[T.at[w]] = w < T.nred ? __fdividef(bv[u] * T.ihs, T.d[w]) : 0.0f;
+      const int k = 8 * s.seg + u;
+      if (k < T.m) G.x[((unsigned)s.i * T.m + s.j) * T.m + k] = v[u];
     }
   }
-  __syncthreads();
-  for (int l = mg.lb; l < last; l++) {
-    const MgBlockLevel L = mg_block_level(mg, smem, l);
-    mg_block_gs(L, 1, t, S);
-    __syncthreads();
-    for (int sw = 1; sw < mg.nu; sw++) {
-      mg_block_gs(L, 0, t, S);
-      __syncthreads();
-      mg_block_gs(L, 1, t, S);
-      __syncthreads();
-    }
-    mg_block_residual(L, t, S);
-    __syncthreads();
-    mg_block_restrict(L, mg_block_level(mg, smem, l + 1), t, S);
-    __syncthreads();
-  }
-  /* coarsest: the first red half sweep is done; the black half sweep that
-   * ends the forward sweeps also starts the backward ones */
-  if (t < 32) {
-    const MgBlockLevel L = mg_block_level(mg, smem, last);
-    mg_block_gs(L, 1, t, 32);
-    __syncwarp();
-    for (int it = 1; it < mg.coarse_sweeps; it++) {
-      mg_block_gs(L, 0, t, 32);
-      __syncwarp();
-      mg_block_gs(L, 1, t, 32);
-      __syncwarp();
-    }
-    for (int it = 0; it < mg.coarse_sweeps; it++) {
-      if (it > 0) {
-        mg_block_gs(L, 1, t, 32);
-        __syncwarp();
-      }
-      mg_block_gs(L, 0, t, 32);
-      __syncwarp();
-    }
-  }
-  __syncthreads();
-  for (int l = last - 1; l >= mg.lb; l--) {
-    const MgBlockLevel L = mg_block_level(mg, smem, l);
-    mg_block_prolong(L, mg_block_level(mg, smem, l + 1), t, S);
-    __syncthreads();
-    for (int sw = 0; sw < mg.nu; sw++) {
-      mg_block_gs(L, 1, t, S);
-      __syncthreads();
-      mg_block_gs(L, 0, t, S);
-      __syncthreads();
-    }
-  }
-  for (int e = t; e < T.ncell; e += S) G.x[e] = T.x[T.at[T.slot[e]]];
 }
 
-/* Level-0 phases on quads of the liquid chunks. */
+/* A middle level's smoothing in one pass: each tile of 8^3 cells works in
+ * shared memory on the 16^3 cells around it, stored as a block level's. A half
+ * sweep and the residual each reach one cell further, so four of them leave
+ * the tile's own cells exact, with the values the grid-wide half sweeps would
+ * give them (nu <= 2: three half sweeps and the residual down, four half
+ * sweeps up). One grid barrier instead of four down and five up: at n = 128 a
+ * grid-wide phase of the 32^3 level took 1.7 us and its barrier 1.3 us. Tiles
+ * without liquid are left out (mg_tile_lists). */
+__host__ __device__ inline unsigned mg_tiles_of(int m) {
+  const unsigned t = (unsigned)(m + MG_TILE - 1) / MG_TILE;
+  return t * t * t;
+}
+
+/* the tile's segments in the shared memory before block 0's levels */
+__device__ __forceinline__ MgBlockLevel mg_tile_level(const MgLevel &G) {
+  MgBlockLevel B;
+  B.m = MG_REGION;
+  B.ns = 2;
+  B.segs = B.act = MG_TILE_LINES;
+  B.id = 0;
+  B.hs = G.hs;
+  B.ihs = G.ihs;
+  B.x[0] = mg_smem;
+  B.x[1] = mg_smem + MG_TILE_PLINES;
+  B.r[0] = B.x[1] + MG_TILE_PLINES;
+  B.r[1] = B.r[0] + MG_TILE_LINES;
+  B.b[0] = B.b[1] = B.d[0] = B.d[1] = nullptr;
+  return B;
+}
+
+/* a thread's segment of the region of tile t and its cells in the level */
+struct MgTileSeg {
+  MgSeg s;
+  int i, j, k; /* the level's coordinates of its first cell */
+  int line;    /* index of cell (i, j, 0), or -1 outside the level */
+};
+__device__ __forceinline__ MgTileSeg mg_tile_seg(const MgBlockLevel &L, int m, unsigned t) {
+  MgTileSeg q;
+  const unsigned nt = (unsigned)(m + MG_TILE - 1) / MG_TILE;
+  const int ti = (int)(t / (nt * nt)), tj = (int)(t / nt % nt), tk = (int)(t % nt);
+  q.s = mg_seg(L, threadIdx.x);
+  q.i = ti * MG_TILE - MG_HALO + q.s.i;
+  q.j = tj * MG_TILE - MG_HALO + q.s.j;
+  q.k = tk * MG_TILE - MG_HALO + 8 * q.s.seg;
+  q.line = q.i >= 0 && q.i < m && q.j >= 0 && q.j < m ? (q.i * m + q.j) * m : -1;
+  return q;
+}
+
+/* the segment's eight values of f as those of even and of odd k, `out` outside */
+__device__ __forceinline__ void mg_tile_load(const float *f, const MgTileSeg &q, int m, float out,
+                                             float4 &e, float4 &o) {
+  float v[8];
+  if ((m & 3) == 0) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int k = q.k + 4 * h;
+      const float4 w = q.line >= 0 && k >= 0 && k < m
+                           ? __ldcg(reinterpret_cast<const float4 *>(f + q.line + k))
+                           : make_float4(out, out, out, out);
+      v[4 * h] = w.x;
+      v[4 * h + 1] = w.y;
+      v[4 * h + 2] = w.z;
+      v[4 * h + 3] = w.w;
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+      v[u] = q.line >= 0 && q.k + u >= 0 && q.k + u < m ? __ldcg(f + q.line + q.k + u) : out;
+  }
+  e = make_float4(v[0], v[2], v[4], v[6]);
+  o = make_float4(v[1], v[3], v[5], v[7]);
+}
+
+/* right-hand side and diagonal of the segment by colour; the level's diagonal
+ * is 0 off the liquid */
+__device__ __forceinline__ void mg_tile_system(const MgLevel &G, const MgTileSeg &q, float4 (&b)[2],
+                                               float4 (&d)[2]) {
+  float4 be, bo, de, dod;
+  mg_tile_load(G.b, q, G.m, 0.0f, be, bo);
+  mg_tile_load(G.diag, q, G.m, 0.0f, de, dod);
+  auto off = [](float &v) { v = v == 0.0f ? INFINITY : v; };
+  off(de.x); off(de.y); off(de.z); off(de.w);
+  off(dod.x); off(dod.y); off(dod.z); off(dod.w);
+  b[0] = q.s.par ? bo : be;
+  b[1] = q.s.par ? be : bo;
+  d[0] = q.s.par ? dod : de;
+  d[1] = q.s.par ? de : dod;
+}
+
+/* the tile's own four cells of the segment to f */
+__device__ __forceinline__ void mg_tile_store(float *f, const MgLevel &G, const MgTileSeg &q,
+                                              const float4 (&own)[2]) {
+  const int lo = MG_HALO, hi = MG_HALO + MG_TILE;
+  if (q.s.i < lo || q.s.i >= hi || q.s.j < lo || q.s.j >= hi || q.line < 0) return;
+  const float4 e = q.s.par ? own[1] : own[0], o = q.s.par ? own[0] : own[1];
+  const int k = q.k + (q.s.seg ? 0 : 4);
+  const float4 w = q.s.seg ? make_float4(e.x, o.x, e.y, o.y) : make_float4(e.z, o.z, e.w, o.w);
+  float *x = f + q.line + k;
+  if ((G.m & 3) == 0) {
+    if (k < G.m) *reinterpret_cast<float4 *>(x) = w;
+  } else {
+    if (k < G.m) x[0] = w.x;
+    if (k + 1 < G.m) x[1] = w.y;
+    if (k + 2 < G.m) x[2] = w.z;
+    if (k + 3 < G.m) x[3] = w.w;
+  }
+}
+
+/* the tiles of level l with liquid, in any order: *count of them in list */
+__device__ __forceinline__ void mg_tile_lists(const MgArgs &mg) {
+  for (int l = 1; l < mg.lb; l++) {
+    const MgLevel &G = mg.lv[l];
+    const int m = G.m, nt = (m + MG_TILE - 1) / MG_TILE;
+    for (unsigned t = blockIdx.x; t < mg_tiles_of(m); t += gridDim.x) {
+      const int i = (int)(t / (unsigned)(nt * nt)) * MG_TILE + (threadIdx.x >> 6),
+                j = (int)(t / (unsigned)nt % (unsigned)nt) * MG_TILE + (threadIdx.x >> 3 & 7),
+                k = (int)(t % (unsigned)nt) * MG_TILE + (threadIdx.x & 7);
+      const bool liquid = i < m && j < m && k < m &&
+                          __ldg(G.flags + ((unsigned)i * m + j) * m + k) == CELL_FLUID;
+      if (__syncthreads_or(liquid) && threadIdx.x == 0) G.tiles[atomicAdd(G.ntiles, 1u)] = t;
+    }
+  }
+}
+
+/* pre-smoothing from x = 0, residual and restriction of a middle level */
+__device__ __forceinline__ void mg_tile_down(const MgArgs &mg, int l) {
+  const MgLevel &F = mg.lv[l], &Cl = mg.lv[l + 1];
+  const MgBlockLevel L = mg_tile_level(F);
+  const unsigned count = __ldcg(F.ntiles);
+  for (unsigned w = blockIdx.x; w < count; w += gridDim.x) {
+    const unsigned t = __ldcg(F.tiles + w);
+    const MgTileSeg q = mg_tile_seg(L, F.m, t);
+    float4 own[2], b[2], d[2];
+    mg_tile_system(F, q, b, d);
+    own[0] = make_float4(__fdividef(b[0].x * L.ihs, d[0].x), __fdividef(b[0].y * L.ihs, d[0].y),
+                         __fdividef(b[0].z * L.ihs, d[0].z), __fdividef(b[0].w * L.ihs, d[0].w));
+    own[1] = make_float4(0, 0, 0, 0);
+    __syncthreads(); /* the previous tile's restriction is done */
+    L.x[0][q.s.at] = own[0];
+    L.x[1][q.s.at] = own[1];
+    __syncthreads();
+    for (int h = 1; h < 2 * mg.nu; h++) {
+      if (h & 1)
+        mg_block_half<1>(L, q.s, b[1], d[1], own);
+      else
+        mg_block_half<0>(L, q.s, b[0], d[0], own);
+      __syncthreads();
+    }
+    mg_tile_store(F.x, F, q, own);
+    mg_block_residuals(L, q.s, threadIdx.x, b, d, own);
+    __syncthreads();
+    /* the tile's 4^3 coarse cells */
+    if (threadIdx.x < 64) {
+      const unsigned nt = (unsigned)(F.m + MG_TILE - 1) / MG_TILE;
+      const int a = threadIdx.x >> 4, c = threadIdx.x >> 2 & 3, e = threadIdx.x & 3;
+      const int I = (int)(t / (nt * nt)) * 4 + a, J = (int)(t / nt % nt) * 4 + c,
+                K = (int)(t % nt) * 4 + e;
+      if (I < Cl.m && J < Cl.m && K < Cl.m) {
+        float sum = 0.0f;
+#pragma unroll
+        for (int x = 0; x < 2; x++)
+#pragma unroll
+          for (int y = 0; y < 2; y++) {
+            const int at = ((MG_HALO + 2 * a + x) * MG_REGION + MG_HALO + 2 * c + y) * 8 +
+                           MG_HALO / 2 + e;
+            sum += reinterpret_cast<const float *>(L.r[0])[at];
+            sum += reinterpret_cast<const float *>(L.r[1])[at];
+          }
+        const unsigned cc = ((unsigned)I * Cl.m + J) * Cl.m + K;
+        mg_coarse_start(Cl, cc, ((I + J + K) & 1) == 0 && __ldg(Cl.flags + cc) == CELL_FLUID, sum);
+      }
+    }
+  }
+}
+
+/* prolongation to and post-smoothing of a middle level: from x to out, since
+ * the tiles around read x meanwhile */
+__device__ __forceinline__ void mg_tile_up(const MgArgs &mg, int l) {
+  const MgLevel &F = mg.lv[l], &Cl = mg.lv[l + 1];
+  const MgBlockLevel L = mg_tile_level(F);
+  const unsigned count = __ldcg(F.ntiles);
+  for (unsigned w = blockIdx.x; w < count; w += gridDim.x) {
+    const MgTileSeg q = mg_tile_seg(L, F.m, __ldcg(F.tiles + w));
+    float4 own[2], b[2], d[2], xe, xo;
+    mg_tile_load(F.x, q, F.m, 0.0f, xe, xo);
+    float p[4]; /* the parents' x */
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int k = q.k + 2 * u;
+      p[u] = q.line >= 0 && k >= 0 && k < F.m
+                 ? __ldcg(Cl.out + ((unsigned)(q.i >> 1) * Cl.m + (q.j >> 1)) * Cl.m + (k >> 1))
+                 : 0.0f;
+    }
+    mg_tile_system(F, q, b, d);
+    own[0] = q.s.par ? xo : xe;
+    own[1] = q.s.par ? xe : xo;
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      own[c].x += d[c].x < INFINITY ? p[0] : 0.0f;
+      own[c].y += d[c].y < INFINITY ? p[1] : 0.0f;
+      own[c].z += d[c].z < INFINITY ? p[2] : 0.0f;
+      own[c].w += d[c].w < INFINITY ? p[3] : 0.0f;
+    }
+    __syncthreads();
+    L.x[0][q.s.at] = own[0];
+    L.x[1][q.s.at] = own[1];
+    __syncthreads();
+    for (int h = 0; h < 2 * mg.nu; h++) {
+      if (h & 1)
+        mg_block_half<0>(L, q.s, b[0], d[0], own);
+      else
+        mg_block_half<1>(L, q.s, b[1], d[1], own);
+      __syncthreads();
+    }
+    mg_tile_store(F.out, F, q, own);
+  }
+}
+
+/* Level-0 phases on quads of the liquid chunks. The fields that a phase reads
+ * at neighbours are loaded through L1 (plain loads: the barrier before the
+ * phase orders them after the other SMs' writes): the lines j - 1 and j + 1
+ * belong to chunks that the block's other warps walk at the same time, and
+ * the phases of large grids are bound by L2 bandwidth. */
 /* MG_BLACK_PROLONG: the black half sweep after the coarse correction, with
  * the prolongation folded in: every value is read as z plus the parent's
  * correction, and only the black cells are written (the red cells keep
  * their uncorrected z, which the neighbours of this phase read and correct
  * themselves; the red half sweep that follows overwrites every red cell). */
-enum MgPhase { MG_MATVEC, MG_UPDATE, MG_BLACK, MG_RES, MG_RED_DOT, MG_BLACK_PROLONG, MG_RED };
+enum MgPhase { MG_MATVEC, MG_UPDATE, MG_HALF, MG_BLACK_PROLONG };
 
+/* MG_HALF: the half sweep of `color`; with dot it also sums r.z */
 template <int PH, int BLOCK>
 __device__ __forceinline__ void mg_quads(const CgArgs &a, float alpha, float beta, const float *pold,
-                                         float *pnew, FF &acc0) {
+                                         float *pnew, int color, bool dot, FF &acc0) {
   const int n = a.s.n, qrow = n / 4;
   const size_t qplane = (size_t)qrow * n, nq = a.nc / 4;
   const size_t warps = (size_t)gridDim.x * (BLOCK / 32);
@@ -1827,6 +2103,8 @@ __device__ __forceinline__ void mg_quads(const CgArgs &a, float alpha, float bet
   const uchar4 *A4p = reinterpret_cast<const uchar4 *>(a.A);
   const float4 *d4p = reinterpret_cast<const float4 *>(a.diag);
   float *zf = L0.x, *rf = a.r;
+  const float4 *z4p = reinterpret_cast<const float4 *>(zf);
+  const float4 *o4p = reinterpret_cast<const float4 *>(pold);
   const float4 zero = make_float4(0, 0, 0, 0);
   const unsigned nact = __ldcg(a.chunk_count);
   unsigned cnext = wid < nact ? __ldg(a.chunk_list + wid) : 0u;
@@ -1843,8 +2121,7 @@ __device__ __forceinline__ void mg_quads(const CgArgs &a, float alpha, float bet
     const uchar4 A4 = A4p[qs];
     const bool fv[4] = {fl(A4.x), fl(A4.y), fl(A4.z), fl(A4.w)};
     const int par0 = (i + j + k0) & 1; /* colour of the quad's first cell */
-    constexpr bool NB = PH == MG_MATVEC || PH == MG_BLACK || PH == MG_RES || PH == MG_RED_DOT ||
-                        PH == MG_BLACK_PROLONG || PH == MG_RED;
+    constexpr bool NB = PH != MG_UPDATE;
     /* the field whose neighbours are summed: p' = z + beta p (MATVEC) or z */
     float4 own = zero, own0 = zero; /* own0: as loaded, before any correction */
     float4 nbq[4] = {zero, zero, zero, zero};
@@ -1865,29 +2142,29 @@ __device__ __forceinline__ void mg_quads(const CgArgs &a, float alpha, float bet
       q4 = __ldcg(reinterpret_cast<const float4 *>(a.q) + qs);
     }
     if (PH == MG_MATVEC) {
-      const float4 z4 = __ldcg(reinterpret_cast<const float4 *>(zf) + qs);
-      const float4 p4 = __ldcg(reinterpret_cast<const float4 *>(pold) + qs);
+      const float4 z4 = z4p[qs];
+      const float4 p4 = o4p[qs];
       own = make_float4(z4.x + beta * p4.x, z4.y + beta * p4.y, z4.z + beta * p4.z,
                         z4.w + beta * p4.w);
 #pragma unroll
       for (int d = 0; d < 4; d++)
         if (has[d]) {
           const size_t qq = (size_t)((long)qs + off[d]);
-          const float4 zn = __ldcg(reinterpret_cast<const float4 *>(zf) + qq);
-          const float4 pn = __ldcg(reinterpret_cast<const float4 *>(pold) + qq);
+          const float4 zn = z4p[qq];
+          const float4 pn = o4p[qq];
           nbq[d] = make_float4(zn.x + beta * pn.x, zn.y + beta * pn.y, zn.z + beta * pn.z,
                                zn.w + beta * pn.w);
         }
-      if (ed) edge = __ldcg(zf + ce) + beta * __ldcg(pold + ce);
+      if (ed) edge = zf[ce] + beta * pold[ce];
     } else {
-      if (NB) own = __ldcg(reinterpret_cast<const float4 *>(zf) + qs);
+      if (NB) own = z4p[qs];
       own0 = own;
       if (NB) {
 #pragma unroll
         for (int d = 0; d < 4; d++)
           if (has[d])
-            nbq[d] = __ldcg(reinterpret_cast<const float4 *>(zf) + (size_t)((long)qs + off[d]));
-        if (ed) edge = __ldcg(zf + ce);
+            nbq[d] = z4p[(size_t)((long)qs + off[d])];
+        if (ed) edge = zf[ce];
       }
       if (PH == MG_BLACK_PROLONG) {
         /* add the parents' corrections on the liquid (level 1 holds them) */
@@ -1896,7 +2173,7 @@ __device__ __forceinline__ void mg_quads(const CgArgs &a, float alpha, float bet
         auto par2 = [&](int ii, int jj) {
           const unsigned idx = (((unsigned)ii >> 1) * m1 + ((unsigned)jj >> 1)) * m1 +
                                (unsigned)(k0 >> 1);
-          return __ldcg(reinterpret_cast<const float2 *>(L1.x + idx));
+          return *reinterpret_cast<const float2 *>(L1.out + idx);
         };
         auto add = [](float4 &v, uchar4 f, float2 e) {
           v.x += fl(f.x) ? e.x : 0.0f;
@@ -1913,7 +2190,7 @@ __device__ __forceinline__ void mg_quads(const CgArgs &a, float alpha, float bet
           const int ke = lane == 0 ? k0 - 1 : k0 + 4;
           const unsigned idx =
               (((unsigned)i >> 1) * m1 + ((unsigned)j >> 1)) * m1 + (unsigned)(ke >> 1);
-          if (fl(a.A[ce])) edge += __ldcg(L1.x + idx);
+          if (fl(a.A[ce])) edge += L1.out[idx];
         }
       }
     }
@@ -1968,14 +2245,7 @@ __device__ __forceinline__ void mg_quads(const CgArgs &a, float alpha, float bet
       reinterpret_cast<float4 *>(a.x)[q] = make_float4(xn[0], xn[1], xn[2], xn[3]);
       reinterpret_cast<float4 *>(rf)[q] = make_float4(rn[0], rn[1], rn[2], rn[3]);
       reinterpret_cast<float4 *>(zf)[q] = make_float4(zn[0], zn[1], zn[2], zn[3]);
-    } else if (PH == MG_RES) {
-      const float rv[4] = {r4.x, r4.y, r4.z, r4.w}, dv[4] = {dg.x, dg.y, dg.z, dg.w};
-      float res[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) res[u] = fv[u] ? rv[u] - hs * (dv[u] * ov[u] - nbs[u]) : 0.0f;
-      reinterpret_cast<float4 *>(L0.res)[q] = make_float4(res[0], res[1], res[2], res[3]);
-    } else { /* MG_BLACK, MG_BLACK_PROLONG, MG_RED, MG_RED_DOT: half sweep of one colour */
-      const int color = (PH == MG_RED_DOT || PH == MG_RED) ? 0 : 1;
+    } else { /* half sweep of one colour */
       const float rv[4] = {r4.x, r4.y, r4.z, r4.w}, dv[4] = {dg.x, dg.y, dg.z, dg.w};
       const float o0[4] = {own0.x, own0.y, own0.z, own0.w};
       float zn[4];
@@ -1983,10 +2253,90 @@ __device__ __forceinline__ void mg_quads(const CgArgs &a, float alpha, float bet
       for (int u = 0; u < 4; u++) {
         zn[u] = o0[u];
         if (fv[u] && ((par0 + u) & 1) == color) zn[u] = __fdividef(rv[u] * ihs + nbs[u], dv[u]);
-        if (PH == MG_RED_DOT && fv[u]) ff_add_prod(acc0, rv[u], zn[u]);
+        if (PH == MG_HALF && dot && fv[u]) ff_add_prod(acc0, rv[u], zn[u]);
       }
       reinterpret_cast<float4 *>(zf)[q] = make_float4(zn[0], zn[1], zn[2], zn[3]);
     }
+  }
+}
+
+/* Level 0's residual r - A z and its restriction in one pass: a thread takes
+ * the quad k0 .. k0 + 3 of the four lines 2 I .. 2 I + 1, 2 J .. 2 J + 1, the
+ * children of two coarse cells (n % 4 == 0, so every line is there). */
+__device__ __forceinline__ void mg0_residual_restrict(const CgArgs &a, unsigned start,
+                                                      unsigned stride) {
+  const MgLevel &F = a.mg.lv[0], &Cl = a.mg.lv[1];
+  const int n = a.s.n, m1 = n / 2;
+  const unsigned qrow = (unsigned)n / 4, tot = (unsigned)m1 * m1 * qrow;
+  const float4 *z4 = reinterpret_cast<const float4 *>(F.x);
+  const float4 zero = make_float4(0, 0, 0, 0);
+  for (unsigned t = start; t < tot; t += stride) {
+    const unsigned row = t / qrow, q = t - row * qrow;
+    const int I = (int)(row / (unsigned)m1), J = (int)(row - (unsigned)I * m1);
+    const unsigned c = row * m1 + 2 * q;
+    const uchar2 cf = __ldg(reinterpret_cast<const uchar2 *>(Cl.flags + c));
+    if (!(fl(cf.x) || fl(cf.y))) continue; /* b and x are zero since the start */
+    float sum0 = 0.0f, sum1 = 0.0f;
+    {
+      const int i0 = 2 * I, j0 = 2 * J;
+      const long q0 = ((long)i0 * n + j0) * qrow + q; /* quad of line (i0, j0) */
+      const long qi = (long)n * qrow, qj = qrow;
+      float4 z[4][4]; /* lines i0 - 1 .. i0 + 2, j0 - 1 .. j0 + 2, no corners */
+      float lo[2][2], hi[2][2];
+#pragma unroll
+      for (int a4 = 0; a4 < 4; a4++)
+#pragma unroll
+        for (int b4 = 0; b4 < 4; b4++) {
+          if ((a4 == 0 || a4 == 3) && (b4 == 0 || b4 == 3)) continue;
+          const int i = i0 + a4 - 1, j = j0 + b4 - 1;
+          z[a4][b4] = i >= 0 && i < n && j >= 0 && j < n ? z4[q0 + (a4 - 1) * qi + (b4 - 1) * qj]
+                                                         : zero;
+        }
+      float4 r4[2][2], d4[2][2];
+      uchar4 f4[2][2];
+#pragma unroll
+      for (int x = 0; x < 2; x++)
+#pragma unroll
+        for (int y = 0; y < 2; y++) {
+          const long qq = q0 + x * qi + y * qj;
+          r4[x][y] = __ldcg(reinterpret_cast<const float4 *>(a.r) + qq);
+          d4[x][y] = __ldg(reinterpret_cast<const float4 *>(a.diag) + qq);
+          f4[x][y] = __ldg(reinterpret_cast<const uchar4 *>(a.A) + qq);
+          lo[x][y] = q > 0 ? F.x[4 * qq - 1] : 0.0f;
+          hi[x][y] = q + 1 < qrow ? F.x[4 * qq + 4] : 0.0f;
+        }
+#pragma unroll
+      for (int x = 0; x < 2; x++)
+#pragma unroll
+        for (int y = 0; y < 2; y++) {
+          const float4 o = z[x + 1][y + 1], ip = z[x + 2][y + 1], im = z[x][y + 1],
+                       jp = z[x + 1][y + 2], jm = z[x + 1][y];
+          const float ov[4] = {o.x, o.y, o.z, o.w}, kl[4] = {lo[x][y], o.x, o.y, o.z},
+                      kr[4] = {o.y, o.z, o.w, hi[x][y]};
+          const float n0[4] = {ip.x, ip.y, ip.z, ip.w}, n1[4] = {im.x, im.y, im.z, im.w};
+          const float n2[4] = {jp.x, jp.y, jp.z, jp.w}, n3[4] = {jm.x, jm.y, jm.z, jm.w};
+          const float rv[4] = {r4[x][y].x, r4[x][y].y, r4[x][y].z, r4[x][y].w};
+          const float dv[4] = {d4[x][y].x, d4[x][y].y, d4[x][y].z, d4[x][y].w};
+          const bool fv[4] = {fl(f4[x][y].x), fl(f4[x][y].y), fl(f4[x][y].z), fl(f4[x][y].w)};
+          float res[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            const float nbs = ((((n0[u] + n1[u]) + n2[u]) + n3[u]) + kl[u]) + kr[u];
+            res[u] = fv[u] ? rv[u] - F.hs * (dv[u] * ov[u] - nbs) : 0.0f;
+          }
+          sum0 += res[0];
+          sum0 += res[1];
+          sum1 += res[2];
+          sum1 += res[3];
+        }
+    }
+    const bool even = ((I + J) & 1) == 0; /* K = 2 q is red, else K = 2 q + 1 */
+    const float2 d2 = __ldg(reinterpret_cast<const float2 *>(Cl.diag + c));
+    const float b0 = sum0 * 0.125f, b1 = sum1 * 0.125f;
+    *reinterpret_cast<float2 *>(Cl.b + c) = make_float2(b0, b1);
+    *reinterpret_cast<float2 *>(Cl.x + c) =
+        make_float2(even && fl(cf.x) ? __fdividef(b0 * Cl.ihs, d2.x) : 0.0f,
+                    !even && fl(cf.y) ? __fdividef(b1 * Cl.ihs, d2.y) : 0.0f);
   }
 }
 
@@ -2002,16 +2352,36 @@ template <int BLOCK> __global__ void __launch_bounds__(BLOCK, 1) k_cg_mg(CgArgs 
   const int lane = threadIdx.x & 31;
   float4 *x4 = reinterpret_cast<float4 *>(a.x);
   const float4 *b4 = reinterpret_cast<const float4 *>(a.b);
-  const MgArgs &mg = a.mg;
+  /* the levels in shared memory: indexed by a variable, the kernel's arguments
+   * would be copied to local memory, whose lines every barrier's acquire drops
+   * from L1 (a round trip to L2 in every phase) */
+  __shared__ MgArgs mg;
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int l = 0; l < MG_MAX_LEVELS; l++) mg.lv[l] = a.mg.lv[l];
+    mg.nlev = a.mg.nlev;
+    mg.lb = a.mg.lb;
+    mg.coarse_sweeps = a.mg.coarse_sweeps;
+    mg.nu = a.mg.nu;
+  }
+  __syncthreads();
   const unsigned gt = blockIdx.x * BLOCK + threadIdx.x, gs = nb * BLOCK;
   unsigned epoch = 0;
   __shared__ float s_alpha, s_beta;
   __shared__ int s_done;
-  extern __shared__ __align__(16) unsigned char mg_smem[];
 
   /* block 0: its levels' lists and diagonals into shared memory (fixed
    * during the solve) */
-  if (blockIdx.x == 0) mg_block_init(mg, mg_smem);
+  if (blockIdx.x == 0) mg_block_init(mg);
+  /* the tiles of the middle levels; x and b are zero outside them */
+  const bool tiled = mg.nu <= MG_TILE_NU;
+  static_assert(BLOCK == MG_TILE_LINES, "a thread a segment, and a cell of a tile");
+  for (int e = threadIdx.x; e < 2 * MG_TILE_PLINES; e += BLOCK) mg_smem[e] = make_float4(0, 0, 0, 0);
+  if (tiled) mg_tile_lists(mg);
+  for (int l = 1; l < mg.lb + 1; l++) {
+    const unsigned c = (unsigned)mg.lv[l].m * mg.lv[l].m * mg.lv[l].m;
+    for (unsigned e = gt; e < c; e += gs) mg.lv[l].x[e] = mg.lv[l].b[e] = 0.0f;
+  }
 
   /* phase 0: r = b - A x on the liquid (x zeroed elsewhere); b.b, r.r */
   FF pbb = ff_zero(), prr = ff_zero();
@@ -2070,136 +2440,110 @@ template <int BLOCK> __global__ void __launch_bounds__(BLOCK, 1) k_cg_mg(CgArgs 
   __syncthreads();
   done = s_done;
 
-  /* z = V-cycle(r) after the level-0 first red half sweep (MG_UPDATE);
-   * the final red half sweep accumulates r.z */
-  auto vcycle_rest = [&](FF &prz) -> bool {
-    FF none = ff_zero();
-    mg_quads<MG_BLACK, BLOCK>(a, 0.0f, 0.0f, nullptr, nullptr, none);
-    if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-    for (int sw = 1; sw < mg.nu; sw++) {
-      mg_quads<MG_RED, BLOCK>(a, 0.0f, 0.0f, nullptr, nullptr, none);
-      if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-      mg_quads<MG_BLACK, BLOCK>(a, 0.0f, 0.0f, nullptr, nullptr, none);
-      if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-    }
-    mg_quads<MG_RES, BLOCK>(a, 0.0f, 0.0f, nullptr, nullptr, none);
-    if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-    mg_restrict(mg.lv[0], mg.lv[1], gt, gs);
-    if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-    for (int l = 1; l < mg.lb; l++) {
-      mg_gs(mg.lv[l], 1, gt, gs);
-      if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-      for (int sw = 1; sw < mg.nu; sw++) {
-        mg_gs(mg.lv[l], 0, gt, gs);
-        if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-        mg_gs(mg.lv[l], 1, gt, gs);
-        if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-      }
-      mg_residual_restrict(mg.lv[l], mg.lv[l + 1], gt, gs);
-      if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-    }
-    if (blockIdx.x == 0) mg_block_levels(mg, mg_smem);
-    if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-    for (int l = mg.lb - 1; l >= 1; l--) {
-      mg_prolong(mg.lv[l], mg.lv[l + 1], gt, gs);
-      if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-      mg_gs(mg.lv[l], 1, gt, gs);
-      if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-      mg_gs(mg.lv[l], 0, gt, gs);
-      if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-      for (int sw = 1; sw < mg.nu; sw++) {
-        mg_gs(mg.lv[l], 1, gt, gs);
-        if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-        mg_gs(mg.lv[l], 0, gt, gs);
-        if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-      }
-    }
-    mg_quads<MG_BLACK_PROLONG, BLOCK>(a, 0.0f, 0.0f, nullptr, nullptr, none);
-    if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-    for (int sw = 1; sw < mg.nu; sw++) {
-      mg_quads<MG_RED, BLOCK>(a, 0.0f, 0.0f, nullptr, nullptr, none);
-      if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-      mg_quads<MG_BLACK, BLOCK>(a, 0.0f, 0.0f, nullptr, nullptr, none);
-      if (!count_barrier(a.bar, epoch, a.iflags)) return false;
-    }
-    mg_quads<MG_RED_DOT, BLOCK>(a, 0.0f, 0.0f, nullptr, nullptr, prz);
-    return true;
-  };
-
+  /* The iterations. Each pass of the loop below is written once (the first
+   * iteration starts at the update with alpha = 0, P and q being zero on
+   * entry), and so is each phase of the V-cycle inside it: the phases are
+   * short, and a second copy's instructions would be fetched anew. */
   float *P[2] = {a.p, a.p2};
   int pc = 0; /* P[pc]: the previous direction (zero before the first) */
-  if (!done) {
-    FF none = ff_zero(), prz = ff_zero();
-    /* with alpha = 0 the update pass only starts the V-cycle (P and q are
-     * zero on entry) */
-    mg_quads<MG_UPDATE, BLOCK>(a, 0.0f, 0.0f, P[0], P[1], none);
-    if (!count_barrier(a.bar, epoch, a.iflags)) return;
-    if (!vcycle_rest(prz)) return;
-    {
-      FF v[1] = {prz};
-      store_partials<1, BLOCK>(a.part, 2, nb, v);
-    }
-    if (!count_barrier(a.bar, epoch, a.iflags)) return;
-    if (threadIdx.x < 32) {
-      double t[1];
-      warp_sum_partials<1>(a.part, 2, nb, t);
-      if (threadIdx.x == 0) {
-        rz = t[0];
-        if (!(rz == rz) || !(rz > 0.0)) done = 2;
-        s_done = done;
-      }
-    }
-    __syncthreads();
-    done = s_done;
-  }
-  float beta_f = 0.0f;
-  while (!done) {
-    /* p' = z + beta p, q = A p', p'.q */
-    FF ppq = ff_zero();
-    mg_quads<MG_MATVEC, BLOCK>(a, 0.0f, beta_f, P[pc], P[pc ^ 1], ppq);
-    {
-      FF v[1] = {ppq};
+  float alpha_f = 0.0f, beta_f = 0.0f;
+  for (bool first = true; !done; first = false) {
+    if (!first) {
+      /* p' = z + beta p, q = A p', p'.q */
+      FF v[1] = {ff_zero()};
+      mg_quads<MG_MATVEC, BLOCK>(a, 0.0f, beta_f, P[pc], P[pc ^ 1], 0, false, v[0]);
       store_partials<1, BLOCK>(a.part, 3, nb, v);
-    }
-    if (!count_barrier(a.bar, epoch, a.iflags)) return;
-    if (threadIdx.x < 32) {
-      double t[1];
-      warp_sum_partials<1>(a.part, 3, nb, t);
-      if (threadIdx.x == 0) {
-        alpha = rz / t[0];
-        if (!(alpha == alpha) || !(t[0] > 0.0)) done = 2;
-        s_alpha = (float)alpha;
-        s_done = done;
+      if (!count_barrier(a.bar, epoch, a.iflags)) return;
+      if (threadIdx.x < 32) {
+        double t[1];
+        warp_sum_partials<1>(a.part, 3, nb, t);
+        if (threadIdx.x == 0) {
+          alpha = rz / t[0];
+          if (!(alpha == alpha) || !(t[0] > 0.0)) done = 2;
+          s_alpha = (float)alpha;
+          s_done = done;
+        }
       }
+      __syncthreads();
+      alpha_f = s_alpha;
+      done = s_done;
+      if (done) break;
     }
-    __syncthreads();
-    done = s_done;
-    if (done) break;
-    /* x += alpha p', r -= alpha q, r.r; the V-cycle's first half sweep */
-    FF prr2 = ff_zero();
-    mg_quads<MG_UPDATE, BLOCK>(a, s_alpha, 0.0f, P[pc], P[pc ^ 1], prr2);
     {
-      FF v[1] = {prr2};
+      /* x += alpha p', r -= alpha q, r.r; the V-cycle's first half sweep */
+      FF v[1] = {ff_zero()};
+      mg_quads<MG_UPDATE, BLOCK>(a, alpha_f, 0.0f, P[pc], P[pc ^ 1], 0, false, v[0]);
       store_partials<1, BLOCK>(a.part, 4, nb, v);
+      if (!count_barrier(a.bar, epoch, a.iflags)) return;
     }
-    if (!count_barrier(a.bar, epoch, a.iflags)) return;
-    iters++;
-    if (threadIdx.x < 32) {
-      double t[1];
-      warp_sum_partials<1>(a.part, 4, nb, t);
-      if (threadIdx.x == 0) {
-        e2 = t[0];
-        if (e2 <= eps) done = 1;
-        else if (!(e2 == e2)) done = 2;
-        else if (iters >= a.max_iters) done = 3;
-        s_done = done;
+    if (!first) {
+      iters++;
+      if (threadIdx.x < 32) {
+        double t[1];
+        warp_sum_partials<1>(a.part, 4, nb, t);
+        if (threadIdx.x == 0) {
+          e2 = t[0];
+          if (e2 <= eps) done = 1;
+          else if (!(e2 == e2)) done = 2;
+          else if (iters >= a.max_iters) done = 3;
+          s_done = done;
+        }
       }
+      __syncthreads();
+      done = s_done;
+      if (done) break;
     }
-    __syncthreads();
-    done = s_done;
-    if (done) break;
+    /* z = V-cycle(r) from there; its last red half sweep sums r.z. Down: the
+     * half sweeps h = 1 .. 2 nu - 1 of a level (odd: black), then residual and
+     * restriction; up: prolongation (on level 0 folded into the first half
+     * sweep), then the half sweeps h = 0 .. 2 nu - 1 (even: black) */
     FF prz = ff_zero();
-    if (!vcycle_rest(prz)) return;
+    bool up = false;
+    int l = 0, h = 1;
+    for (;;) {
+      const MgLevel &L = mg.lv[l];
+      if (!up && l == mg.lb) {
+        if (blockIdx.x == 0) mg_block_levels(mg);
+        up = true;
+        l--;
+        h = l == 0 ? 0 : -1;
+      } else if (l > 0 && tiled) {
+        if (up) {
+          mg_tile_up(mg, l);
+          l--;
+          h = 0;
+        } else {
+          mg_tile_down(mg, l);
+          l++;
+        }
+      } else if (!up && h == 2 * mg.nu) {
+        if (l == 0)
+          mg0_residual_restrict(a, gt, gs);
+        else
+          mg_residual_restrict(L, mg.lv[l + 1], gt, gs);
+        l++;
+        h = 1;
+      } else if (up && h < 0) {
+        mg_prolong(L, mg.lv[l + 1], gt, gs);
+        h = 0;
+      } else {
+        const bool last = up && h == 2 * mg.nu - 1;
+        const int color = up ? (h & 1) ^ 1 : h & 1;
+        if (l > 0)
+          mg_gs(L, color, gt, gs);
+        else if (up && h == 0)
+          mg_quads<MG_BLACK_PROLONG, BLOCK>(a, 0.0f, 0.0f, nullptr, nullptr, color, false, prz);
+        else
+          mg_quads<MG_HALF, BLOCK>(a, 0.0f, 0.0f, nullptr, nullptr, color, last, prz);
+        h++;
+        if (last) {
+          if (l == 0) break;
+          l--;
+          h = l == 0 ? 0 : -1;
+        }
+      }
+      if (!count_barrier(a.bar, epoch, a.iflags)) return;
+    }
     {
       FF v[1] = {prz};
       store_partials<1, BLOCK>(a.part, 5, nb, v);
@@ -2210,17 +2554,23 @@ template <int BLOCK> __global__ void __launch_bounds__(BLOCK, 1) k_cg_mg(CgArgs 
       warp_sum_partials<1>(a.part, 5, nb, t);
       if (threadIdx.x == 0) {
         const double rzn = t[0];
-        beta = rzn / rz;
+        if (first) {
+          if (!(rzn == rzn) || !(rzn > 0.0)) done = 2;
+        } else {
+          beta = rzn / rz;
+          if (!(beta == beta)) done = 2;
+          s_beta = (float)beta;
+        }
         rz = rzn;
-        if (!(beta == beta)) done = 2;
-        s_beta = (float)beta;
         s_done = done;
       }
     }
     __syncthreads();
-    beta_f = s_beta;
     done = s_done;
-    pc ^= 1;
+    if (!first) {
+      beta_f = s_beta;
+      pc ^= 1;
+    }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.iflags[IF_DONE] = done;
@@ -3210,7 +3560,8 @@ constexpr int MG_COARSE_SWEEPS = 2; /* the iteration count does not depend on it
 constexpr int MG_SWEEPS_DEFAULT = 2; /* measured: 1 -> 2 sweeps cut the solve 11 % at
                                           n=128 and 35 % at n=256; 3 gain nothing */
 constexpr int CG_MG_BLOCK = 512;
-constexpr size_t MG_SMEM_MAX = 128 * 1024; /* block 0's levels: <= 16^3 + 8^3 + 4^3 cells */
+constexpr size_t MG_SMEM_MAX = 128 * 1024; /* a tile, and block 0's levels: <= 16^3 + 8^3 + 4^3
+                                              cells */
 
 /* threads per block of a persistent CG kernel */
 static int cg_block_of(const void *kern) {
@@ -3223,7 +3574,7 @@ static int cg_block_of(const void *kern) {
 
 /* The level sizes (n, ceil(n/2), ... down to at most 4 per axis), the first
  * level solved in block 0 (at most 16^3 cells) and the buffers of levels
- * 1.. plus the level-0 scratch (residual, second direction, A p). */
+ * 1.. plus the level-0 scratch (second direction, A p). */
 int mg_alloc(FlipGpu *h) {
   if (h->mg_nlev > 0) return FLIPGPU_OK;
   int m = h->n, nlev = 0;
@@ -3236,11 +3587,10 @@ int mg_alloc(FlipGpu *h) {
   if (nlev < 2 || lv[nlev - 1] > 4) return FLIPGPU_EINVAL;
   int lb = 1;
   while (lb < nlev - 1 && (size_t)lv[lb] * lv[lb] * lv[lb] > MG_BLOCK_CELLS) lb++;
-  if (nlev - lb > MG_BLOCK_LEVELS || mg_block_bytes(lv, lb, nlev) > MG_SMEM_MAX)
+  if (lv[lb] > MG_BLOCK_MAX || MG_TILE_BYTES + mg_block_bytes(lv, lb, nlev) > MG_SMEM_MAX)
     return FLIPGPU_EINVAL;
   const size_t nc = h->nc;
-  bool ok = cudaMalloc(&h->mg_res[0], nc * sizeof(float)) == cudaSuccess &&
-            cudaMalloc(&h->mg_p2, nc * sizeof(float)) == cudaSuccess &&
+  bool ok = cudaMalloc(&h->mg_p2, nc * sizeof(float)) == cudaSuccess &&
             cudaMalloc(&h->mg_q, nc * sizeof(float)) == cudaSuccess;
   for (int l = 1; ok && l < nlev; l++) {
     const size_t c = (size_t)lv[l] * lv[l] * lv[l];
@@ -3248,7 +3598,8 @@ int mg_alloc(FlipGpu *h) {
          cudaMalloc(&h->mg_diag[l], c * sizeof(float)) == cudaSuccess &&
          cudaMalloc(&h->mg_x[l], c * sizeof(float)) == cudaSuccess &&
          cudaMalloc(&h->mg_b[l], c * sizeof(float)) == cudaSuccess &&
-         cudaMalloc(&h->mg_res[l], c * sizeof(float)) == cudaSuccess;
+         (l >= lb || cudaMalloc(&h->mg_y[l], c * sizeof(float)) == cudaSuccess) &&
+         cudaMalloc(&h->mg_tiles[l], mg_tiles_of(lv[l]) * sizeof(unsigned)) == cudaSuccess;
   }
   if (!ok) {
     mg_free(h);
@@ -3266,9 +3617,12 @@ void mg_free(FlipGpu *h) {
     if (h->mg_diag[l]) cudaFree(h->mg_diag[l]);
     if (h->mg_x[l]) cudaFree(h->mg_x[l]);
     if (h->mg_b[l]) cudaFree(h->mg_b[l]);
-    if (h->mg_res[l]) cudaFree(h->mg_res[l]);
+    if (h->mg_y[l]) cudaFree(h->mg_y[l]);
+    if (h->mg_tiles[l]) cudaFree(h->mg_tiles[l]);
+    h->mg_y[l] = nullptr;
+    h->mg_tiles[l] = nullptr;
     h->mg_flags[l] = nullptr;
-    h->mg_diag[l] = h->mg_x[l] = h->mg_b[l] = h->mg_res[l] = nullptr;
+    h->mg_diag[l] = h->mg_x[l] = h->mg_b[l] = nullptr;
   }
   if (h->mg_p2) cudaFree(h->mg_p2);
   if (h->mg_q) cudaFree(h->mg_q);
@@ -3471,7 +3825,7 @@ int run_solve(FlipGpu *h, FlipGpuSolveStats *st) {
     a.ic_part = h->ic_part;
     a.ic_ctr = h->ic_ctr;
     a.ic_factor = 1;
-    cudaMemsetAsync(h->bar, 0, 2 * sizeof(unsigned), S);
+    cudaMemsetAsync(h->bar, 0, BAR_WORDS * sizeof(unsigned), S);
     void *kargs[] = {&a};
     const void *kern = mode == FLIPGPU_SOLVE_REF ? (const void *)k_cg<FLIPGPU_SOLVE_REF>
                                                  : (const void *)k_cg<FLIPGPU_SOLVE_FAST>;
@@ -3511,7 +3865,7 @@ int run_solve(FlipGpu *h, FlipGpuSolveStats *st) {
     if (precond == FLIPGPU_PRECOND_MG) {
       kern = (const void *)k_cg_mg<CG_MG_BLOCK>;
       grid = h->cg_grid[5];
-      smem = mg_block_bytes(h->mg_m, h->mg_lb, h->mg_nlev);
+      smem = MG_TILE_BYTES + mg_block_bytes(h->mg_m, h->mg_lb, h->mg_nlev);
       cudaError_t e = chunk_list();
       /* levels: 0 = the solver's grid (z the correction, r its right-hand
        * side); coarser ones from the coarsened flags */
@@ -3528,10 +3882,12 @@ int run_solve(FlipGpu *h, FlipGpuSolveStats *st) {
         L.diag = l == 0 ? h->diag : h->mg_diag[l];
         L.x = l == 0 ? h->z : h->mg_x[l];
         L.b = l == 0 ? h->r : h->mg_b[l];
-        L.res = h->mg_res[l];
         L.hs = hs;
         L.ihs = 1.0f / hs;
         L.lgm = (L.m & (L.m - 1)) == 0 ? __builtin_ctz((unsigned)L.m) : -1;
+        L.out = l > 0 && l < mg.lb && mg.nu <= MG_TILE_NU ? h->mg_y[l] : L.x;
+        L.tiles = h->mg_tiles[l];
+        L.ntiles = h->bar + 2 + l;
         hs *= 0.25f;
       }
       for (int l = 1; e == cudaSuccess && l < mg.nlev; l++) {
@@ -3546,7 +3902,7 @@ int run_solve(FlipGpu *h, FlipGpuSolveStats *st) {
       a.q = h->mg_q;
       /* zero off the liquid chunks (the sweeps only write inside them) and
        * finite direction buffers for the first iteration */
-      float *zero_bufs[5] = {h->z, h->mg_res[0], h->pdir, h->mg_p2, h->mg_q};
+      float *zero_bufs[4] = {h->z, h->pdir, h->mg_p2, h->mg_q};
       for (float *zb : zero_bufs)
         if (e == cudaSuccess) e = cudaMemsetAsync(zb, 0, nc * sizeof(float), S);
       if (e != cudaSuccess) {
@@ -3581,7 +3937,7 @@ int run_solve(FlipGpu *h, FlipGpuSolveStats *st) {
     a.ir_tol = nullptr;
     const int block = cg_block_of(kern);
     auto reset_flags = [&]() {
-      cudaMemsetAsync(h->bar, 0, 2 * sizeof(unsigned), S);
+      cudaMemsetAsync(h->bar, 0, BAR_WORDS * sizeof(unsigned), S);
       if (precond == FLIPGPU_PRECOND_IC) cudaMemsetAsync(h->ticket, 0, sizeof(unsigned), S);
     };
     if (mode == FLIPGPU_SOLVE_FAST && h->prm.refine_steps > 0) {
