@@ -1686,19 +1686,48 @@ __device__ __forceinline__ float4 mg_block_nbs(const MgBlockLevel &L, const MgSe
   return mg_add4(mg_add4(v, lo), hi);
 }
 
-/* half sweep of colour C by the segment's thread; own[]: its cells */
+/* b / hs and 1 / d (0 off the liquid): the products of a half sweep are then
+ * those of its fast division */
+__device__ __forceinline__ float4 mg_scaled(float4 b, float f) {
+  return make_float4(b.x * f, b.y * f, b.z * f, b.w * f);
+}
+__device__ __forceinline__ float mg_rcp(float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  return r;
+}
+__device__ __forceinline__ float4 mg_rcp4(float4 d) {
+  return make_float4(mg_rcp(d.x), mg_rcp(d.y), mg_rcp(d.z), mg_rcp(d.w));
+}
+
+/* half sweep of colour C by the segment's thread: x = (b / hs + neighbours) / d
+ * from bs = b / hs and rd = 1 / d; own[]: its cells */
 template <int C>
-__device__ __forceinline__ void mg_block_half(const MgBlockLevel &L, const MgSeg &s, float4 b,
-                                              float4 d, float4 (&own)[2]) {
+__device__ __forceinline__ void mg_block_half(const MgBlockLevel &L, const MgSeg &s, float4 bs,
+                                              float4 rd, float4 (&own)[2]) {
   const float4 v = mg_block_nbs(L, s, L.x[C ^ 1], own[C ^ 1], s.par ? C == 0 : C == 1);
-  own[C] = make_float4(
-      __fdividef(b.x * L.ihs + v.x, d.x), __fdividef(b.y * L.ihs + v.y, d.y),
-      __fdividef(b.z * L.ihs + v.z, d.z), __fdividef(b.w * L.ihs + v.w, d.w));
+  own[C] = make_float4((bs.x + v.x) * rd.x, (bs.y + v.y) * rd.y, (bs.z + v.z) * rd.z,
+                       (bs.w + v.w) * rd.w);
   L.x[C][s.at] = own[C];
+}
+
+/* the first red half sweep from x = 0 */
+__device__ __forceinline__ void mg_block_start(const MgBlockLevel &L, const MgSeg &s, float4 bs,
+                                               float4 rd, float4 (&own)[2]) {
+  own[0] = make_float4(bs.x * rd.x, bs.y * rd.y, bs.z * rd.z, bs.w * rd.w);
+  own[1] = make_float4(0, 0, 0, 0);
+  L.x[0][s.at] = own[0];
+  L.x[1][s.at] = own[1];
 }
 
 __device__ __forceinline__ float mg_block_res(float b, float hs, float d, float x, float nbs) {
   return d < INFINITY ? b - hs * (d * x - nbs) : 0.0f;
+}
+
+/* x plus the parents' corrections on the liquid */
+__device__ __forceinline__ float4 mg_corrected(float4 x, float4 rd, float4 add) {
+  return make_float4(x.x + (rd.x != 0.0f ? add.x : 0.0f), x.y + (rd.y != 0.0f ? add.y : 0.0f),
+                     x.z + (rd.z != 0.0f ? add.z : 0.0f), x.w + (rd.w != 0.0f ? add.w : 0.0f));
 }
 
 /* the segment's residuals, by the parity of k */
@@ -1739,28 +1768,40 @@ __device__ __forceinline__ void mg_block_levels(const MgArgs &mg) {
     if (t >= L.act) continue;
     const bool in = t < L.segs;
     const MgSeg s = mg_seg(L, in ? t : 0);
-    float4 own[2], b[2], d[2];
+    float4 own[2], b[2], d[2], bs[2], rd[2];
     if (in) {
       float v[2][4]; /* b of even and odd k */
       if (l == mg.lb) {
+        const float *gb = G.b + ((unsigned)s.i * L.m + s.j) * L.m + 8 * s.seg;
+        const int left = L.m - 8 * s.seg; /* cells of the line from the segment on */
+        if ((L.m & 3) == 0) {
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-          const int k = 8 * s.seg + u;
-          v[u & 1][u >> 1] = k < L.m ? __ldcg(G.b + ((unsigned)s.i * L.m + s.j) * L.m + k) : 0.0f;
+          for (int h = 0; h < 2; h++) {
+            const float4 w = 4 * h < left ? __ldcg(reinterpret_cast<const float4 *>(gb) + h)
+                                          : make_float4(0, 0, 0, 0);
+            v[0][2 * h] = w.x;
+            v[1][2 * h] = w.y;
+            v[0][2 * h + 1] = w.z;
+            v[1][2 * h + 1] = w.w;
+          }
+        } else {
+#pragma unroll
+          for (int u = 0; u < 8; u++) v[u & 1][u >> 1] = u < left ? __ldcg(gb + u) : 0.0f;
         }
       } else {
         /* the mean of the 8 children's residuals, lines in i, then j, then k */
         const MgBlockLevel F = mg_block_level(mg, l - 1);
 #pragma unroll
         for (int u = 0; u < 8; u++) v[u & 1][u >> 1] = 0.0f;
+#pragma unroll
         for (int c = 0; c < 4; c++) {
           const int i = 2 * s.i + (c >> 1), j = 2 * s.j + (c & 1);
-          if (i >= F.m || j >= F.m) continue;
 #pragma unroll
           for (int h = 0; h < 2; h++) { /* children of cells 4 h .. 4 h + 3 */
-            if (h >= F.ns) continue;
-            const int at = (i * F.m + j) * F.ns + h;
-            const float4 e = F.r[0][at], o = F.r[1][at];
+            const bool have = i < F.m && j < F.m && h < F.ns;
+            const int at = have ? (i * F.m + j) * F.ns + h : 0;
+            const float4 zero = make_float4(0, 0, 0, 0);
+            const float4 e = have ? F.r[0][at] : zero, o = have ? F.r[1][at] : zero;
             const float ev[4] = {e.x, e.y, e.z, e.w}, ov[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
             for (int q = 0; q < 4; q++) {
@@ -1781,20 +1822,20 @@ __device__ __forceinline__ void mg_block_levels(const MgArgs &mg) {
       d[1] = L.d[1][t];
       L.b[0][t] = b[0];
       L.b[1][t] = b[1];
-      own[0] = make_float4(__fdividef(b[0].x * L.ihs, d[0].x), __fdividef(b[0].y * L.ihs, d[0].y),
-                           __fdividef(b[0].z * L.ihs, d[0].z), __fdividef(b[0].w * L.ihs, d[0].w));
-      own[1] = make_float4(0, 0, 0, 0);
-      L.x[0][s.at] = own[0];
-      L.x[1][s.at] = own[1];
+      bs[0] = mg_scaled(b[0], L.ihs);
+      bs[1] = mg_scaled(b[1], L.ihs);
+      rd[0] = mg_rcp4(d[0]);
+      rd[1] = mg_rcp4(d[1]);
+      mg_block_start(L, s, bs[0], rd[0], own);
     }
     mg_bar(L);
     const int halves = l == last ? 4 * mg.coarse_sweeps - 2 : 2 * mg.nu - 1;
     for (int h = 0; h < halves; h++) {
       if (in) {
         if (h & 1)
-          mg_block_half<0>(L, s, b[0], d[0], own);
+          mg_block_half<0>(L, s, bs[0], rd[0], own);
         else
-          mg_block_half<1>(L, s, b[1], d[1], own);
+          mg_block_half<1>(L, s, bs[1], rd[1], own);
       }
       mg_bar(L);
     }
@@ -1809,7 +1850,7 @@ __device__ __forceinline__ void mg_block_levels(const MgArgs &mg) {
     mg_bar(L); /* the coarser level is done */
     const bool in = t < L.segs;
     const MgSeg s = mg_seg(L, in ? t : 0);
-    float4 own[2], b[2], d[2];
+    float4 own[2], bs[2], rd[2];
     if (in) {
       const MgBlockLevel C = mg_block_level(mg, l + 1);
       const int ci = s.i / 2, cj = s.j / 2;
@@ -1824,23 +1865,19 @@ __device__ __forceinline__ void mg_block_levels(const MgArgs &mg) {
       const float4 add = make_float4(ce.x, co.x, ce.y, co.y);
 #pragma unroll
       for (int q = 0; q < 2; q++) {
-        b[q] = L.b[q][t];
-        d[q] = L.d[q][t];
-        float4 x = L.x[q][s.at];
-        x.x += d[q].x < INFINITY ? add.x : 0.0f;
-        x.y += d[q].y < INFINITY ? add.y : 0.0f;
-        x.z += d[q].z < INFINITY ? add.z : 0.0f;
-        x.w += d[q].w < INFINITY ? add.w : 0.0f;
-        L.x[q][s.at] = own[q] = x;
+        bs[q] = mg_scaled(L.b[q][t], L.ihs);
+        rd[q] = mg_rcp4(L.d[q][t]);
+        own[q] = mg_corrected(L.x[q][s.at], rd[q], add);
+        L.x[q][s.at] = own[q];
       }
     }
     mg_bar(L);
     for (int h = 0; h < 2 * mg.nu; h++) {
       if (in) {
         if (h & 1)
-          mg_block_half<0>(L, s, b[0], d[0], own);
+          mg_block_half<0>(L, s, bs[0], rd[0], own);
         else
-          mg_block_half<1>(L, s, b[1], d[1], own);
+          mg_block_half<1>(L, s, bs[1], rd[1], own);
       }
       mg_bar(L);
     }
@@ -1849,11 +1886,17 @@ __device__ __forceinline__ void mg_block_levels(const MgArgs &mg) {
   if (t < T.segs) {
     const MgSeg s = mg_seg(T, t);
     const float4 x0 = T.x[s.par][s.at], x1 = T.x[s.par ^ 1][s.at]; /* even and odd k */
-    const float v[8] = {x0.x, x1.x, x0.y, x1.y, x0.z, x1.z, x0.w, x1.w};
+    float *gx = G.x + ((unsigned)s.i * T.m + s.j) * T.m + 8 * s.seg;
+    const int left = T.m - 8 * s.seg;
+    if ((T.m & 3) == 0) {
+      float4 *g4 = reinterpret_cast<float4 *>(gx);
+      if (left > 0) g4[0] = make_float4(x0.x, x1.x, x0.y, x1.y);
+      if (left > 4) g4[1] = make_float4(x0.z, x1.z, x0.w, x1.w);
+    } else {
+      const float v[8] = {x0.x, x1.x, x0.y, x1.y, x0.z, x1.z, x0.w, x1.w};
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int k = 8 * s.seg + u;
-      if (k < T.m) G.x[((unsigned)s.i * T.m + s.j) * T.m + k] = v[u];
+      for (int u = 0; u < 8; u++)
+        if (u < left) gx[u] = v[u];
     }
   }
 }
@@ -1987,23 +2030,23 @@ __device__ __forceinline__ void mg_tile_down(const MgArgs &mg, int l) {
   const MgLevel &F = mg.lv[l], &Cl = mg.lv[l + 1];
   const MgBlockLevel L = mg_tile_level(F);
   const unsigned count = __ldcg(F.ntiles);
+  unsigned next = blockIdx.x < count ? __ldcg(F.tiles + blockIdx.x) : 0u;
   for (unsigned w = blockIdx.x; w < count; w += gridDim.x) {
-    const unsigned t = __ldcg(F.tiles + w);
+    const unsigned t = next;
     const MgTileSeg q = mg_tile_seg(L, F.m, t);
     float4 own[2], b[2], d[2];
     mg_tile_system(F, q, b, d);
-    own[0] = make_float4(__fdividef(b[0].x * L.ihs, d[0].x), __fdividef(b[0].y * L.ihs, d[0].y),
-                         __fdividef(b[0].z * L.ihs, d[0].z), __fdividef(b[0].w * L.ihs, d[0].w));
-    own[1] = make_float4(0, 0, 0, 0);
+    const float4 bs[2] = {mg_scaled(b[0], L.ihs), mg_scaled(b[1], L.ihs)};
+    const float4 rd[2] = {mg_rcp4(d[0]), mg_rcp4(d[1])};
+    next = w + gridDim.x < count ? __ldcg(F.tiles + w + gridDim.x) : 0u;
     __syncthreads(); /* the previous tile's restriction is done */
-    L.x[0][q.s.at] = own[0];
-    L.x[1][q.s.at] = own[1];
+    mg_block_start(L, q.s, bs[0], rd[0], own);
     __syncthreads();
     for (int h = 1; h < 2 * mg.nu; h++) {
       if (h & 1)
-        mg_block_half<1>(L, q.s, b[1], d[1], own);
+        mg_block_half<1>(L, q.s, bs[1], rd[1], own);
       else
-        mg_block_half<0>(L, q.s, b[0], d[0], own);
+        mg_block_half<0>(L, q.s, bs[0], rd[0], own);
       __syncthreads();
     }
     mg_tile_store(F.x, F, q, own);
@@ -2039,8 +2082,9 @@ __device__ __forceinline__ void mg_tile_up(const MgArgs &mg, int l) {
   const MgLevel &F = mg.lv[l], &Cl = mg.lv[l + 1];
   const MgBlockLevel L = mg_tile_level(F);
   const unsigned count = __ldcg(F.ntiles);
+  unsigned next = blockIdx.x < count ? __ldcg(F.tiles + blockIdx.x) : 0u;
   for (unsigned w = blockIdx.x; w < count; w += gridDim.x) {
-    const MgTileSeg q = mg_tile_seg(L, F.m, __ldcg(F.tiles + w));
+    const MgTileSeg q = mg_tile_seg(L, F.m, next);
     float4 own[2], b[2], d[2], xe, xo;
     mg_tile_load(F.x, q, F.m, 0.0f, xe, xo);
     float p[4]; /* the parents' x */
@@ -2052,24 +2096,21 @@ __device__ __forceinline__ void mg_tile_up(const MgArgs &mg, int l) {
                  : 0.0f;
     }
     mg_tile_system(F, q, b, d);
-    own[0] = q.s.par ? xo : xe;
-    own[1] = q.s.par ? xe : xo;
-#pragma unroll
-    for (int c = 0; c < 2; c++) {
-      own[c].x += d[c].x < INFINITY ? p[0] : 0.0f;
-      own[c].y += d[c].y < INFINITY ? p[1] : 0.0f;
-      own[c].z += d[c].z < INFINITY ? p[2] : 0.0f;
-      own[c].w += d[c].w < INFINITY ? p[3] : 0.0f;
-    }
+    const float4 bs[2] = {mg_scaled(b[0], L.ihs), mg_scaled(b[1], L.ihs)};
+    const float4 rd[2] = {mg_rcp4(d[0]), mg_rcp4(d[1])};
+    const float4 add = make_float4(p[0], p[1], p[2], p[3]);
+    own[0] = mg_corrected(q.s.par ? xo : xe, rd[0], add);
+    own[1] = mg_corrected(q.s.par ? xe : xo, rd[1], add);
+    next = w + gridDim.x < count ? __ldcg(F.tiles + w + gridDim.x) : 0u;
     __syncthreads();
     L.x[0][q.s.at] = own[0];
     L.x[1][q.s.at] = own[1];
     __syncthreads();
     for (int h = 0; h < 2 * mg.nu; h++) {
       if (h & 1)
-        mg_block_half<0>(L, q.s, b[0], d[0], own);
+        mg_block_half<0>(L, q.s, bs[0], rd[0], own);
       else
-        mg_block_half<1>(L, q.s, b[1], d[1], own);
+        mg_block_half<1>(L, q.s, bs[1], rd[1], own);
       __syncthreads();
     }
     mg_tile_store(F.out, F, q, own);
