@@ -65,7 +65,7 @@ struct SimConst {
 };
 
 constexpr int BAR_WORDS = 12;
-constexpr int CG_VARIANTS = 6; /* persistent CG kernels (k_pcg.cu cg_grid_size) */
+constexpr int CG_VARIANTS = 7; /* persistent CG kernels (k_pcg.cu cg_grid_size) */
 
 struct FlipGpu {
   FlipGpuParams prm;
@@ -145,7 +145,7 @@ struct FlipGpu {
                          then the number of tiles in each level's mg_tiles */
   int cg_grid[CG_VARIANTS]; /* cooperative CG grids (0 = none): REF, FAST, FAST single-
                                reduction (small blocks), FAST IC, single-reduction (large),
-                               FAST MG */
+                               FAST MG, cells in registers */
   int solve_blocks;   /* cap on the persistent solve's grid (0 = none; not the IC
                          wavefront), so that concurrent simulations' solves share the GPU */
   int solve_capacity; /* co-resident grid of the last solve's kernel */

@@ -43,6 +43,7 @@ struct SolveArgs {
   double inv_h2;   /* 1/(double)h2 */
   double h2;       /* (double)(float)(1.0/(n*n)) */
   float inv_h2_f;
+  float ih, il;    /* inv_h2 as a float pair */
 };
 
 __device__ __forceinline__ bool in_range(int n, int i, int j, int k) {
@@ -99,6 +100,7 @@ k_setup(SolveArgs s, int mode, const uint8_t *__restrict__ A, const float *__res
   if (mode == FLIPGPU_SOLVE_REF) {
     double pv = 1.0 / (double)sqrtf(d);
     P[c] = pv;
+    reinterpret_cast<float2 *>(P + nc)[c] = make_float2((float)pv, (float)(pv - (double)(float)pv));
     if (pv == 1.0) atomicOr(iflags + IF_EXOTIC, 1);
   } else {
     diag[c] = d;
@@ -479,6 +481,7 @@ struct CgArgs {
   const unsigned *chunk_list;  /* single-reduction CG: the 32-quad chunks holding liquid */
   const unsigned *chunk_count; /* ... and their number */
   const double *P;
+  const float2 *Ps;            /* P as float pairs */
   const float *diag;
   const float *Pf;
   float2 *part;
@@ -648,17 +651,12 @@ __device__ __forceinline__ float cg_matvec(const CgArgs &a, size_t c, int i, int
       uint8_t aa = a.A[q];
       if (aa == CELL_FLUID) return q == c ? sc : snew(q);
       if (aa == CELL_WALL) return sc;
-      return a.s.subcell ? (float)((double)a.L[q] / fmin(1.0e-6, (double)Lc) * (double)sc)
-                         : 0.0f;
+      return a.s.subcell ? refmath::ghost_ref(a.L[q], Lc, sc) : 0.0f;
     };
-    double v = 6.0 * (double)sc;
-    v -= (double)xref(i + 1, j, k);
-    v -= (double)xref(i - 1, j, k);
-    v -= (double)xref(i, j + 1, k);
-    v -= (double)xref(i, j - 1, k);
-    v -= (double)xref(i, j, k + 1);
-    v -= (double)xref(i, j, k - 1);
-    return a.s.pow2 ? (float)(v * a.s.inv_h2) : (float)(v / a.s.h2);
+    const float x0 = xref(i + 1, j, k), x1 = xref(i - 1, j, k), x2 = xref(i, j + 1, k),
+                x3 = xref(i, j - 1, k), x4 = xref(i, j, k + 1), x5 = xref(i, j, k - 1);
+    return refmath::stencil_ref(sc, x0, x1, x2, x3, x4, x5, a.s.ih, a.s.il, a.s.h2, a.s.inv_h2,
+                                a.s.pow2);
   } else {
     float acc = a.diag[c] * sc;
     const size_t sj = n, si = (size_t)n * n;
@@ -678,6 +676,12 @@ template <int MODE>
 __device__ __forceinline__ float cg_precond(const CgArgs &a, size_t c, int i, int j, int k,
                                             float rc) {
   if (MODE == FLIPGPU_SOLVE_REF) {
+    const double pc = a.P[c];
+    const float2 ps = a.Ps[c];
+    if (rc != 0.0f) {
+      const float z = refmath::scale2_ref(rc, ps.x, ps.y, pc);
+      if (z != 0.0f) return z;
+    }
     const int n = a.s.n;
     const uint8_t *A = a.A;
     double t = (double)rc;
@@ -687,7 +691,6 @@ __device__ __forceinline__ float cg_precond(const CgArgs &a, size_t c, int i, in
                   (k > 0 && A[cell_id(n, i, j, k - 1)] == CELL_FLUID);
       t = (signbit(rc) && !back) ? -0.0 : 0.0;
     }
-    const double pc = a.P[c];
     double q = t * pc;
     double t2 = q;
     if (q == 0.0) {
@@ -699,131 +702,6 @@ __device__ __forceinline__ float cg_precond(const CgArgs &a, size_t c, int i, in
     return (float)(t2 * pc);
   } else {
     return rc * a.Pf[c];
-  }
-}
-
-template <int MODE>
-__global__ void __launch_bounds__(CG_BLOCK) k_cg(CgArgs a) {
-  if (MODE != FLIPGPU_SOLVE_REF && ir_skipped(a)) return;
-  const unsigned nb = gridDim.x;
-  const size_t stride = (size_t)nb * CG_BLOCK;
-  const size_t t0 = (size_t)blockIdx.x * CG_BLOCK + threadIdx.x;
-  const int n = a.s.n;
-  const size_t nc = a.nc;
-
-  /* phase 0: r = b - A x, z = M^-1 r; b.b, r.r, z.r */
-  FF pbb = ff_zero(), prr = ff_zero(), pzr = ff_zero();
-  for (size_t c = t0; c < nc; c += stride) {
-    float rv = 0.0f, zv = 0.0f;
-    if (a.A[c] == CELL_FLUID) {
-      int i, j, k;
-      decode(c, n, i, j, k);
-      float bc = a.b[c];
-      dot_acc<MODE>(pbb, bc, bc);
-      float xc = a.x[c];
-      /* the initial matvec reads x, which nobody writes in this phase */
-      float ax = cg_matvec<MODE>(a, c, i, j, k, xc, a.x, a.x, 0.0f, true);
-      rv = bc + -1.0f * ax;
-      dot_acc<MODE>(prr, rv, rv);
-      zv = cg_precond<MODE>(a, c, i, j, k, rv);
-      dot_acc<MODE>(pzr, zv, rv);
-    }
-    a.r[c] = rv;
-    a.z[c] = zv;
-  }
-  store_partial(a.part, 0, nb, pbb);
-  store_partial(a.part, 1, nb, prr);
-  store_partial(a.part, 2, nb, pzr);
-  if (!grid_barrier(a.bar, a.iflags)) return;
-  double b2, rr, azr, unused;
-  sum_partials(a.part, 0, 1, nb, b2, rr);
-  sum_partials(a.part, 2, -1, nb, azr, unused);
-  double eps;
-  if (MODE == FLIPGPU_SOLVE_REF) {
-    eps = a.ref_eps;
-    if (a.eps_abs >= 0.0) {
-      eps = a.eps_abs;
-    } else if (a.rel_tol > 0.0) {
-      double target = a.rel_tol * a.rel_tol * b2;
-      while (eps > target && eps > 0.0) eps *= 0.25;
-    }
-  } else {
-    const double rt = cg_rel_tol(a);
-    eps = rt * rt * b2;
-  }
-  int done = 0, iters = 0;
-  double e2 = rr;
-  if (MODE != FLIPGPU_SOLVE_REF && rr <= eps) done = 1;
-  float *so = a.s0, *sn = a.s1;
-  float beta_f = 0.0f;
-  bool first = true;
-  while (!done) {
-    /* phase A: s_new = z + beta*s_old (op), w = A s_new, w.s_new */
-    FF pws = ff_zero();
-    for (size_t c = t0; c < nc; c += stride) {
-      float snv = 0.0f, wv = 0.0f;
-      if (a.A[c] == CELL_FLUID) {
-        int i, j, k;
-        decode(c, n, i, j, k);
-        float zc = a.z[c];
-        snv = first ? zc : zc + beta_f * so[c];
-        wv = cg_matvec<MODE>(a, c, i, j, k, snv, a.z, so, beta_f, first);
-        dot_acc<MODE>(pws, wv, snv);
-      }
-      sn[c] = snv;
-      a.w[c] = wv;
-    }
-    store_partial(a.part, 3, nb, pws);
-    if (!grid_barrier(a.bar, a.iflags)) return;
-    double ws;
-    sum_partials(a.part, 3, -1, nb, ws, unused);
-    const double alpha = azr / ws;
-    const float alpha_f = (float)alpha, nalpha_f = (float)(-alpha);
-    /* phase B: x += alpha s, r -= alpha w, z = M^-1 r; r.r, z.r */
-    prr = ff_zero();
-    pzr = ff_zero();
-    for (size_t c = t0; c < nc; c += stride) {
-      if (a.A[c] == CELL_FLUID) {
-        int i, j, k;
-        decode(c, n, i, j, k);
-        a.x[c] = a.x[c] + alpha_f * sn[c];
-        float rv = a.r[c] + nalpha_f * a.w[c];
-        a.r[c] = rv;
-        dot_acc<MODE>(prr, rv, rv);
-        float zv = cg_precond<MODE>(a, c, i, j, k, rv);
-        a.z[c] = zv;
-        dot_acc<MODE>(pzr, zv, rv);
-      } else {
-        a.x[c] = 0.0f;
-        a.r[c] = 0.0f;
-        a.z[c] = 0.0f;
-      }
-    }
-    store_partial(a.part, 4, nb, prr);
-    store_partial(a.part, 5, nb, pzr);
-    if (!grid_barrier(a.bar, a.iflags)) return;
-    double zr;
-    sum_partials(a.part, 4, 5, nb, rr, zr);
-    iters++;
-    e2 = (MODE == FLIPGPU_SOLVE_REF) ? (double)(float)rr : rr;
-    if (e2 <= eps) done = 1;
-    else if (!(e2 == e2)) done = 2;
-    else if (iters >= a.max_iters) done = 3;
-    const double beta = zr / azr;
-    azr = zr;
-    beta_f = (float)beta;
-    first = false;
-    float *t = so;
-    so = sn;
-    sn = t;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    a.iflags[IF_DONE] = done;
-    a.iflags[IF_ITERS] = iters;
-    a.iflags[IF_NAN] = done == 2;
-    a.scal[SC_ERR2] = e2;
-    a.scal[SC_B2] = b2;
-    a.scal[SC_EPS] = eps;
   }
 }
 
@@ -1012,6 +890,369 @@ struct Cg1Q {
   uchar4 A;
   float4 u, w, s;
 };
+
+template <int MODE>
+__global__ void __launch_bounds__(CG_BLOCK) k_cg(CgArgs a) {
+  if (MODE != FLIPGPU_SOLVE_REF && ir_skipped(a)) return;
+  const unsigned nb = gridDim.x;
+  const size_t stride = (size_t)nb * CG_BLOCK;
+  const size_t t0 = (size_t)blockIdx.x * CG_BLOCK + threadIdx.x;
+  const int n = a.s.n;
+  const size_t nc = a.nc;
+  unsigned epoch = 0;
+  __shared__ double s_sum[3];
+  /* the partials of slots k0 .. k0 + K - 1, summed by one warp for the block */
+  auto sums = [&](int k0, auto K) {
+    if (threadIdx.x < 32) {
+      double t[decltype(K)::value];
+      warp_sum_partials<decltype(K)::value>(a.part, k0, nb, t);
+      if (threadIdx.x == 0)
+        for (int q = 0; q < decltype(K)::value; q++) s_sum[q] = t[q];
+    }
+    __syncthreads();
+  };
+  using std::integral_constant;
+
+  /* phase 0: r = b - A x, z = M^-1 r; b.b, r.r, z.r */
+  FF pbb = ff_zero(), prr = ff_zero(), pzr = ff_zero();
+  for (size_t c = t0; c < nc; c += stride) {
+    float rv = 0.0f, zv = 0.0f;
+    if (a.A[c] == CELL_FLUID) {
+      int i, j, k;
+      decode(c, n, i, j, k);
+      float bc = a.b[c];
+      dot_acc<MODE>(pbb, bc, bc);
+      float xc = a.x[c];
+      /* the initial matvec reads x, which nobody writes in this phase */
+      float ax = cg_matvec<MODE>(a, c, i, j, k, xc, a.x, a.x, 0.0f, true);
+      rv = bc + -1.0f * ax;
+      dot_acc<MODE>(prr, rv, rv);
+      zv = cg_precond<MODE>(a, c, i, j, k, rv);
+      dot_acc<MODE>(pzr, zv, rv);
+    }
+    a.r[c] = rv;
+    a.z[c] = zv;
+  }
+  {
+    FF v[3] = {pbb, prr, pzr};
+    store_partials<3, CG_BLOCK>(a.part, 0, nb, v);
+  }
+  if (!count_barrier(a.bar, epoch, a.iflags)) return;
+  sums(0, integral_constant<int, 3>{});
+  double b2 = s_sum[0], rr = s_sum[1], azr = s_sum[2];
+  double eps;
+  if (MODE == FLIPGPU_SOLVE_REF) {
+    eps = a.ref_eps;
+    if (a.eps_abs >= 0.0) {
+      eps = a.eps_abs;
+    } else if (a.rel_tol > 0.0) {
+      double target = a.rel_tol * a.rel_tol * b2;
+      while (eps > target && eps > 0.0) eps *= 0.25;
+    }
+  } else {
+    const double rt = cg_rel_tol(a);
+    eps = rt * rt * b2;
+  }
+  int done = 0, iters = 0;
+  double e2 = rr;
+  if (MODE != FLIPGPU_SOLVE_REF && rr <= eps) done = 1;
+  float *so = a.s0, *sn = a.s1;
+  float beta_f = 0.0f;
+  bool first = true;
+  while (!done) {
+    /* phase A: s_new = z + beta*s_old (op), w = A s_new, w.s_new */
+    FF pws = ff_zero();
+    for (size_t c = t0; c < nc; c += stride) {
+      float snv = 0.0f, wv = 0.0f;
+      if (a.A[c] == CELL_FLUID) {
+        int i, j, k;
+        decode(c, n, i, j, k);
+        float zc = a.z[c];
+        snv = first ? zc : zc + beta_f * so[c];
+        wv = cg_matvec<MODE>(a, c, i, j, k, snv, a.z, so, beta_f, first);
+        dot_acc<MODE>(pws, wv, snv);
+      }
+      sn[c] = snv;
+      a.w[c] = wv;
+    }
+    {
+      FF v[1] = {pws};
+      store_partials<1, CG_BLOCK>(a.part, 3, nb, v);
+    }
+    if (!count_barrier(a.bar, epoch, a.iflags)) return;
+    sums(3, integral_constant<int, 1>{});
+    const double ws = s_sum[0];
+    const double alpha = azr / ws;
+    const float alpha_f = (float)alpha, nalpha_f = (float)(-alpha);
+    /* phase B: x += alpha s, r -= alpha w, z = M^-1 r; r.r, z.r */
+    prr = ff_zero();
+    pzr = ff_zero();
+    for (size_t c = t0; c < nc; c += stride) {
+      if (a.A[c] == CELL_FLUID) {
+        int i, j, k;
+        decode(c, n, i, j, k);
+        a.x[c] = a.x[c] + alpha_f * sn[c];
+        float rv = a.r[c] + nalpha_f * a.w[c];
+        a.r[c] = rv;
+        dot_acc<MODE>(prr, rv, rv);
+        float zv = cg_precond<MODE>(a, c, i, j, k, rv);
+        a.z[c] = zv;
+        dot_acc<MODE>(pzr, zv, rv);
+      } else {
+        a.x[c] = 0.0f;
+        a.r[c] = 0.0f;
+        a.z[c] = 0.0f;
+      }
+    }
+    {
+      FF v[2] = {prr, pzr};
+      store_partials<2, CG_BLOCK>(a.part, 4, nb, v);
+    }
+    if (!count_barrier(a.bar, epoch, a.iflags)) return;
+    sums(4, integral_constant<int, 2>{});
+    rr = s_sum[0];
+    const double zr = s_sum[1];
+    iters++;
+    e2 = (MODE == FLIPGPU_SOLVE_REF) ? (double)(float)rr : rr;
+    if (e2 <= eps) done = 1;
+    else if (!(e2 == e2)) done = 2;
+    else if (iters >= a.max_iters) done = 3;
+    const double beta = zr / azr;
+    azr = zr;
+    beta_f = (float)beta;
+    first = false;
+    float *t = so;
+    so = sn;
+    sn = t;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.iflags[IF_DONE] = done;
+    a.iflags[IF_ITERS] = iters;
+    a.iflags[IF_NAN] = done == 2;
+    a.scal[SC_ERR2] = e2;
+    a.scal[SC_B2] = b2;
+    a.scal[SC_EPS] = eps;
+  }
+}
+
+
+/* k_cg for grids of at most CGR_CELLS cells a thread on one block an SM
+ * (n <= 67): a thread's cells stay in registers through the solve (x, r, w,
+ * the direction, the preconditioner, which neighbours are liquid or air), so
+ * an iteration only exchanges z and the directions and waits for two
+ * barriers. The arithmetic is k_cg's cell by cell. Reading everything anew in
+ * every phase, with the reference's double expressions in FP64 (1/64 of the
+ * FP32 rate, and a division where n is no power of two), a step of n = 48 in
+ * the reference's arithmetic took 5.6 ms; it takes 2.0. */
+constexpr int CGR_BLOCK = 512, CGR_CELLS = 4;
+
+template <int MODE, int E>
+__global__ void __launch_bounds__(CGR_BLOCK, 1) k_cg_reg(CgArgs a) {
+  if (MODE != FLIPGPU_SOLVE_REF && ir_skipped(a)) return;
+  constexpr bool REF = MODE == FLIPGPU_SOLVE_REF;
+  const unsigned nb = gridDim.x, stride = nb * CGR_BLOCK;
+  const unsigned t0 = blockIdx.x * CGR_BLOCK + threadIdx.x;
+  const int n = a.s.n;
+  const unsigned nc = (unsigned)a.nc;
+  unsigned epoch = 0;
+  __shared__ double s_eps, s_b2, s_azr;
+  __shared__ float s_alpha, s_nalpha, s_beta;
+  __shared__ int s_done;
+  /* bits 0..5: the neighbours i+1, i-1, j+1, j-1, k+1, k-1 that are liquid;
+   * 8..13: those that are air; 31: the cell is liquid */
+  unsigned mask[E];
+  float x[E], r[E], z[E], sd[E], w[E], ph[E], pl[E];
+  const int off[6] = {n * n, -n * n, n, -n, 1, -1};
+  FF pbb = ff_zero(), prr = ff_zero(), pzr = ff_zero();
+
+  /* w = A v at the thread's cell e; at(q) gives v at a liquid neighbour */
+  auto matvec = [&](int e, unsigned c, float v, auto at) -> float {
+    float xs[6];
+#pragma unroll
+    for (int q = 0; q < 6; q++) xs[q] = mask[e] >> q & 1 ? at(c + off[q]) : (REF ? v : 0.0f);
+    if (REF) {
+      if (mask[e] >> 8 & 0x3f) {
+        const float Lc = __ldg(a.L + c);
+#pragma unroll
+        for (int q = 0; q < 6; q++)
+          if (mask[e] >> (8 + q) & 1)
+            xs[q] = a.s.subcell ? refmath::ghost_ref(__ldg(a.L + c + off[q]), Lc, v) : 0.0f;
+      }
+      return refmath::stencil_ref(v, xs[0], xs[1], xs[2], xs[3], xs[4], xs[5], a.s.ih, a.s.il,
+                                  a.s.h2, a.s.inv_h2, a.s.pow2);
+    }
+    float acc = pl[e] * v; /* FAST: ph = 1 / diag, pl = diag */
+#pragma unroll
+    for (int q = 0; q < 6; q++)
+      if (mask[e] >> q & 1) acc -= xs[q];
+    return acc * a.s.inv_h2_f;
+  };
+  auto precond = [&](int e, unsigned c, float rc) -> float {
+    if (!REF) return rc * ph[e];
+    if (rc != 0.0f) {
+      const float v = refmath::scale2_ref(rc, ph[e], pl[e], a.P[c]);
+      if (v != 0.0f) return v;
+    }
+    int i, j, k;
+    decode(c, n, i, j, k);
+    return cg_precond<MODE>(a, c, i, j, k, rc); /* signed zeros */
+  };
+
+#pragma unroll
+  for (int e = 0; e < E; e++) {
+    const unsigned c = t0 + e * stride;
+    mask[e] = 0;
+    x[e] = r[e] = z[e] = sd[e] = w[e] = ph[e] = pl[e] = 0.0f;
+    if (c >= nc || a.A[c] != CELL_FLUID) continue;
+    int i, j, k;
+    decode(c, n, i, j, k);
+    const bool in[6] = {i + 1 < n, i > 0, j + 1 < n, j > 0, k + 1 < n, k > 0};
+    unsigned m = 0x80000000u;
+#pragma unroll
+    for (int q = 0; q < 6; q++)
+      if (in[q]) {
+        const uint8_t f = a.A[c + off[q]];
+        m |= f == CELL_FLUID ? 1u << q : (f == CELL_WALL ? 0u : 0x100u << q);
+      }
+    mask[e] = m;
+    if (REF) {
+      const float2 ps = a.Ps[c];
+      ph[e] = ps.x;
+      pl[e] = ps.y;
+    } else {
+      ph[e] = a.Pf[c];
+      pl[e] = a.diag[c];
+    }
+    const float bc = a.b[c];
+    dot_acc<MODE>(pbb, bc, bc);
+    x[e] = a.x[c];
+    const float ax = matvec(e, c, x[e], [&](unsigned q) { return __ldcg(a.x + q); });
+    r[e] = bc + -1.0f * ax;
+    dot_acc<MODE>(prr, r[e], r[e]);
+    z[e] = precond(e, c, r[e]);
+    dot_acc<MODE>(pzr, z[e], r[e]);
+    a.z[c] = z[e];
+  }
+  {
+    FF v[3] = {pbb, prr, pzr};
+    store_partials<3, CGR_BLOCK>(a.part, 0, nb, v);
+  }
+  if (!count_barrier(a.bar, epoch, a.iflags)) return;
+  double e2 = 0.0; /* thread 0's */
+  if (threadIdx.x < 32) {
+    double t[3];
+    warp_sum_partials<3>(a.part, 0, nb, t);
+    if (threadIdx.x == 0) {
+      double eps;
+      if (REF) {
+        eps = a.ref_eps;
+        if (a.eps_abs >= 0.0) {
+          eps = a.eps_abs;
+        } else if (a.rel_tol > 0.0) {
+          const double target = a.rel_tol * a.rel_tol * t[0];
+          while (eps > target && eps > 0.0) eps *= 0.25;
+        }
+      } else {
+        const double rt = cg_rel_tol(a);
+        eps = rt * rt * t[0];
+      }
+      s_b2 = t[0];
+      s_eps = eps;
+      s_azr = t[2];
+      e2 = t[1];
+      s_done = !REF && e2 <= eps ? 1 : 0;
+    }
+  }
+  __syncthreads();
+  int done = s_done, iters = 0;
+  float *so = a.s0, *sn = a.s1;
+  float beta = 0.0f;
+  bool first = true;
+  while (!done) {
+    /* s = z + beta s (op), w = A s, w.s */
+    FF pws = ff_zero();
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      if (!mask[e]) continue;
+      const unsigned c = t0 + e * stride;
+      sd[e] = first ? z[e] : z[e] + beta * sd[e];
+      w[e] = matvec(e, c, sd[e], [&](unsigned q) {
+        const float zq = __ldcg(a.z + q);
+        return first ? zq : zq + beta * __ldcg(so + q);
+      });
+      dot_acc<MODE>(pws, w[e], sd[e]);
+      sn[c] = sd[e];
+    }
+    {
+      FF v[1] = {pws};
+      store_partials<1, CGR_BLOCK>(a.part, 3, nb, v);
+    }
+    if (!count_barrier(a.bar, epoch, a.iflags)) return;
+    if (threadIdx.x < 32) {
+      double t[1];
+      warp_sum_partials<1>(a.part, 3, nb, t);
+      if (threadIdx.x == 0) {
+        const double alpha = s_azr / t[0];
+        s_alpha = (float)alpha;
+        s_nalpha = (float)(-alpha);
+      }
+    }
+    __syncthreads();
+    const float alpha = s_alpha, nalpha = s_nalpha;
+    /* x += alpha s, r -= alpha w, z = M^-1 r; r.r, z.r */
+    prr = ff_zero();
+    pzr = ff_zero();
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      if (!mask[e]) continue;
+      const unsigned c = t0 + e * stride;
+      x[e] = x[e] + alpha * sd[e];
+      r[e] = r[e] + nalpha * w[e];
+      dot_acc<MODE>(prr, r[e], r[e]);
+      z[e] = precond(e, c, r[e]);
+      a.z[c] = z[e];
+      dot_acc<MODE>(pzr, z[e], r[e]);
+    }
+    {
+      FF v[2] = {prr, pzr};
+      store_partials<2, CGR_BLOCK>(a.part, 4, nb, v);
+    }
+    if (!count_barrier(a.bar, epoch, a.iflags)) return;
+    iters++;
+    if (threadIdx.x < 32) {
+      double t[2];
+      warp_sum_partials<2>(a.part, 4, nb, t);
+      if (threadIdx.x == 0) {
+        e2 = REF ? (double)(float)t[0] : t[0];
+        done = e2 <= s_eps ? 1 : (!(e2 == e2) ? 2 : (iters >= a.max_iters ? 3 : 0));
+        s_beta = (float)(t[1] / s_azr);
+        s_azr = t[1];
+        s_done = done;
+      }
+    }
+    __syncthreads();
+    done = s_done;
+    beta = s_beta;
+    first = false;
+    float *t = so;
+    so = sn;
+    sn = t;
+  }
+  if (iters > 0)
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      const unsigned c = t0 + e * stride;
+      if (c < nc) a.x[c] = mask[e] ? x[e] : 0.0f;
+    }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.iflags[IF_DONE] = done;
+    a.iflags[IF_ITERS] = iters;
+    a.iflags[IF_NAN] = done == 2;
+    a.scal[SC_ERR2] = e2;
+    a.scal[SC_B2] = s_b2;
+    a.scal[SC_EPS] = s_eps;
+  }
+}
 
 /* The 32-quad chunks of the single-reduction CG that hold liquid, in
  * increasing order (flags by one warp per chunk, an exclusive scan, a
@@ -3604,12 +3845,22 @@ constexpr int CG_MG_BLOCK = 512;
 constexpr size_t MG_SMEM_MAX = 128 * 1024; /* a tile, and block 0's levels: <= 16^3 + 8^3 + 4^3
                                               cells */
 
+static const void *cg_reg_kernel(bool ref, int cells) {
+  constexpr int R = FLIPGPU_SOLVE_REF, F = FLIPGPU_SOLVE_FAST;
+  if (cells == 1) return ref ? (const void *)k_cg_reg<R, 1> : (const void *)k_cg_reg<F, 1>;
+  if (cells == 2) return ref ? (const void *)k_cg_reg<R, 2> : (const void *)k_cg_reg<F, 2>;
+  return ref ? (const void *)k_cg_reg<R, 4> : (const void *)k_cg_reg<F, 4>;
+}
+
 /* threads per block of a persistent CG kernel */
 static int cg_block_of(const void *kern) {
   if (kern == (const void *)k_cg_cg1<CG1_BLOCK_SMALL>) return CG1_BLOCK_SMALL;
   if (kern == (const void *)k_cg_cg1<CG1_BLOCK_LARGE>) return CG1_BLOCK_LARGE;
   if (kern == (const void *)k_cg_mg<CG_MG_BLOCK>) return CG_MG_BLOCK;
   if (kern == (const void *)k_cg_ic) return IC_BLOCK;
+  for (int ref = 0; ref < 2; ref++)
+    for (int e = 1; e <= CGR_CELLS; e *= 2)
+      if (kern == cg_reg_kernel(ref != 0, e)) return CGR_BLOCK;
   return CG_BLOCK;
 }
 
@@ -3749,6 +4000,8 @@ int run_solve(FlipGpu *h, FlipGpuSolveStats *st) {
   sa.h2 = (double)h2f;
   sa.inv_h2 = 1.0 / (double)h2f;
   sa.inv_h2_f = (float)sa.inv_h2;
+  sa.ih = sa.inv_h2_f;
+  sa.il = (float)(sa.inv_h2 - (double)sa.ih);
   const double ref_eps = 1.0e-2 * ((double)n * n * n);
   long cap = h->prm.max_iters > 0 ? h->prm.max_iters : (long)nc;
   /* a multigrid solve that needs more than this has failed: stop early */
@@ -3842,6 +4095,7 @@ int run_solve(FlipGpu *h, FlipGpuSolveStats *st) {
     a.w1 = h->w1;
     a.p = h->pdir;
     a.P = h->P;
+    a.Ps = reinterpret_cast<const float2 *>(h->P + nc);
     a.diag = h->diag;
     a.Pf = h->Pf;
     a.part = (float2 *)h->partial;
@@ -3903,6 +4157,20 @@ int run_solve(FlipGpu *h, FlipGpuSolveStats *st) {
         return FLIPGPU_ECUDA;
       }
     }
+    /* small grids: the cells in registers, as few to a thread as the blocks
+     * allow */
+    int reg_cells = 0;
+    if (mode == FLIPGPU_SOLVE_REF ||
+        (precond == FLIPGPU_PRECOND_JACOBI && kern == (const void *)k_cg<FLIPGPU_SOLVE_FAST>)) {
+      int most = h->cg_grid[6];
+      if (h->solve_blocks > 0 && h->solve_blocks < most) most = h->solve_blocks;
+      for (int e = 1; e <= CGR_CELLS && reg_cells == 0; e *= 2)
+        if (nc <= (size_t)most * CGR_BLOCK * e) reg_cells = e;
+      if (reg_cells > 0) {
+        kern = cg_reg_kernel(mode == FLIPGPU_SOLVE_REF, reg_cells);
+        grid = h->cg_grid[6];
+      }
+    }
     if (precond == FLIPGPU_PRECOND_MG) {
       kern = (const void *)k_cg_mg<CG_MG_BLOCK>;
       grid = h->cg_grid[5];
@@ -3956,7 +4224,7 @@ int run_solve(FlipGpu *h, FlipGpuSolveStats *st) {
      * of the GPU to other simulations */
     if (precond != FLIPGPU_PRECOND_IC) {
       h->solve_capacity = grid;
-      const size_t per_block = (size_t)cg_block_of(kern) * 8;
+      const size_t per_block = (size_t)cg_block_of(kern) * (reg_cells > 0 ? reg_cells : 8);
       const size_t want = (nc + per_block - 1) / per_block;
       if (want < (size_t)grid) grid = want > 0 ? (int)want : 1;
       /* the caller's share of the GPU (flipgpu_set_solve_blocks) */
@@ -4184,7 +4452,7 @@ int ic_init_device() {
 }
 
 /* Cooperative grid of each CG variant (REF, FAST, single-reduction with
- * small blocks, IC, single-reduction with large blocks, MG): SMs x resident
+ * small blocks, IC, single-reduction with large blocks, MG, cells in registers): SMs x resident
  * blocks (at most 4). */
 int cg_grid_size(int *out) {
   int dev = 0, sms = 0, coop = 0;
@@ -4198,7 +4466,7 @@ int cg_grid_size(int *out) {
                                 (const void *)k_cg<FLIPGPU_SOLVE_FAST>,
                                 (const void *)k_cg_cg1<CG1_BLOCK_SMALL>, (const void *)k_cg_ic,
                                 (const void *)k_cg_cg1<CG1_BLOCK_LARGE>,
-                                (const void *)k_cg_mg<CG_MG_BLOCK>};
+                                (const void *)k_cg_mg<CG_MG_BLOCK>, cg_reg_kernel(true, CGR_CELLS)};
   for (int v = 0; v < CG_VARIANTS; v++) {
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(

@@ -221,6 +221,95 @@ RM_FN float axpy_fd(float p, float v, float ch, float cl, double c) {
   return out;
 }
 
+/* ---- the solver's expressions. The pair's error is bounded, and the
+ * rounding is decided when both ends of the error interval round to the same
+ * float; magnitudes outside the given range, zeros and NaN go to the double
+ * expressions. ---- */
+RM_COLD float stencil_d(float s, float x0, float x1, float x2, float x3, float x4, float x5,
+                        double h2, double inv_h2, int pow2) {
+  double v = 6.0 * (double)s;
+  v -= (double)x0;
+  v -= (double)x1;
+  v -= (double)x2;
+  v -= (double)x3;
+  v -= (double)x4;
+  v -= (double)x5;
+  return pow2 ? (float)(v * inv_h2) : (float)(v / h2);
+}
+RM_COLD float ghost_d(float lq, float lc, float s) {
+  return (float)((double)lq / fmin(1.0e-6, (double)lc) * (double)s);
+}
+RM_COLD float scale2_d(float r, double p) { return (float)((double)r * p * p); }
+
+RM_FN bool in_range_f(float x) {
+  float a = fabsf(x);
+  return a > 1.0e-25f && a < 1.0e30f;
+}
+
+/* compute_Ax (src/solver.cpp:29-41) at one cell: (6 s - x0 - .. - x5) / h2 in
+ * double from floats, rounded once; ih + il = 1/h2 as a float pair. The sums'
+ * errors are gathered in lo, whose own roundings stay below 2^-43 of the sum
+ * of the terms' magnitudes. */
+RM_FN float stencil_ref(float s, float x0, float x1, float x2, float x3, float x4, float x5,
+                        float ih, float il, double h2, double inv_h2, int pow2) {
+  float hi, lo, e;
+  two_prod(6.0f, s, hi, lo);
+  const float big = fabsf(hi) + (((fabsf(x0) + fabsf(x1)) + (fabsf(x2) + fabsf(x3))) +
+                                 (fabsf(x4) + fabsf(x5)));
+  two_sum(hi, -x0, hi, e);
+  lo += e;
+  two_sum(hi, -x1, hi, e);
+  lo += e;
+  two_sum(hi, -x2, hi, e);
+  lo += e;
+  two_sum(hi, -x3, hi, e);
+  lo += e;
+  two_sum(hi, -x4, hi, e);
+  lo += e;
+  two_sum(hi, -x5, hi, e);
+  lo += e;
+  float v, vl, m, me;
+  two_sum(hi, lo, v, vl);
+  two_prod(v, ih, m, me);
+  me = fmaf(v, il, fmaf(vl, ih, me));
+  const float err = big * ih * 0x1p-42f;
+  const float up = m + (me + err), dn = m + (me - err);
+  if (!(up == dn) || !in_range_f(up) || !(big < 1.0e30f))
+    return stencil_d(s, x0, x1, x2, x3, x4, x5, h2, inv_h2, pow2);
+  return up;
+}
+
+/* The ghost value of an air neighbour (src/solver.cpp:18-26):
+ * (float)(lq / fmin(1e-6, lc) * s) in double. */
+RM_FN float ghost_ref(float lq, float lc, float s) {
+  if (!(lc < 9.0e-7f) || !in_range_f(lc) || !in_range_f(lq) || !in_range_f(s))
+    return ghost_d(lq, lc, s);
+  const float q = lq / lc;
+  const float ql = fmaf(-q, lc, lq) / lc;
+  float p, e;
+  two_prod(q, s, p, e);
+  e = fmaf(ql, s, e);
+  const float err = fabsf(p) * 0x1p-44f;
+  const float up = p + (e + err), dn = p + (e - err);
+  if (!(up == dn) || !in_range_f(q) || !in_range_f(p)) return ghost_d(lq, lc, s);
+  return up;
+}
+
+/* (float)((double)r * p * p) for a double p = ph + pl + o(2^-47 p): the
+ * reference's preconditioner with no entry equal to 1.0
+ * (src/solver.cpp:141-180). */
+RM_FN float scale2_ref(float r, float ph, float pl, double p) {
+  float a, ae, m, me;
+  two_prod(r, ph, a, ae);
+  ae = fmaf(r, pl, ae);
+  two_prod(a, ph, m, me);
+  me = fmaf(a, pl, fmaf(ae, ph, me));
+  const float err = fabsf(m) * 0x1p-43f;
+  const float up = m + (me + err), dn = m + (me - err);
+  if (!(up == dn) || !in_range_f(r) || !in_range_f(a) || !in_range_f(m)) return scale2_d(r, p);
+  return up;
+}
+
 } // namespace refmath
 
 #endif
