@@ -139,6 +139,50 @@ template <int BLOCK> __device__ __forceinline__ FF block_sum_ff(FF v) {
   return r;
 }
 
+/* A counting grid barrier: bar[0] counts the arrivals of the whole launch
+ * (zeroed before it), so the epoch-th barrier is complete when it reaches
+ * epoch x gridDim.x. Thread 0 arrives with an acquire-release add after the
+ * block's __syncthreads (the last block to arrive reads no more) and polls
+ * with acquire loads: two L2 round trips, no reset and no generation word. The wait gives up after 2 s of %globaltimer,
+ * flags FLIPGPU_ETIMEOUT and returns false in that block (the others give up
+ * at their next barrier). */
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+__device__ __forceinline__ bool count_barrier(unsigned *bar, unsigned &epoch, int *iflags) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    epoch++;
+    const unsigned target = epoch * gridDim.x;
+    unsigned v;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(bar) : "memory");
+    v += 1;
+    bool good = true;
+    unsigned long long t0 = 0;
+    unsigned spins = 0;
+    while ((int)(v - target) < 0) {
+      if ((++spins & 1023u) == 0) {
+        const unsigned long long t = global_ns();
+        if (t0 == 0) {
+          t0 = t;
+        } else if (t - t0 > 2000000000ull) {
+          atomicExch(iflags + IF_TIMEOUT, 1);
+          good = false;
+          break;
+        }
+      }
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+    }
+    ok = good;
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
 __device__ __forceinline__ double ff_to_double(FF v) { return (double)v.hi + (double)v.lo; }
 
 #endif

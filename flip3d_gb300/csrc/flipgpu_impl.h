@@ -234,7 +234,8 @@ enum {
   IF_NWATER,
   IF_NAN,
   IF_TIMEOUT,
-  IF_REPO_LEFT,
+  IF_REPO_LEFT,  /* reposition: stuck particles not yet resampled */
+  IF_REPO_BAR,   /* ... and the barrier of the kernel that resamples them */
   IF_IR_DONE,    /* refinement: 0 running, 1 converged, 2 non-finite, 3 no
                     convergence, 4 zero right-hand side (x = 0) */
   IF_IR_ITERS,   /* refinement: inner CG iterations of all passes */

@@ -608,40 +608,84 @@ __global__ void k_repo_place(SimConst c, const int *__restrict__ counts,
   }
 }
 
-/* corrector::resample (src/corrector.cpp:15-47) at the position of stuck
- * particle q. The reference resamples the stuck particles one after another
- * (src/flip3D.cpp:445-450), so particle q sees the new velocity of every
- * stuck particle q' < q and the old velocity of every q' >= q. `vel_of`
- * supplies a neighbour's velocity under that rule; `dep` is set when a
- * contributing neighbour is a stuck particle q' < q. */
+/* corrector::resample (src/corrector.cpp:15-47) at the position P of stuck
+ * particle q, by one warp. The reference resamples the stuck particles one
+ * after another (src/flip3D.cpp:445-450), so particle q sees the new velocity of
+ * every stuck particle q' < q and the old velocity of every q' >= q. vel_of
+ * supplies a neighbour's velocity under that rule; dep is set when a
+ * contributing neighbour is a stuck particle q' < q. The lanes take 32
+ * consecutive candidates of the 27 cells at a time, in the reference's order;
+ * the contributing ones are then added in that order. */
 template <class V>
-__device__ __forceinline__ float3 repo_resample_one(const SimConst &c, float3 P, uint32_t q,
-                                                    const uint32_t *__restrict__ cs,
-                                                    const uint32_t *__restrict__ perm,
-                                                    const float4 *__restrict__ spos,
-                                                    const uint8_t *__restrict__ stuck,
-                                                    const uint32_t *__restrict__ rank,
-                                                    bool &dep, V vel_of) {
-  int ci = cell_clamp(P.x, c.fn, c.n), cj = cell_clamp(P.y, c.fn, c.n),
-      ck = cell_clamp(P.z, c.fn, c.n);
-  float u[3] = {0.0f, 0.0f, 0.0f};
-  float wsum = 0.0f;
-  visit_cells(c.n, cs, ci - 1, ci + 1, cj - 1, cj + 1, ck - 1, ck + 1, [&](uint32_t b) {
-    float4 Q = spos[b];
-    if (unpack_type(Q.w) != CELL_FLUID) return;
-    float d2 = hypot2_ref(P.x - Q.x, P.y - Q.y, P.z - Q.z);
-    if (!(d2 < c.re_repo_hh)) return; /* weight exactly 0 */
-    float wt = sharp_ref(d2, c.re_repo_hh, c.r2_floor, c.sharp_small_repo);
-    uint32_t o = perm[b];
-    bool is_stuck = stuck[o] != 0;
-    uint32_t ro = is_stuck ? rank[o] : 0xffffffffu;
-    if (is_stuck && ro < q) dep = true;
-    float3 v = vel_of(o, is_stuck, ro);
-    u[0] += wt * v.x;
-    u[1] += wt * v.y;
-    u[2] += wt * v.z;
-    wsum += wt;
-  });
+__device__ __forceinline__ float3 repo_resample_warp(const SimConst &c, float3 P, uint32_t q,
+                                                     const uint32_t *__restrict__ cs,
+                                                     const uint32_t *__restrict__ perm,
+                                                     const float4 *__restrict__ spos,
+                                                     const uint8_t *__restrict__ stuck,
+                                                     const uint32_t *__restrict__ rank, bool &dep,
+                                                     V vel_of) {
+  constexpr unsigned ALL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, n = c.n;
+  const int ci = cell_clamp(P.x, c.fn, n), cj = cell_clamp(P.y, c.fn, n),
+            ck = cell_clamp(P.z, c.fn, n);
+  /* lane r: the run of slots of row (ci - 1 + r / 3, cj - 1 + r % 3) */
+  uint32_t first = 0, len = 0;
+  const int si = ci - 1 + lane / 3, sj = cj - 1 + lane % 3;
+  if (lane < 9 && si >= 0 && si < n && sj >= 0 && sj < n) {
+    const size_t row = ((size_t)si * n + sj) * n;
+    first = __ldg(cs + row + max(ck - 1, 0));
+    len = __ldg(cs + row + min(ck + 1, n - 1) + 1) - first;
+  }
+  uint32_t end = len; /* candidates up to the row's last */
+#pragma unroll
+  for (int o = 1; o < 16; o <<= 1) {
+    const uint32_t v = __shfl_up_sync(ALL, end, o);
+    if (lane >= o) end += v;
+  }
+  const uint32_t total = __shfl_sync(ALL, end, 8), skip = first - (end - len);
+  float u[3] = {0.0f, 0.0f, 0.0f}, wsum = 0.0f;
+  bool seen = false;
+  constexpr int CHUNKS = 4; /* 128 candidates' positions requested at once */
+  for (uint32_t t0 = 0; t0 < total; t0 += 32 * CHUNKS) {
+    uint32_t slot[CHUNKS];
+    float4 Q[CHUNKS];
+#pragma unroll
+    for (int h = 0; h < CHUNKS; h++) {
+      const uint32_t t = t0 + 32 * h + lane;
+      int r = 0; /* t's row */
+#pragma unroll
+      for (int x = 0; x < 8; x++) r += t >= __shfl_sync(ALL, end, x);
+      slot[h] = __shfl_sync(ALL, skip, r) + t;
+      Q[h] = t < total ? __ldg(spos + slot[h]) : make_float4(0, 0, 0, pack_type(CELL_WALL));
+    }
+#pragma unroll
+    for (int h = 0; h < CHUNKS; h++) {
+      bool hit = unpack_type(Q[h].w) == CELL_FLUID;
+      float wt = 0.0f;
+      float3 v = make_float3(0.0f, 0.0f, 0.0f);
+      if (hit) {
+        const float d2 = hypot2_ref(P.x - Q[h].x, P.y - Q[h].y, P.z - Q[h].z);
+        hit = d2 < c.re_repo_hh; /* else the weight is exactly 0 */
+        if (hit) {
+          wt = sharp_ref(d2, c.re_repo_hh, c.r2_floor, c.sharp_small_repo);
+          const uint32_t o = __ldg(perm + slot[h]);
+          const bool is_stuck = __ldg(stuck + o) != 0;
+          const uint32_t ro = is_stuck ? __ldg(rank + o) : 0xffffffffu;
+          if (is_stuck && ro < q) seen = true;
+          v = vel_of(o, is_stuck, ro);
+        }
+      }
+      for (unsigned hits = __ballot_sync(ALL, hit); hits; hits &= hits - 1) {
+        const int src = __ffs(hits) - 1;
+        const float w = __shfl_sync(ALL, wt, src);
+        u[0] += w * __shfl_sync(ALL, v.x, src);
+        u[1] += w * __shfl_sync(ALL, v.y, src);
+        u[2] += w * __shfl_sync(ALL, v.z, src);
+        wsum += w;
+      }
+    }
+  }
+  dep = __any_sync(ALL, seen);
   if (wsum != 0.0f) {
     u[0] /= wsum;
     u[1] /= wsum;
@@ -650,123 +694,94 @@ __device__ __forceinline__ float3 repo_resample_one(const SimConst &c, float3 P,
   return make_float3(u[0], u[1], u[2]);
 }
 
-/* Round 0: every stuck particle with the velocities before the resample.
- * A particle with no earlier stuck particle among its contributing
- * neighbours has its final value (state READY); the others stay PENDING for
- * the later rounds. old[q] keeps the velocity before the resample. */
 enum { RP_PENDING = 0, RP_DONE = 1, RP_READY = 2 };
 
-__global__ void k_repo_gather(SimConst c, const int *__restrict__ counts,
-                              const uint32_t *__restrict__ stuck_idx,
-                              const uint32_t *__restrict__ cs, const uint32_t *__restrict__ perm,
-                              const float4 *__restrict__ spos, const uint8_t *__restrict__ stuck,
-                              const uint32_t *__restrict__ rank, const float *__restrict__ px,
-                              const float *__restrict__ py, const float *__restrict__ pz,
-                              const float *__restrict__ vx, const float *__restrict__ vy,
-                              const float *__restrict__ vz, float4 *__restrict__ res,
-                              float4 *__restrict__ old, uint8_t *__restrict__ state,
-                              int *__restrict__ left) {
-  const int m = counts[IF_NSTUCK], w = counts[IF_NWATER];
-  if (w == 0) return;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += gridDim.x * blockDim.x) {
-    uint32_t p = stuck_idx[q];
-    float3 P = make_float3(px[p], py[p], pz[p]);
-    bool dep = false;
-    float3 u = repo_resample_one(c, P, (uint32_t)q, cs, perm, spos, stuck, rank, dep,
-                                 [&](uint32_t o, bool, uint32_t) {
-                                   return make_float3(vx[o], vy[o], vz[o]);
-                                 });
-    res[q] = make_float4(u.x, u.y, u.z, 0.0f);
-    old[q] = make_float4(vx[p], vy[p], vz[p], 0.0f);
-    state[q] = dep ? RP_PENDING : RP_READY;
-    if (dep) atomicAdd(left, 1);
+/* The resample of the stuck particles, in one cooperative launch. Round 0: every
+ * stuck particle with the velocities before the resample; one with no earlier
+ * stuck particle among its contributing neighbours has its final value
+ * (READY), the others stay PENDING. Each later round computes the PENDING
+ * particles whose earlier stuck neighbours are all DONE: new velocities of
+ * stuck q' < q, old ones of q' > q. The READY values are committed between two
+ * rounds. Whatever is PENDING after the rounds runs in increasing q on one
+ * warp: every earlier stuck particle is final by then. Nearly always round 0
+ * leaves nothing, and the rest is two grid barriers; as 34 launches, one
+ * particle a thread, the chain took 0.25 ms at n = 24. */
+__global__ void __launch_bounds__(BLK)
+k_repo_resample(SimConst c, int *__restrict__ flags, const uint32_t *__restrict__ stuck_idx,
+                const uint32_t *__restrict__ cs, const uint32_t *__restrict__ perm,
+                const float4 *__restrict__ spos, const uint8_t *__restrict__ stuck,
+                const uint32_t *__restrict__ rank, const float *__restrict__ px,
+                const float *__restrict__ py, const float *__restrict__ pz, float *vx, float *vy,
+                float *vz, float4 *res, float4 *old, volatile uint8_t *state) {
+  const int m = flags[IF_NSTUCK], w = flags[IF_NWATER];
+  if (w == 0 || m == 0) return;
+  volatile int *left = flags + IF_REPO_LEFT;
+  unsigned *bar = reinterpret_cast<unsigned *>(flags + IF_REPO_BAR), epoch = 0;
+  const int lane = threadIdx.x & 31, warps = gridDim.x * (BLK / 32);
+  const int gw = blockIdx.x * (BLK / 32) + (threadIdx.x >> 5);
+  auto at = [&](uint32_t p) { return make_float3(px[p], py[p], pz[p]); };
+  auto now = [&](uint32_t o) { return make_float3(vx[o], vy[o], vz[o]); };
+  for (int round = 0; round <= REPO_ROUNDS; round++) {
+    for (int q = gw; q < m; q += warps) {
+      if (round > 0 && state[q] != RP_PENDING) continue;
+      const uint32_t p = stuck_idx[q];
+      bool dep = false, blocked = false;
+      const float3 u = repo_resample_warp(c, at(p), (uint32_t)q, cs, perm, spos, stuck, rank, dep,
+                                          [&](uint32_t o, bool is_stuck, uint32_t ro) {
+                                            if (round > 0 && is_stuck) {
+                                              if (ro >= (uint32_t)q) {
+                                                const float4 v = old[ro];
+                                                return make_float3(v.x, v.y, v.z);
+                                              }
+                                              if (state[ro] != RP_DONE) blocked = true;
+                                            }
+                                            return now(o);
+                                          });
+      const bool wait = round == 0 ? dep : __any_sync(0xffffffffu, blocked);
+      if (lane == 0) {
+        res[q] = make_float4(u.x, u.y, u.z, 0.0f);
+        if (round == 0) {
+          const float3 v = now(p);
+          old[q] = make_float4(v.x, v.y, v.z, 0.0f);
+          if (wait) atomicAdd((int *)left, 1);
+        }
+        if (round == 0 || !wait) state[q] = wait ? RP_PENDING : RP_READY;
+      }
+    }
+    if (!count_barrier(bar, epoch, flags)) return;
+    for (int q = blockIdx.x * BLK + threadIdx.x; q < m; q += gridDim.x * BLK) {
+      if (state[q] != RP_READY) continue;
+      const float4 r = res[q];
+      const uint32_t p = stuck_idx[q];
+      vx[p] = r.x;
+      vy[p] = r.y;
+      vz[p] = r.z;
+      state[q] = RP_DONE;
+      if (round > 0) atomicSub((int *)left, 1);
+    }
+    if (round == 0 && *left == 0) return; /* nothing adds to it after the barrier */
+    if (!count_barrier(bar, epoch, flags)) return;
+    if (*left == 0) return;
   }
-}
-
-/* Later rounds: a PENDING particle whose earlier stuck neighbours are all
- * DONE computes its value — new velocities for stuck q' < q, old ones for
- * q' > q — and becomes READY. */
-__global__ void k_repo_round(SimConst c, const int *__restrict__ counts,
-                             const uint32_t *__restrict__ stuck_idx,
-                             const uint32_t *__restrict__ cs, const uint32_t *__restrict__ perm,
-                             const float4 *__restrict__ spos, const uint8_t *__restrict__ stuck,
-                             const uint32_t *__restrict__ rank, const float *__restrict__ px,
-                             const float *__restrict__ py, const float *__restrict__ pz,
-                             const float *__restrict__ vx, const float *__restrict__ vy,
-                             const float *__restrict__ vz, float4 *__restrict__ res,
-                             const float4 *__restrict__ old, uint8_t *__restrict__ state,
-                             const int *__restrict__ left) {
-  const int m = counts[IF_NSTUCK], w = counts[IF_NWATER];
-  if (w == 0 || *left == 0) return;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += gridDim.x * blockDim.x) {
-    if (state[q] != RP_PENDING) continue;
-    uint32_t p = stuck_idx[q];
-    float3 P = make_float3(px[p], py[p], pz[p]);
-    bool dep = false, blocked = false;
-    float3 u = repo_resample_one(c, P, (uint32_t)q, cs, perm, spos, stuck, rank, dep,
-                                 [&](uint32_t o, bool is_stuck, uint32_t ro) {
-                                   if (is_stuck && ro >= (uint32_t)q) {
-                                     float4 v = old[ro];
-                                     return make_float3(v.x, v.y, v.z);
-                                   }
-                                   if (is_stuck && state[ro] != RP_DONE) blocked = true;
-                                   return make_float3(vx[o], vy[o], vz[o]);
-                                 });
-    if (blocked) continue;
-    res[q] = make_float4(u.x, u.y, u.z, 0.0f);
-    state[q] = RP_READY;
-  }
-}
-
-__global__ void k_repo_commit(const int *__restrict__ counts,
-                              const uint32_t *__restrict__ stuck_idx,
-                              const float4 *__restrict__ res, uint8_t *__restrict__ state,
-                              float *__restrict__ vx, float *__restrict__ vy,
-                              float *__restrict__ vz, int *__restrict__ left, int round) {
-  const int m = counts[IF_NSTUCK], w = counts[IF_NWATER];
-  if (w == 0 || (round > 0 && *left == 0)) return;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += gridDim.x * blockDim.x) {
-    if (state[q] != RP_READY) continue;
-    float4 r = res[q];
-    uint32_t p = stuck_idx[q];
-    vx[p] = r.x;
-    vy[p] = r.y;
-    vz[p] = r.z;
-    state[q] = RP_DONE;
-    if (round > 0) atomicSub(left, 1);
-  }
-}
-
-/* Whatever is still PENDING after the rounds, in increasing q on one
- * thread: every earlier stuck particle is final by then. */
-__global__ void k_repo_ordered(SimConst c, const int *__restrict__ counts,
-                               const uint32_t *__restrict__ stuck_idx,
-                               const uint32_t *__restrict__ cs, const uint32_t *__restrict__ perm,
-                               const float4 *__restrict__ spos, const uint8_t *__restrict__ stuck,
-                               const uint32_t *__restrict__ rank, const float *__restrict__ px,
-                               const float *__restrict__ py, const float *__restrict__ pz,
-                               float *__restrict__ vx, float *__restrict__ vy,
-                               float *__restrict__ vz, const float4 *__restrict__ old,
-                               const uint8_t *__restrict__ state, const int *__restrict__ left) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const int m = counts[IF_NSTUCK], w = counts[IF_NWATER];
-  if (w == 0 || *left == 0) return;
+  if (gw != 0) return;
   for (int q = 0; q < m; q++) {
     if (state[q] == RP_DONE) continue;
-    uint32_t p = stuck_idx[q];
-    float3 P = make_float3(px[p], py[p], pz[p]);
+    const uint32_t p = stuck_idx[q];
     bool dep = false;
-    float3 u = repo_resample_one(c, P, (uint32_t)q, cs, perm, spos, stuck, rank, dep,
-                                 [&](uint32_t o, bool is_stuck, uint32_t ro) {
-                                   if (is_stuck && ro >= (uint32_t)q) {
-                                     float4 v = old[ro];
-                                     return make_float3(v.x, v.y, v.z);
-                                   }
-                                   return make_float3(vx[o], vy[o], vz[o]);
-                                 });
-    vx[p] = u.x;
-    vy[p] = u.y;
-    vz[p] = u.z;
+    const float3 u = repo_resample_warp(c, at(p), (uint32_t)q, cs, perm, spos, stuck, rank, dep,
+                                        [&](uint32_t o, bool is_stuck, uint32_t ro) {
+                                          if (is_stuck && ro >= (uint32_t)q) {
+                                            const float4 v = old[ro];
+                                            return make_float3(v.x, v.y, v.z);
+                                          }
+                                          return now(o);
+                                        });
+    if (lane == 0) {
+      vx[p] = u.x;
+      vy[p] = u.y;
+      vz[p] = u.z;
+    }
+    __syncwarp();
   }
 }
 
@@ -1404,27 +1419,25 @@ cudaError_t launch_reposition(FlipGpu *h, int *stuck_host, bool in_step) {
   /* sorter::sort (src/flip3D.cpp:443), shared with the corrector's sort. */
   if ((e = launch_sort(h, 0, in_step ? 0 : PL_ALL)) != cudaSuccess) return e;
   /* corrector::resample of each stuck particle in order (src/flip3D.cpp:445-450) */
-  int *left = h->iflags + IF_REPO_LEFT;
-  if ((e = cudaMemsetAsync(left, 0, sizeof(int), h->stream)) != cudaSuccess) return e;
-  k_repo_gather<<<REPO_GRID, BLK, 0, h->stream>>>(
-      c, h->iflags, h->stuck_idx, h->cell_start, h->perm, h->spos, h->flag, h->scan_a, h->px,
-      h->py, h->pz, h->vx, h->vy, h->vz, h->repo_res, h->repo_old, h->repo_state, left);
-  k_repo_commit<<<REPO_GRID, BLK, 0, h->stream>>>(h->iflags, h->stuck_idx, h->repo_res,
-                                                  h->repo_state, h->vx, h->vy, h->vz, left, 0);
-  FG_LAUNCHED(h, 2);
-  for (int r = 1; r <= REPO_ROUNDS; r++) {
-    k_repo_round<<<REPO_GRID, BLK, 0, h->stream>>>(
-        c, h->iflags, h->stuck_idx, h->cell_start, h->perm, h->spos, h->flag, h->scan_a, h->px,
-        h->py, h->pz, h->vx, h->vy, h->vz, h->repo_res, h->repo_old, h->repo_state, left);
-    k_repo_commit<<<REPO_GRID, BLK, 0, h->stream>>>(h->iflags, h->stuck_idx, h->repo_res,
-                                                    h->repo_state, h->vx, h->vy, h->vz, left, r);
-    FG_LAUNCHED(h, 2);
+  static_assert(IF_REPO_BAR == IF_REPO_LEFT + 1, "cleared together");
+  if ((e = cudaMemsetAsync(h->iflags + IF_REPO_LEFT, 0, 2 * sizeof(int), h->stream)) !=
+      cudaSuccess)
+    return e;
+  {
+    int *flags = h->iflags;
+    float4 *res = h->repo_res, *old = h->repo_old;
+    uint8_t *state = h->repo_state;
+    void *args[] = {&c,     &flags, &h->stuck_idx, &h->cell_start, &h->perm, &h->spos,
+                    &h->flag, &h->scan_a, &h->px, &h->py, &h->pz, &h->vx, &h->vy, &h->vz,
+                    &res,   &old,   &state};
+    /* a warp for about every 512 particles, at most two blocks an SM */
+    const unsigned want = grid_for(h->np, 512 * (BLK / 32));
+    const unsigned g = want < 2 * 152 ? want : 2 * 152;
+    e = cudaLaunchCooperativeKernel((const void *)k_repo_resample, dim3(g), dim3(BLK), args, 0,
+                                    h->stream);
+    FG_LAUNCHED(h, 1);
+    if (e != cudaSuccess) return e;
   }
-  k_repo_ordered<<<1, 32, 0, h->stream>>>(c, h->iflags, h->stuck_idx, h->cell_start, h->perm,
-                                          h->spos, h->flag, h->scan_a, h->px, h->py, h->pz,
-                                          h->vx, h->vy, h->vz, h->repo_old, h->repo_state, left);
-  FG_LAUNCHED(h, 1);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   /* refresh the sorted velocities of the resampled particles (positions,
    * grid positions and densities are those of the sort above); in a step only
    * the corrector's resample reads them */
