@@ -240,6 +240,7 @@ enum {
                     convergence, 4 zero right-hand side (x = 0) */
   IF_IR_ITERS,   /* refinement: inner CG iterations of all passes */
   IF_IR_PASS,    /* refinement: inner solves run */
+  IF_IR_TICKET,  /* refinement: blocks of the residual that have finished */
   IF_COUNT
 };
 

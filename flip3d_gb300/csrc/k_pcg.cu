@@ -3566,6 +3566,84 @@ constexpr double IR_INNER_FLOOR = 1e-3; /* tightest inner tolerance asked for:
 
 constexpr int IR_BLOCKS = 4 * RED_BLOCKS; /* residual blocks (partials: 2 x IR_BLOCKS <= 8192) */
 
+/* What the outer loop of the refinement decides by. */
+struct IrCheck {
+  double rel_tol, floor_tol;
+  int max_passes;
+  double *scal;
+};
+
+/* The true r.r (and b.b) in a fixed tree over the residual's block partials,
+ * then the outer loop's decision: converged, failed, or the next inner solve's
+ * relative tolerance, aimed at half the remaining reduction and no tighter
+ * than IR_INNER_FLOOR. One block of BLK threads, the last of the residual's (as
+ * a launch of its own it took 8 us of every pass). The tree has RED_BLOCKS
+ * leaves of IR_BLOCKS / RED_BLOCKS partials in order, leaf t paired with leaf
+ * t + w, whatever the number of blocks: absent partials are zero. */
+template <bool FIRST>
+__device__ __forceinline__ void ir_check(const IrCheck &k, const double *part, int *iflags) {
+  constexpr int PER = IR_BLOCKS / RED_BLOCKS, LEAVES = RED_BLOCKS / BLK;
+  __shared__ double sh[BLK], sb[FIRST ? BLK : 1];
+  double a[LEAVES], bs[LEAVES];
+#pragma unroll
+  for (int l = 0; l < LEAVES; l++) {
+    a[l] = bs[l] = 0.0;
+#pragma unroll
+    for (int q = 0; q < PER; q++) {
+      const unsigned i = (threadIdx.x + l * BLK) * PER + q;
+      if (i < gridDim.x) {
+        a[l] += __ldcg(part + i);
+        if (FIRST) bs[l] += __ldcg(part + IR_BLOCKS + i);
+      }
+    }
+  }
+#pragma unroll
+  for (int w = LEAVES / 2; w > 0; w >>= 1)
+#pragma unroll
+    for (int l = 0; l < w; l++) {
+      a[l] += a[l + w];
+      bs[l] += bs[l + w];
+    }
+  sh[threadIdx.x] = a[0];
+  if (FIRST) sb[threadIdx.x] = bs[0];
+  __syncthreads();
+  for (int w = BLK / 2; w >= 32; w >>= 1) {
+    if ((int)threadIdx.x < w) {
+      sh[threadIdx.x] += sh[threadIdx.x + w];
+      if (FIRST) sb[threadIdx.x] += sb[threadIdx.x + w];
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x >= 32) return;
+  double rr = sh[threadIdx.x], b2 = FIRST ? sb[threadIdx.x] : 0.0;
+  for (int w = 16; w > 0; w >>= 1) {
+    rr += __shfl_down_sync(0xffffffffu, rr, w);
+    if (FIRST) b2 += __shfl_down_sync(0xffffffffu, b2, w);
+  }
+  if (threadIdx.x != 0) return;
+  double *scal = k.scal;
+  if (FIRST)
+    scal[SC_IR_B2] = b2;
+  else
+    b2 = scal[SC_IR_B2];
+  scal[SC_TRUE2] = rr;
+  const int pass = iflags[IF_IR_PASS];
+  int done = 0;
+  if (!(rr == rr) || !(b2 == b2)) done = 2;
+  else if (b2 == 0.0) done = 4;
+  else if (rr <= k.rel_tol * k.rel_tol * b2) done = 1;
+  else if (pass >= k.max_passes) done = 3;
+  else if (pass > 0 && rr > 0.81 * scal[SC_IR_PREV]) done = 3; /* < 10 % per pass: stalled */
+  if (done) {
+    iflags[IF_IR_DONE] = done;
+    return;
+  }
+  double t = 0.5 * k.rel_tol * sqrt(b2 / rr);
+  t = t < k.floor_tol ? k.floor_tol : (t > 0.5 ? 0.5 : t);
+  scal[SC_IR_TOL] = t;
+  scal[SC_IR_PREV] = rr;
+}
+
 /* r = b - A (xhi + xlo) on the liquid, rb = float(r), e = 0, and the block
  * partials of r.r (and, on the first pass, b.b). The first pass starts from
  * xlo = 0 and zeroes x off the liquid, as every FAST solve leaves it. */
@@ -3573,8 +3651,8 @@ template <bool FIRST>
 __global__ void __launch_bounds__(BLK)
 k_ir_residual(SolveArgs s, const uint8_t *__restrict__ A, const float *__restrict__ diag,
               const float *__restrict__ b, float *__restrict__ xhi, float *__restrict__ xlo,
-              float *__restrict__ rb, float *__restrict__ e, const int *__restrict__ iflags,
-              double *__restrict__ part) {
+              float *__restrict__ rb, float *__restrict__ e, int *__restrict__ iflags,
+              double *__restrict__ part, IrCheck chk) {
   if (!FIRST && *(volatile const int *)(iflags + IF_IR_DONE)) return;
   const int n = s.n;
   const size_t nc = (size_t)n * n * n;
@@ -3625,53 +3703,16 @@ k_ir_residual(SolveArgs s, const uint8_t *__restrict__ A, const float *__restric
     const FF t2 = block_sum_ff<BLK>(bb);
     if (threadIdx.x == 0) part[IR_BLOCKS + blockIdx.x] = ff_to_double(t2);
   }
-}
-
-/* One block of RED_BLOCKS threads: the true r.r (and b.b) in a fixed tree,
- * then the outer loop's decision: converged, failed, or the next inner
- * solve's relative tolerance, aimed at half the remaining reduction and no
- * tighter than IR_INNER_FLOOR. */
-__global__ void __launch_bounds__(RED_BLOCKS)
-k_ir_check(int first, double rel_tol, int max_passes, double floor_tol,
-           const double *__restrict__ part, double *__restrict__ scal, int *__restrict__ iflags) {
-  __shared__ double sh[RED_BLOCKS], sb[RED_BLOCKS];
-  if (!first && iflags[IF_IR_DONE]) return;
-  /* each thread first adds IR_BLOCKS / RED_BLOCKS partials in order */
-  double a = 0.0, bsum = 0.0;
-  for (int q = 0; q < IR_BLOCKS / RED_BLOCKS; q++) {
-    a += part[threadIdx.x * (IR_BLOCKS / RED_BLOCKS) + q];
-    if (first) bsum += part[IR_BLOCKS + threadIdx.x * (IR_BLOCKS / RED_BLOCKS) + q];
+  /* the last block to finish decides */
+  __shared__ int last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(iflags + IF_IR_TICKET, 1) == (int)gridDim.x - 1;
+    if (last) iflags[IF_IR_TICKET] = 0;
+    __threadfence();
   }
-  sh[threadIdx.x] = a;
-  sb[threadIdx.x] = bsum;
   __syncthreads();
-  for (int w = RED_BLOCKS / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      sh[threadIdx.x] += sh[threadIdx.x + w];
-      sb[threadIdx.x] += sb[threadIdx.x + w];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x != 0) return;
-  const double rr = sh[0];
-  if (first) scal[SC_IR_B2] = sb[0];
-  const double b2 = scal[SC_IR_B2];
-  scal[SC_TRUE2] = rr;
-  const int pass = iflags[IF_IR_PASS];
-  int done = 0;
-  if (!(rr == rr) || !(b2 == b2)) done = 2;
-  else if (b2 == 0.0) done = 4;
-  else if (rr <= rel_tol * rel_tol * b2) done = 1;
-  else if (pass >= max_passes) done = 3;
-  else if (pass > 0 && rr > 0.81 * scal[SC_IR_PREV]) done = 3; /* < 10 % per pass: stalled */
-  if (done) {
-    iflags[IF_IR_DONE] = done;
-    return;
-  }
-  double t = 0.5 * rel_tol * sqrt(b2 / rr);
-  t = t < floor_tol ? floor_tol : (t > 0.5 ? 0.5 : t);
-  scal[SC_IR_TOL] = t;
-  scal[SC_IR_PREV] = rr;
+  if (last) ir_check<FIRST>(chk, part, iflags);
 }
 
 /* x += e after an inner solve (double-float add), unless the inner solve
@@ -4222,12 +4263,11 @@ int run_solve(FlipGpu *h, FlipGpuSolveStats *st) {
         const double v = atof(ev);
         if (v > 0.0 && v < 1.0) floor_tol = v;
       }
-      k_ir_residual<true><<<IR_BLOCKS, BLK, 0, S>>>(sa, h->A, h->diag, h->div, h->press,
-                                                      h->press_lo, h->ir_b, h->ir_e, h->iflags,
-                                                      h->partial);
-      k_ir_check<<<1, RED_BLOCKS, 0, S>>>(1, h->prm.rel_tol, passes, floor_tol, h->partial,
-                                          h->scal, h->iflags);
-      FG_LAUNCHED(h, 2);
+      const IrCheck chk = {h->prm.rel_tol, floor_tol, passes, h->scal};
+      const unsigned rg = grid_for(nc, BLK) < IR_BLOCKS ? grid_for(nc, BLK) : IR_BLOCKS;
+      k_ir_residual<true><<<rg, BLK, 0, S>>>(sa, h->A, h->diag, h->div, h->press, h->press_lo,
+                                             h->ir_b, h->ir_e, h->iflags, h->partial, chk);
+      FG_LAUNCHED(h, 1);
       for (int pass = 0; pass < passes; pass++) {
         if (pass > 0) reset_flags();
         a.ic_factor = pass == 0;
@@ -4240,12 +4280,9 @@ int run_solve(FlipGpu *h, FlipGpuSolveStats *st) {
           return FLIPGPU_ECUDA;
         }
         k_ir_update<<<ug, BLK, 0, S>>>(nc, h->A, h->ir_e, h->press, h->press_lo, h->iflags);
-        k_ir_residual<false><<<IR_BLOCKS, BLK, 0, S>>>(sa, h->A, h->diag, h->div, h->press,
-                                                         h->press_lo, h->ir_b, h->ir_e,
-                                                         h->iflags, h->partial);
-        k_ir_check<<<1, RED_BLOCKS, 0, S>>>(0, h->prm.rel_tol, passes, floor_tol, h->partial,
-                                            h->scal, h->iflags);
-        FG_LAUNCHED(h, 3);
+        k_ir_residual<false><<<rg, BLK, 0, S>>>(sa, h->A, h->diag, h->div, h->press, h->press_lo,
+                                                h->ir_b, h->ir_e, h->iflags, h->partial, chk);
+        FG_LAUNCHED(h, 2);
       }
       h->press_lo_valid = 1;
       if (h->async_mode) return FLIPGPU_OK; /* stats stay on the device (read_solve_stats) */
