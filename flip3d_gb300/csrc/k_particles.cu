@@ -238,8 +238,9 @@ k_density(SimConst c, const uint32_t *__restrict__ cs, const uint32_t *__restric
  * tangent cell j-2 lies at least 1.5 cells from the face centre, beyond the
  * kernel radius RE=1.4, so its weights are exactly 0 and it is skipped.
  * Writes the saved grid (save_grid) and the boundary-enforced grid
- * (enforce_boundary, src/flip3D.cpp:783-805) in one pass. */
-template <class AR>
+ * (enforce_boundary, src/flip3D.cpp:783-805) in one pass. AHEAD requests the
+ * next candidate of a run, its velocity too, before the present one is used. */
+template <class AR, bool AHEAD>
 __global__ void __launch_bounds__(BLK)
 k_p2g(SimConst c, int enforce, const uint32_t *__restrict__ cs, const float4 *__restrict__ spg,
       const float4 *__restrict__ svel, const uint8_t *__restrict__ A, float *__restrict__ u0,
@@ -263,17 +264,42 @@ k_p2g(SimConst c, int enforce, const uint32_t *__restrict__ cs, const float4 *__
   if (comp == 2) { fp[2] = (float)k; hi[2] = k; }
   const float hh = c.re_p2g_hh;
   float sumw = 0.0f, sumx = 0.0f;
-  visit_cells(n, cs, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], [&](uint32_t b) {
-    float4 Q = __ldg(spg + b);
-    if (unpack_type(Q.w) != CELL_FLUID) return;
+  auto add = [&](float4 Q, auto velocity) {
     float r2 = AR::hypot2(Q.x - fp[0], Q.y - fp[1], Q.z - fp[2]);
     if (!(r2 < hh)) return; /* weight exactly 0 */
     float w = AR::sharp(r2, hh, c.r2_floor, c.sharp_small_p2g);
-    float4 V = __ldg(svel + b);
+    const float4 V = velocity();
     float vc = comp == 0 ? V.x : (comp == 1 ? V.y : V.z);
     sumx += w * vc;
     sumw += w;
-  });
+  };
+  if (AHEAD) {
+    const int k0 = max(lo[2], 0), k1 = min(hi[2], n - 1);
+    for (int si = max(lo[0], 0); si <= min(hi[0], n - 1); si++)
+      for (int sj = max(lo[1], 0); sj <= min(hi[1], n - 1); sj++) {
+        if (k0 > k1) continue;
+        const size_t row = ((size_t)si * n + sj) * n;
+        const uint32_t a = __ldg(cs + row + k0), e = __ldg(cs + row + k1 + 1);
+        float4 Qn = make_float4(0, 0, 0, 0), Vn = Qn;
+        if (a < e) {
+          Qn = __ldg(spg + a);
+          Vn = __ldg(svel + a);
+        }
+        for (uint32_t b = a; b < e; b++) {
+          const float4 Q = Qn, V = Vn;
+          if (b + 1 < e) {
+            Qn = __ldg(spg + b + 1);
+            Vn = __ldg(svel + b + 1);
+          }
+          if (unpack_type(Q.w) == CELL_FLUID) add(Q, [&]() { return V; });
+        }
+      }
+  } else {
+    visit_cells(n, cs, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], [&](uint32_t b) {
+      const float4 Q = __ldg(spg + b);
+      if (unpack_type(Q.w) == CELL_FLUID) add(Q, [&]() { return __ldg(svel + b); });
+    });
+  }
   float val = (sumw != 0.0f) ? sumx / sumw : 0.0f;
   /* enforce_boundary */
   int a = comp == 0 ? i : (comp == 1 ? j : k);
@@ -947,8 +973,8 @@ __device__ __forceinline__ void cell_decode(size_t c, int n, int &i, int &j, int
  * when j, k < n; u1 when i, k < n; u2 when i, j < n). Their neighbourhoods
  * lie in cells [i-1, i+1] x [j-1, j+1] x [k-1, k+1]: each particle there is
  * loaded once and tested against each face whose own cells hold it, which
- * keeps every face's sums in k_p2g's order. */
-template <class AR, int B = BLK>
+ * keeps every face's sums in k_p2g's order. AHEAD as in k_p2g. */
+template <class AR, bool AHEAD, int B = BLK>
 __global__ void __launch_bounds__(B)
 k_p2g_cells(SimConst c, int enforce, const uint32_t *__restrict__ cs,
             const float4 *__restrict__ spg, const float4 *__restrict__ svel,
@@ -976,8 +1002,18 @@ k_p2g_cells(SimConst c, int enforce, const uint32_t *__restrict__ cs,
         const uint32_t a = __ldg(cs + base + k0), b = __ldg(cs + base + k1 + 1);
         /* u2's cells stop at k: the particles of cell k+1 are not its */
         const uint32_t split = k + 1 <= k1 ? __ldg(cs + base + k + 1) : b;
+        float4 Qn = make_float4(0, 0, 0, 0), Vn = Qn;
+        if (AHEAD && a < b) {
+          Qn = __ldg(spg + a);
+          Vn = __ldg(svel + a);
+        }
         for (uint32_t x = a; x < b; x++) {
-          const float4 Q = __ldg(spg + x);
+          const float4 Q = AHEAD ? Qn : __ldg(spg + x);
+          const float4 Va = Vn;
+          if (AHEAD && x + 1 < b) {
+            Qn = __ldg(spg + x + 1);
+            Vn = __ldg(svel + x + 1);
+          }
           if (unpack_type(Q.w) != CELL_FLUID) continue;
           float w[3] = {0.0f, 0.0f, 0.0f};
           bool acc[3] = {false, false, false};
@@ -1003,7 +1039,7 @@ k_p2g_cells(SimConst c, int enforce, const uint32_t *__restrict__ cs,
             }
           }
           if (!(acc[0] || acc[1] || acc[2])) continue;
-          const float4 V = __ldg(svel + x);
+          const float4 V = AHEAD ? Va : __ldg(svel + x);
           if (acc[0]) {
             sx[0] += w[0] * V.x;
             sw[0] += w[0];
@@ -1291,26 +1327,46 @@ cudaError_t launch_density(FlipGpu *h) {
   return cudaGetLastError();
 }
 
+/* Which P2G kernel a grid takes (all give the same bits; us at n = 24, 48, 64,
+ * 96, 128 on pool scenes):
+ *   a face a thread, next candidate requested ahead    43   84  141  371  837
+ *   a face cell a thread, ahead                        94  110  143  297  593
+ *   a face cell a thread                              119  132  152  317  572
+ * Small grids leave SMs idle and wait for each candidate's loads in turn, so
+ * they take more threads and overlap the loads; large ones are bound by the L1
+ * data pipe and take the fewest loads. */
+constexpr int P2G_FACES_N = 64, P2G_AHEAD_N = 112;
+
 cudaError_t launch_p2g(FlipGpu *h, int enforce) {
   SimConst c = make_const(h);
-  if (cell_gathers(h)) {
+  auto go = [&](auto kernel, unsigned grid, int block) {
+    kernel<<<grid, block, 0, h->stream>>>(c, enforce, h->cell_start, h->spg, h->svel, h->A, h->u[0],
+                                          h->u[1], h->u[2], h->us[0], h->us[1], h->us[2]);
+  };
+  const bool faces = !cell_gathers(h) || h->n < P2G_FACES_N;
+  if (!faces) {
     const size_t m1 = (size_t)h->n + 1, cells = m1 * m1 * m1;
     return tuned_gather(h, "k_p2g_cells", cells, [&](auto B) {
       constexpr int b = decltype(B)::value;
-      k_p2g_cells<FastArith, b><<<grid_for(cells, b), b, 0, h->stream>>>(
-          c, enforce, h->cell_start, h->spg, h->svel, h->A, h->u[0], h->u[1], h->u[2], h->us[0],
-          h->us[1], h->us[2]);
+      if (h->n < P2G_AHEAD_N)
+        go(k_p2g_cells<FastArith, true, b>, grid_for(cells, b), b);
+      else
+        go(k_p2g_cells<FastArith, false, b>, grid_for(cells, b), b);
     });
   }
   const unsigned grid = 3u * grid_for(h->nf, BLK);
-  if (h->prm.arith == FLIPGPU_ARITH_FAST)
-    k_p2g<FastArith><<<grid, BLK, 0, h->stream>>>(c, enforce, h->cell_start, h->spg, h->svel,
-                                                  h->A, h->u[0], h->u[1], h->u[2], h->us[0],
-                                                  h->us[1], h->us[2]);
-  else
-    k_p2g<RefArith><<<grid, BLK, 0, h->stream>>>(c, enforce, h->cell_start, h->spg, h->svel,
-                                                 h->A, h->u[0], h->u[1], h->u[2], h->us[0],
-                                                 h->us[1], h->us[2]);
+  const bool fast = h->prm.arith == FLIPGPU_ARITH_FAST;
+  if (h->n < P2G_FACES_N && cell_gathers(h)) {
+    ktime_begin(h, "k_p2g_cells"); /* the kernel clock's name of the FAST P2G */
+    go(k_p2g<FastArith, true>, grid, BLK);
+    ktime_end(h);
+  } else if (h->n < P2G_FACES_N && !fast) {
+    go(k_p2g<RefArith, true>, grid, BLK);
+  } else if (fast) {
+    go(k_p2g<FastArith, false>, grid, BLK);
+  } else {
+    go(k_p2g<RefArith, false>, grid, BLK);
+  }
   FG_LAUNCHED(h, 1);
   return cudaGetLastError();
 }
