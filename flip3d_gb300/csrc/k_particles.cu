@@ -231,6 +231,136 @@ k_density(SimConst c, const uint32_t *__restrict__ cs, const uint32_t *__restric
   sdens[a] = d;
 }
 
+/* two floats in one 64-bit register pair and the packed FP32 operations on
+ * them (each half rounds like the scalar instruction): half the issue slots */
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_get(F2 x, float &a, float &b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+/* a * b + c clamped to [0, 1] (0 for NaN) by the instruction's saturation */
+__device__ __forceinline__ float fma_sat(float a, float b, float c) {
+  float r;
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+/* computeDensity in FAST arithmetic with two particles of a cell a thread:
+ * k_density's sums, terms and order for each of them. A candidate is loaded once
+ * for both, and the products and the sum run packed. With a particle a thread
+ * the loads bound the kernel (the L1 data pipe at 85 to 91 % of its peak);
+ * 1.44 -> 0.96 ms at n = 160 (10.5M particles). The block's cells are a tile of
+ * 4 x 4 x 8: their candidates, 6 x 6 runs of ten cells, stay in L1, and the
+ * pairs of all 128 cells are shared out to the block's threads, 288 for about
+ * 544 pairs at eight particles a cell (128, 192 and 256 threads: 1.05, 0.98,
+ * 0.99 ms; four particles a thread: the same; tiles of 4 x 4 x 16 and 2 x 4 x
+ * 8: slower). */
+constexpr int CT_I = 4, CT_J = 4, CT_K = 8, CT_CELLS = CT_I * CT_J * CT_K;
+constexpr int CT_BLOCK = 288;
+
+inline unsigned cell_tiles(int n) {
+  const unsigned a = (unsigned)(n + CT_I - 1) / CT_I, b = (unsigned)(n + CT_K - 1) / CT_K;
+  return a * a * b;
+}
+
+__global__ void __launch_bounds__(CT_BLOCK)
+k_density_tile(SimConst c, const uint32_t *__restrict__ cs, const uint32_t *__restrict__ perm,
+               const float4 *__restrict__ spos, float *__restrict__ dens,
+               float *__restrict__ sdens) {
+  /* off[q]: the pairs of the tile's cells before cell q; first[q]: its first slot */
+  __shared__ uint32_t off[CT_CELLS + 1], first[CT_CELLS], warp_pairs[CT_CELLS / 32];
+  static_assert(CT_BLOCK >= CT_CELLS, "a thread a cell");
+  const int n = c.n, lane = threadIdx.x & 31;
+  const unsigned tj = (unsigned)(n + CT_J - 1) / CT_J, tk = (unsigned)(n + CT_K - 1) / CT_K;
+  const unsigned line = blockIdx.x / tk;
+  const int i0 = (int)(line / tj) * CT_I, j0 = (int)(line % tj) * CT_J,
+            k0 = (int)(blockIdx.x % tk) * CT_K;
+  uint32_t upto = 0;
+  if (threadIdx.x < CT_CELLS) {
+    const int q = threadIdx.x, i = i0 + q / (CT_J * CT_K), j = j0 + q / CT_K % CT_J,
+              k = k0 + q % CT_K;
+    if (i < n && j < n && k < n) {
+      const size_t cell = cell_id(n, i, j, k);
+      first[q] = __ldg(cs + cell);
+      upto = (__ldg(cs + cell + 1) - first[q] + 1) / 2;
+    }
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += y;
+    }
+    if (lane == 31) warp_pairs[q / 32] = upto;
+  }
+  __syncthreads();
+  if (threadIdx.x < CT_CELLS) {
+    for (int w = 0; w < (int)threadIdx.x / 32; w++) upto += warp_pairs[w];
+    off[threadIdx.x + 1] = upto;
+    if (threadIdx.x == 0) off[0] = 0;
+  }
+  __syncthreads();
+  for (uint32_t t = threadIdx.x; t < off[CT_CELLS]; t += CT_BLOCK) {
+    int q = 0; /* the cell of pair t: the last with off[q] <= t */
+#pragma unroll
+    for (int w = CT_CELLS / 2; w > 0; w >>= 1)
+      if (off[q + w] <= t) q += w;
+    const int i = i0 + q / (CT_J * CT_K), j = j0 + q / CT_K % CT_J, k = k0 + q % CT_K;
+    const uint32_t s = first[q] + 2 * (t - off[q]);
+    const bool two = s + 1 < __ldg(cs + cell_id(n, i, j, k) + 1);
+    const float4 P = __ldg(spos + s), R = two ? __ldg(spos + s + 1) : P;
+    const bool wall = unpack_type(P.w) == CELL_WALL, wall2 = unpack_type(R.w) == CELL_WALL;
+    F2 sum = f2(0.0f, 0.0f);
+    if (!(wall && wall2)) {
+      const int ka = max(k - 1, 0), kb = min(k + 1, n - 1);
+      for (int si = max(i - 1, 0); si <= min(i + 1, n - 1); si++)
+        for (int sj = max(j - 1, 0); sj <= min(j + 1, n - 1); sj++) {
+          const size_t row = ((size_t)si * n + sj) * n;
+          const uint32_t e = __ldg(cs + row + kb + 1);
+          for (uint32_t b = __ldg(cs + row + ka); b < e; b++) {
+            const float4 Q = __ldg(spos + b);
+            /* a wall particle weighs nothing: out of reach of any other */
+            const float x = unpack_type(Q.w) == CELL_WALL ? INFINITY : Q.x;
+            const F2 dx = f2(x - P.x, x - R.x), dy = f2(Q.y - P.y, Q.y - R.y),
+                     dz = f2(Q.z - P.z, Q.z - R.z);
+            const F2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
+            float ra, rb;
+            f2_get(r2, ra, rb);
+            sum = f2_add(sum, f2(fma_sat(-ra, c.kd_inv, 1.0f), fma_sat(-rb, c.kd_inv, 1.0f)));
+          }
+        }
+    }
+    float w, w2;
+    f2_get(sum, w, w2);
+    const float d = wall ? 1.0f : w / c.max_dens;
+    dens[__ldg(perm + s)] = d;
+    sdens[s] = d;
+    if (two) {
+      const float d2 = wall2 ? 1.0f : w2 / c.max_dens;
+      dens[__ldg(perm + s + 1)] = d2;
+      sdens[s + 1] = d2;
+    }
+  }
+}
+
 /* ------------------------------------------------------------ mapP2G */
 
 /* One MAC face per thread (src/mapper.cpp:17-88). The reference gathers
@@ -1312,9 +1442,21 @@ static cudaError_t tuned_gather(FlipGpu *h, const char *kernel, size_t threads, 
   return err;
 }
 
+constexpr int DENSITY_TILE_N = 64;
+
 cudaError_t launch_density(FlipGpu *h) {
   if (h->np == 0) return cudaSuccess;
   SimConst c = make_const(h);
+  /* the tile kernel pays from n = 64 (85 against 98 us; at n = 48 its blocks are
+   * too few, 56 against 49); both give the same bits */
+  if (cell_gathers(h) && h->n >= DENSITY_TILE_N) {
+    ktime_begin(h, "k_density");
+    k_density_tile<<<cell_tiles(h->n), CT_BLOCK, 0, h->stream>>>(c, h->cell_start, h->perm, h->spos,
+                                                                 h->dens, h->sdens);
+    ktime_end(h);
+    FG_LAUNCHED(h, 1);
+    return cudaGetLastError();
+  }
   if (h->prm.arith == FLIPGPU_ARITH_FAST)
     return tuned_gather(h, "k_density", h->np, [&](auto B) {
       constexpr int b = decltype(B)::value;
