@@ -387,7 +387,7 @@ int flipgpu_create(const FlipGpuParams *p, FlipGpu **out) {
   AL(h->px, cap) AL(h->py, cap) AL(h->pz, cap) AL(h->vx, cap) AL(h->vy, cap) AL(h->vz, cap)
   AL(h->dens, cap) AL(h->type, cap) AL(h->nx, cap) AL(h->ny, cap) AL(h->nz, cap)
   AL(h->key, cap) AL(h->rank, cap) AL(h->perm, cap) AL(h->cell_start, nc + 1)
-  AL(h->cell_count, nc + 1) AL(h->spos, cap) AL(h->spg, cap) AL(h->svel, cap)
+  AL(h->cell_count, nc + 1) AL(h->spos, cap + 3 /* read ahead by the corrector */) AL(h->spg, cap) AL(h->svel, cap)
   AL(h->sdens, cap) AL(h->wall_start, nc + 1) AL(h->cell_mid, nc)
   for (int c = 0; c < 3; c++) {
     AL(h->u[c], nf) AL(h->us[c], nf)

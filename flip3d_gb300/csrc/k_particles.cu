@@ -118,52 +118,109 @@ __device__ __forceinline__ void visit_cells(int n, const uint32_t *__restrict__ 
     }
 }
 
-/* visit_cells restricted to a ball of radius sqrt(r2) around (px, py, pz):
- * rows (si, sj) whose cells lie wholly outside the ball are skipped and
- * each row's k-range is trimmed to the cells the ball reaches. A cell's
- * particles lie in its interval [s h, (s+1) h) of each axis, except the
- * first and last cells, which also hold the clamped particles outside the
- * grid (their interval is open on that side). With mid (the lists of
- * FAST arithmetic, each cell's lower z half first), a row's run also
- * starts at the first cell's upper half, or stops before the last cell's
- * upper half, when the ball's z-extent lies wholly on the other side of
- * that cell's mid-plane (k + 0.5) h: the sort placed the particles by an
- * exact compare with that plane. Callers pass r2 a little above their own
- * cut-off (the corrector's reach), so every particle that passes their
- * exact distance test is visited, in the same order. */
-template <class F>
+/* visit_cells for the corrector: test(position and type) over the particles that
+ * a ball of radius sqrt(r2) around (px, py, pz) can hold and pair(slot) over those
+ * that pass, in visit_cells' order. Rows (si, sj) whose cells lie wholly outside
+ * the ball are skipped and each row's k-range is trimmed to the cells the ball
+ * reaches. A cell's particles lie in its interval [s h, (s+1) h) of each axis,
+ * except the first and last cells, which also hold the clamped particles outside
+ * the grid (their interval is open on that side). A row's run also starts at the
+ * first cell's upper half, or stops before the last cell's upper half, when the
+ * ball's z-extent lies wholly on the other side of that cell's mid-plane
+ * (k + 0.5) h: the lists of FAST arithmetic put each cell's lower z half first
+ * (mid: where the upper one starts), by an exact compare with that plane.
+ * Callers pass r2 a little above their own cut-off (the corrector's reach), so
+ * every particle that passes their exact distance test is visited.
+ *
+ * About one candidate in nine passes, at a different place in each lane: the
+ * tests of a row's candidates run first, four at a time, into a mask of up to 32,
+ * and the pair arithmetic then runs over the masks of several rows (L: a column of
+ * shared memory a thread), as often as the lane with the most pairs needs instead
+ * of in nearly every trip. spos is read up to three slots past a row's end. */
+constexpr int CORR_ROWS = 4;
+template <int B>
+struct CorrRows {
+  uint32_t slot[CORR_ROWS][B], mask[CORR_ROWS][B];
+};
+template <int B, class T, class P>
 __device__ __forceinline__ void visit_ball(int n, float fn, float h, const uint32_t *__restrict__ cs,
-                                           const uint32_t *__restrict__ mid, float px, float py,
+                                           const uint32_t *__restrict__ mid,
+                                           const float4 *__restrict__ spos, float px, float py,
                                            float pz, float r2, int i0, int i1, int j0, int j1,
-                                           int k0, int k1, F f) {
+                                           int k0, int k1, uint32_t self, CorrRows<B> &L, T test,
+                                           P pair) {
   i0 = max(i0, 0);
   i1 = min(i1, n - 1);
   j0 = max(j0, 0);
   j1 = min(j1, n - 1);
   k0 = max(k0, 0);
   k1 = min(k1, n - 1);
-  if (k0 > k1) return;
+  if (k0 > k1 || j0 > j1) return;
+  const unsigned col = threadIdx.x;
   auto gap = [&](float p, int s) -> float {
     const float lo = s == 0 ? -INFINITY : (float)s * h;
     const float hi = s == n - 1 ? INFINITY : (float)(s + 1) * h;
     return fmaxf(0.0f, fmaxf(lo - p, p - hi));
   };
-  for (int si = i0; si <= i1; si++) {
-    const float gx = gap(px, si), gx2 = gx * gx;
-    if (gx2 > r2) continue;
-    for (int sj = j0; sj <= j1; sj++) {
-      const float gy = gap(py, sj), g2 = gx2 + gy * gy;
-      if (g2 > r2) continue;
-      const float rem = sqrtf(r2 - g2);
-      const int ka = max(k0, (int)floorf(fn * (pz - rem))), kb = min(k1, (int)floorf(fn * (pz + rem)));
-      if (ka > kb) continue;
-      const size_t base = ((size_t)si * n + sj) * n;
-      uint32_t s = __ldg(cs + base + ka), e = __ldg(cs + base + kb + 1);
-      if (mid) {
-        if (pz - rem >= ((float)ka + 0.5f) * h) s = __ldg(mid + base + ka);
-        if (pz + rem < ((float)kb + 0.5f) * h) e = __ldg(mid + base + kb);
+  int si = i0, sj = j0;
+  uint32_t s = 0, e = 0, s2 = 0, e2 = 0; /* this row's run and the next one's */
+  auto next_row = [&]() {
+    s2 = e2 = 0;
+    if (si > i1) return;
+    const float gx = gap(px, si), gy = gap(py, sj), g2 = gx * gx + gy * gy;
+    const size_t base = ((size_t)si * n + sj) * n;
+    if (++sj > j1) {
+      sj = j0;
+      si++;
+    }
+    if (g2 > r2) return;
+    const float rem = sqrtf(r2 - g2);
+    /* clamped like the particles' cells: a ball outside the grid reaches the edge cell */
+    const int ka = max(k0, min((int)floorf(fn * (pz - rem)), n - 1)),
+              kb = min(k1, max((int)floorf(fn * (pz + rem)), 0));
+    if (ka > kb) return;
+    s2 = pz - rem >= ((float)ka + 0.5f) * h ? __ldg(mid + base + ka) : __ldg(cs + base + ka);
+    e2 = pz + rem < ((float)kb + 0.5f) * h ? __ldg(mid + base + kb) : __ldg(cs + base + kb + 1);
+  };
+  next_row();
+  while (si <= i1 || s < e || s2 < e2) {
+    int rows = 0;
+    while (rows < CORR_ROWS && (si <= i1 || s < e || s2 < e2)) {
+      if (s >= e) {
+        s = s2;
+        e = e2;
+        next_row();
+        if (s >= e) continue;
       }
-      for (uint32_t b = s; b < e; b++) f(b);
+      const uint32_t len = min(e - s, 32u);
+      uint32_t m = 0;
+      for (uint32_t t = 0; t < len; t += 4) {
+        const float4 *q = spos + (s + t);
+        const float4 Q0 = __ldg(q), Q1 = __ldg(q + 1), Q2 = __ldg(q + 2), Q3 = __ldg(q + 3);
+        uint32_t four = 0;
+        if (test(Q0)) four |= 1u;
+        if (test(Q1)) four |= 2u;
+        if (test(Q2)) four |= 4u;
+        if (test(Q3)) four |= 8u;
+        m |= four << t;
+      }
+      m &= 0xffffffffu >> (32 - len);
+      if (self - s < 32) m &= ~(1u << (self - s));
+      if (m) {
+        L.slot[rows][col] = s;
+        L.mask[rows][col] = m;
+        rows++;
+      }
+      s += len;
+    }
+    uint32_t m = 0, b = 0;
+    for (int r = 0; m || r < rows; m &= m - 1) {
+      if (!m) {
+        b = L.slot[r][col];
+        m = L.mask[r][col];
+        r++;
+      }
+      pair(b + __ffs(m) - 1);
     }
   }
 }
@@ -1221,13 +1278,16 @@ k_p2g_cells(SimConst c, int enforce, const uint32_t *__restrict__ cs,
   }
 }
 
-/* The corrector's spring and resample with the near-pair work inline
- * instead of through k_spring's and k_resample's per-thread near lists
- * (which hold 24 KB of shared memory per block); the same pairs in the same
- * order, so the same results. */
-/* 1280 resident threads per SM (five blocks of 256): 48 registers (a few
- * spilled) instead of 56; the kernel is issue- and occupancy-bound, and
- * this is 5 % faster at N=256 (six blocks spill more and gain less) */
+/* The FAST corrector: k_spring's and k_resample's pairs, in the same order, so
+ * the same results, from the rows the ball reaches (visit_ball). At n = 128 (4.9
+ * million liquid particles) the pair arithmetic inside the candidate loop took 627
+ * and 500 us, with 14 and 16 of 32 lanes in an instruction; testing first takes
+ * 372 and 372 us with 22 and 23 lanes, and waits for loads (82 and 72 % L1 hits).
+ * More resident warps lose more L1 lines than they hide: 1536 threads an SM take
+ * 433 and 407 us. Tried and slower: row bounds and slots in a list of 42 words a
+ * thread (499 and 800 us, the lists take the L1), two particles a thread sharing
+ * one walk (809 and 755 us). */
+/* 1280 resident threads per SM (five blocks of 256): 48 registers */
 template <class AR, int B = BLK>
 __global__ void __launch_bounds__(B, 1280 / B)
 k_spring_inline(SimConst c, const uint32_t *__restrict__ cs, const uint32_t *__restrict__ mid,
@@ -1235,6 +1295,7 @@ k_spring_inline(SimConst c, const uint32_t *__restrict__ cs, const uint32_t *__r
                 const float *__restrict__ nx,
                 const float *__restrict__ ny, const float *__restrict__ nz,
                 float *__restrict__ px, float *__restrict__ py, float *__restrict__ pz) {
+  __shared__ CorrRows<B> L;
   const int a = blockIdx.x * B + threadIdx.x;
   if (a >= c.np) return;
   const float4 P = __ldg(spos + a);
@@ -1249,11 +1310,11 @@ k_spring_inline(SimConst c, const uint32_t *__restrict__ cs, const uint32_t *__r
   reach_range(P.z, c.corr_reach, c.fn, c.n, z, k0, k1);
   float spring[3] = {0.0f, 0.0f, 0.0f};
   const float reach2 = c.corr_reach * c.corr_reach;
-  visit_ball(c.n, c.fn, c.h, cs, mid, P.x, P.y, P.z, reach2, i0, i1, j0, j1, k0, k1,
-             [&](uint32_t b) {
-    if (b == (uint32_t)a) return;
+  visit_ball(c.n, c.fn, c.h, cs, mid, spos, P.x, P.y, P.z, reach2, i0, i1, j0, j1, k0, k1,
+             (uint32_t)a, L, [&](float4 Q) {
+    return !(AR::hypot2(P.x - Q.x, P.y - Q.y, P.z - Q.z) > c.corr_cut2);
+  }, [&](uint32_t b) {
     const float4 Q = __ldg(spos + b);
-    if (AR::hypot2(P.x - Q.x, P.y - Q.y, P.z - Q.z) > c.corr_cut2) return;
     const float dx = P.x - Q.x, dy = P.y - Q.y, dz = P.z - Q.z;
     const float dist = AR::length(dx, dy, dz);
     const float w = 50.0f * AR::smooth_corr(c, dist * dist);
@@ -1288,6 +1349,7 @@ k_resample_inline(SimConst c, const uint32_t *__restrict__ cs,
                   const float *__restrict__ px, const float *__restrict__ py,
                   const float *__restrict__ pz, float *__restrict__ vx, float *__restrict__ vy,
                   float *__restrict__ vz) {
+  __shared__ CorrRows<B> L;
   const int a = blockIdx.x * B + threadIdx.x;
   if (a >= c.np) return;
   if (unpack_type(__ldg(spos + a).w) != CELL_FLUID) return;
@@ -1302,12 +1364,13 @@ k_resample_inline(SimConst c, const uint32_t *__restrict__ cs,
   float u[3] = {0.0f, 0.0f, 0.0f};
   float wsum = 0.0f;
   const float reach2 = c.corr_reach * c.corr_reach;
-  visit_ball(c.n, c.fn, c.h, cs, mid, T[0], T[1], T[2], reach2, i0, i1, j0, j1, k0, k1,
-             [&](uint32_t b) {
+  visit_ball(c.n, c.fn, c.h, cs, mid, spos, T[0], T[1], T[2], reach2, i0, i1, j0, j1, k0, k1,
+             UINT32_MAX, L, [&](float4 Q) {
+    return AR::hypot2(T[0] - Q.x, T[1] - Q.y, T[2] - Q.z) < c.re_corr_hh &&
+           unpack_type(Q.w) == CELL_FLUID;
+  }, [&](uint32_t b) {
     const float4 Q = __ldg(spos + b);
-    if (unpack_type(Q.w) != CELL_FLUID) return;
     const float d2 = AR::hypot2(T[0] - Q.x, T[1] - Q.y, T[2] - Q.z);
-    if (!(d2 < c.re_corr_hh)) return;
     const float w = AR::sharp(d2, c.re_corr_hh, c.r2_floor, c.sharp_small_corr);
     const float4 V = __ldg(svel + b);
     u[0] += w * V.x;
