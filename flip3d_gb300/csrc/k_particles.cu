@@ -64,6 +64,14 @@ struct RefArith {
   }
 };
 
+/* a / b for normal b and quotient: __fdividef without its handling of denormal
+ * and huge divisors */
+__device__ __forceinline__ float div_normal(float a, float b) {
+  float q;
+  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(q) : "f"(a), "f"(b));
+  return q;
+}
+
 /* The same formulas in native FP32. */
 struct FastArith {
   static __device__ __forceinline__ float hypot2(float a, float b, float c) {
@@ -73,7 +81,11 @@ struct FastArith {
     return sqrtf(hypot2(a, b, c));
   }
   static __device__ __forceinline__ float sharp(float r2, float hh, float, float) {
-    return r2 < hh ? fmaxf(__fdividef(hh, fmaxf(r2, 1.0e-5f)) - 1.0f, 0.0f) : 0.0f;
+    return r2 < hh ? fmaxf(div_normal(hh, fmaxf(r2, 1.0e-5f)) - 1.0f, 0.0f) : 0.0f;
+  }
+  /* sharp for r2 < hh */
+  static __device__ __forceinline__ float sharp_near(float r2, float hh) {
+    return fmaxf(div_normal(hh, fmaxf(r2, 1.0e-5f)) - 1.0f, 0.0f);
   }
   static __device__ __forceinline__ float smooth_density(const SimConst &c, float r2) {
     return fmaxf(fmaf(-r2, c.kd_inv, 1.0f), 0.0f);
@@ -91,7 +103,7 @@ struct FastArith {
     return fmaf((float)c.push_re - dist, nq, p);
   }
   static __device__ __forceinline__ float spring_term(float w, float d, float dist, float re) {
-    return __fdividef(w * re, dist) * d;
+    return div_normal(w * re, dist) * d;
   }
 };
 
@@ -1155,13 +1167,18 @@ __device__ __forceinline__ void cell_decode(size_t c, int n, int &i, int &j, int
   j = (int)(row - (unsigned)i * n);
 }
 
-/* mapP2G (k_p2g's arithmetic and order): one thread per face cell (i, j, k)
- * of the (n+1)^3 lattice computes the three faces there (u0 at (i, j, k)
- * when j, k < n; u1 when i, k < n; u2 when i, j < n). Their neighbourhoods
- * lie in cells [i-1, i+1] x [j-1, j+1] x [k-1, k+1]: each particle there is
- * loaded once and tested against each face whose own cells hold it, which
- * keeps every face's sums in k_p2g's order. AHEAD as in k_p2g. */
-template <class AR, bool AHEAD, int B = BLK>
+/* mapP2G in FAST arithmetic (k_p2g's arithmetic and order): one thread per face
+ * cell (i, j, k) of the (n+1)^3 lattice computes the three faces there (u0 at
+ * (i, j, k) when j, k < n; u1 when i, k < n; u2 when i, j < n). Their
+ * neighbourhoods lie in cells [i-1, i+1] x [j-1, j+1] x [k-1, k+1]: each particle
+ * there is loaded once and tested against each face whose own cells hold it, which
+ * keeps every face's sums in k_p2g's order. About two candidates in three are in
+ * reach, so the weights of all are computed without a branch, the two faces that
+ * share a z packed, and a predicate adds them; n = 128: 572 to 456 us (490 million
+ * warp instructions at 2.7 a cycle before; a block's tile in three dimensions, with
+ * fewer L1 misses, is slower at 490 us, and so are two or four candidates in
+ * flight). */
+template <int B>
 __global__ void __launch_bounds__(B)
 k_p2g_cells(SimConst c, int enforce, const uint32_t *__restrict__ cs,
             const float4 *__restrict__ spg, const float4 *__restrict__ svel,
@@ -1189,57 +1206,35 @@ k_p2g_cells(SimConst c, int enforce, const uint32_t *__restrict__ cs,
         const uint32_t a = __ldg(cs + base + k0), b = __ldg(cs + base + k1 + 1);
         /* u2's cells stop at k: the particles of cell k+1 are not its */
         const uint32_t split = k + 1 <= k1 ? __ldg(cs + base + k + 1) : b;
-        float4 Qn = make_float4(0, 0, 0, 0), Vn = Qn;
-        if (AHEAD && a < b) {
-          Qn = __ldg(spg + a);
-          Vn = __ldg(svel + a);
-        }
-        for (uint32_t x = a; x < b; x++) {
-          const float4 Q = AHEAD ? Qn : __ldg(spg + x);
-          const float4 Va = Vn;
-          if (AHEAD && x + 1 < b) {
-            Qn = __ldg(spg + x + 1);
-            Vn = __ldg(svel + x + 1);
-          }
-          if (unpack_type(Q.w) != CELL_FLUID) continue;
-          float w[3] = {0.0f, 0.0f, 0.0f};
-          bool acc[3] = {false, false, false};
-          if (in0) {
-            const float r2 = AR::hypot2(Q.x - fi, Q.y - hj, Q.z - hk);
-            if (r2 < hh) {
-              acc[0] = true;
-              w[0] = AR::sharp(r2, hh, c.r2_floor, c.sharp_small_p2g);
+        auto one = [&](const float4 Q, const float4 V, uint32_t x) {
+          /* a wall particle is out of every face's reach */
+          const float qx = unpack_type(Q.w) == CELL_FLUID ? Q.x : INFINITY;
+          const float xf = qx - fi, xh = qx - hi, yf = Q.y - fj, yh = Q.y - hj, zf = Q.z - fk,
+                      zh = Q.z - hk;
+          if (in0 || in1) {
+            const F2 dx = f2(xf, xh), dy = f2(yh, yf);
+            const float zz = zh * zh;
+            float r0, r1;
+            f2_get(f2_fma(dx, dx, f2_fma(dy, dy, f2(zz, zz))), r0, r1);
+            const float w0 = FastArith::sharp_near(r0, hh), w1 = FastArith::sharp_near(r1, hh),
+                        p0 = w0 * V.x, p1 = w1 * V.y;
+            if (r0 < hh && in0) {
+              sx[0] += p0;
+              sw[0] += w0;
+            }
+            if (r1 < hh && in1) {
+              sx[1] += p1;
+              sw[1] += w1;
             }
           }
-          if (in1) {
-            const float r2 = AR::hypot2(Q.x - hi, Q.y - fj, Q.z - hk);
-            if (r2 < hh) {
-              acc[1] = true;
-              w[1] = AR::sharp(r2, hh, c.r2_floor, c.sharp_small_p2g);
-            }
+          const float r2 = FastArith::hypot2(xh, yh, zf), w = FastArith::sharp_near(r2, hh),
+                      p = w * V.z;
+          if (r2 < hh && in2 && x < split) {
+            sx[2] += p;
+            sw[2] += w;
           }
-          if (in2 && x < split) {
-            const float r2 = AR::hypot2(Q.x - hi, Q.y - hj, Q.z - fk);
-            if (r2 < hh) {
-              acc[2] = true;
-              w[2] = AR::sharp(r2, hh, c.r2_floor, c.sharp_small_p2g);
-            }
-          }
-          if (!(acc[0] || acc[1] || acc[2])) continue;
-          const float4 V = AHEAD ? Va : __ldg(svel + x);
-          if (acc[0]) {
-            sx[0] += w[0] * V.x;
-            sw[0] += w[0];
-          }
-          if (acc[1]) {
-            sx[1] += w[1] * V.y;
-            sw[1] += w[1];
-          }
-          if (acc[2]) {
-            sx[2] += w[2] * V.z;
-            sw[2] += w[2];
-          }
-        }
+        };
+        for (uint32_t x = a; x < b; x++) one(__ldg(spg + x), __ldg(svel + x), x);
       }
   }
   const bool valid[3] = {v0, v1, v2};
@@ -1532,15 +1527,15 @@ cudaError_t launch_density(FlipGpu *h) {
   return cudaGetLastError();
 }
 
-/* Which P2G kernel a grid takes (all give the same bits; us at n = 24, 48, 64,
- * 96, 128 on pool scenes):
- *   a face a thread, next candidate requested ahead    43   84  141  371  837
- *   a face cell a thread, ahead                        94  110  143  297  593
- *   a face cell a thread                              119  132  152  317  572
+/* Which P2G kernel a grid takes (all give the same bits; us at n = 16, 24, 32, 40,
+ * 48, 64, 128 on pool scenes, FAST):
+ *   a face a thread, next candidate requested ahead    35   42   47   61   80  141  837
+ *   a face cell a thread                               44   54   54   58   70   99  456
  * Small grids leave SMs idle and wait for each candidate's loads in turn, so
- * they take more threads and overlap the loads; large ones are bound by the L1
- * data pipe and take the fewest loads. */
-constexpr int P2G_FACES_N = 64, P2G_AHEAD_N = 112;
+ * they take more threads and overlap the loads; larger ones are bound by the
+ * instructions issued. REF takes a face a thread at every size, and requests ahead
+ * below P2G_AHEAD_N. */
+constexpr int P2G_CELLS_N = 40, P2G_AHEAD_N = 64;
 
 cudaError_t launch_p2g(FlipGpu *h, int enforce) {
   SimConst c = make_const(h);
@@ -1548,24 +1543,20 @@ cudaError_t launch_p2g(FlipGpu *h, int enforce) {
     kernel<<<grid, block, 0, h->stream>>>(c, enforce, h->cell_start, h->spg, h->svel, h->A, h->u[0],
                                           h->u[1], h->u[2], h->us[0], h->us[1], h->us[2]);
   };
-  const bool faces = !cell_gathers(h) || h->n < P2G_FACES_N;
-  if (!faces) {
+  if (cell_gathers(h) && h->n >= P2G_CELLS_N) {
     const size_t m1 = (size_t)h->n + 1, cells = m1 * m1 * m1;
     return tuned_gather(h, "k_p2g_cells", cells, [&](auto B) {
       constexpr int b = decltype(B)::value;
-      if (h->n < P2G_AHEAD_N)
-        go(k_p2g_cells<FastArith, true, b>, grid_for(cells, b), b);
-      else
-        go(k_p2g_cells<FastArith, false, b>, grid_for(cells, b), b);
+      go(k_p2g_cells<b>, grid_for(cells, b), b);
     });
   }
   const unsigned grid = 3u * grid_for(h->nf, BLK);
   const bool fast = h->prm.arith == FLIPGPU_ARITH_FAST;
-  if (h->n < P2G_FACES_N && cell_gathers(h)) {
+  if (cell_gathers(h)) {
     ktime_begin(h, "k_p2g_cells"); /* the kernel clock's name of the FAST P2G */
     go(k_p2g<FastArith, true>, grid, BLK);
     ktime_end(h);
-  } else if (h->n < P2G_FACES_N && !fast) {
+  } else if (h->n < P2G_AHEAD_N && !fast) {
     go(k_p2g<RefArith, true>, grid, BLK);
   } else if (fast) {
     go(k_p2g<FastArith, false>, grid, BLK);

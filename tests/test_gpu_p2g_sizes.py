@@ -1,6 +1,7 @@
-"""P2G on both sides of the sizes where its kernel changes (n = 63, 64 and 111,
-112; 9 for the smallest), FAST arithmetic against the per-particle kernels
-(FLIPGPU_GATHER=particle) and REF arithmetic against the oracle: bit for bit."""
+"""P2G on both sides of the sizes where its kernel changes (n = 39, 40 in FAST
+and 63, 64 in REF arithmetic; 9 for the smallest, 112 for a large grid), FAST
+arithmetic against the per-particle kernels (FLIPGPU_GATHER=particle) and REF
+arithmetic against the oracle: bit for bit."""
 import os
 
 import numpy as np
@@ -26,7 +27,7 @@ def faces(gpu, sc, vel, arith, mode=None):
         os.environ.pop("FLIPGPU_GATHER", None)
 
 
-@pytest.mark.parametrize("n", [9, 63, 64, 111, 112])
+@pytest.mark.parametrize("n", [9, 39, 40, 63, 64, 112])
 def test_p2g_kernels_agree(n):
     from flip3d_gb300 import gpu
     from oracle import pyoracle as orc
