@@ -110,7 +110,7 @@ __global__ void k_scan_down(const uint32_t *__restrict__ in, uint32_t *__restric
 
 /* key = the particle's cell; with HALVES (FAST arithmetic) bit 31 also
  * marks a particle at or above its cell's mid-plane in z, (k + 0.5) h, and
- * the scatter carries that bit into perm for k_sort_fixup_halves (cell ids
+ * the scatter carries that bit into perm for k_sort_fixup (cell ids
  * stay below 2^30, as flipgpu_create allows n <= 1024, and particle
  * indices below 2^31). */
 template <bool HALVES>
@@ -140,67 +140,70 @@ __global__ void k_sort_scatter(int np, const uint32_t *__restrict__ key,
   perm[cell_start[kk & 0x7fffffffu] + rank[p]] = (uint32_t)p | (kk & 0x80000000u);
 }
 
-/* Order each cell's slots by particle index: insertion sort for the usual
- * handful, heapsort for crowded cells. */
-__global__ void k_sort_fixup(size_t nc, const uint32_t *__restrict__ cell_start,
-                             uint32_t *__restrict__ perm) {
-  size_t cidx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (cidx >= nc) return;
-  uint32_t s = cell_start[cidx], e = cell_start[cidx + 1];
-  uint32_t len = e - s;
-  if (len < 2) return;
-  uint32_t *a = perm + s;
-  if (len <= 32) {
-    for (uint32_t i = 1; i < len; i++) {
-      uint32_t v = a[i];
-      uint32_t j = i;
-      while (j > 0 && a[j - 1] > v) {
-        a[j] = a[j - 1];
-        j--;
-      }
-      a[j] = v;
-    }
-    return;
-  }
-  auto sift = [&](uint32_t root, uint32_t end) {
-    while (true) {
-      uint32_t child = 2 * root + 1;
-      if (child >= end) break;
-      if (child + 1 < end && a[child] < a[child + 1]) child++;
-      if (a[root] >= a[child]) break;
-      uint32_t t = a[root];
-      a[root] = a[child];
-      a[child] = t;
-      root = child;
-    }
-  };
-  for (uint32_t i = len / 2; i-- > 0;) sift(i, len);
-  for (uint32_t end = len - 1; end > 0; end--) {
-    uint32_t t = a[0];
-    a[0] = a[end];
-    a[end] = t;
-    sift(0, end);
-  }
+/* v[0..N) ascending: Batcher's odd-even merge network */
+template <int N>
+__device__ __forceinline__ void sort_network(uint32_t (&v)[N]) {
+#pragma unroll
+  for (int p = 1; p < N; p *= 2)
+#pragma unroll
+    for (int k = p; k >= 1; k /= 2)
+#pragma unroll
+      for (int j = k % p; j + k < N; j += 2 * k)
+#pragma unroll
+        for (int i = 0; i < k; i++)
+          if (i + j + k < N && (i + j) / (2 * p) == (i + j + k) / (2 * p)) {
+            const uint32_t x = v[i + j], y = v[i + j + k];
+            v[i + j] = min(x, y);
+            v[i + j + k] = max(x, y);
+          }
 }
 
-/* FAST arithmetic: each cell's slots ordered by (z half, particle index),
- * the particles below the cell's mid-plane (k + 0.5) h first, and
- * cell_mid[c] the slot where the upper half starts, so that a walk along a
- * row of cells can start or stop at half a cell. The half arrives in bit
- * 31 of each slot (k_sort_count<true>, k_sort_scatter), which makes it the
- * leading sort key; the bit is cleared at the end. */
-__global__ void k_sort_fixup_halves(size_t nc, const uint32_t *__restrict__ cell_start,
-                                    uint32_t *__restrict__ perm,
-                                    uint32_t *__restrict__ cell_mid) {
+/* len <= N keys at a in order, without their top bit; returns how many have it
+ * unset. Keys differ, and none is 0xffffffff. */
+template <int N>
+__device__ __forceinline__ uint32_t sort_small(uint32_t *a, uint32_t len) {
+  uint32_t v[N], low = 0;
+#pragma unroll
+  for (int q = 0; q < N; q++) {
+    v[q] = q < len ? a[q] : 0xffffffffu;
+    low += (v[q] >> 31) ^ 1u;
+  }
+  sort_network(v);
+#pragma unroll
+  for (int q = 0; q < N; q++)
+    if (q < len) a[q] = v[q] & 0x7fffffffu;
+  return low;
+}
+
+/* Each cell's slots by particle index: cells of up to 16 particles through a
+ * network in registers, insertion sort up to 32, heapsort for crowded cells.
+ *
+ * With HALVES (FAST arithmetic) the slots are ordered by (z half, particle index),
+ * the particles below the cell's mid-plane (k + 0.5) h first, and cell_mid[c]
+ * is the slot where the upper half starts, so that a walk along a row of cells can
+ * start or stop at half a cell. The half arrives in bit 31 of each slot
+ * (k_sort_count<true>, k_sort_scatter), which makes it the leading sort key; the
+ * bit is cleared at the end.
+ *
+ * Insertion in global memory is a chain of loads and stores a lane: a sort of a
+ * pool at n = 128 (5 million particles) took 40 us more with it than with the
+ * networks, most of the 67 us of this pass. */
+template <bool HALVES>
+__global__ void k_sort_fixup(size_t nc, const uint32_t *__restrict__ cell_start,
+                             uint32_t *__restrict__ perm, uint32_t *__restrict__ cell_mid) {
   size_t cidx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (cidx >= nc) return;
   const uint32_t s = cell_start[cidx], e = cell_start[cidx + 1];
   const uint32_t len = e - s;
   uint32_t *a = perm + s;
   uint32_t low = 0;
-  for (uint32_t i = 0; i < len; i++) low += a[i] >> 31 ? 0u : 1u;
-  cell_mid[cidx] = s + low;
-  if (len >= 2) {
+  if (len == 0) {
+  } else if (len <= 8) {
+    low = sort_small<8>(a, len);
+  } else if (len <= 16) {
+    low = sort_small<16>(a, len);
+  } else {
+    for (uint32_t i = 0; i < len; i++) low += a[i] >> 31 ? 0u : 1u;
     if (len <= 32) {
       for (uint32_t i = 1; i < len; i++) {
         uint32_t v = a[i];
@@ -232,8 +235,9 @@ __global__ void k_sort_fixup_halves(size_t nc, const uint32_t *__restrict__ cell
         sift(0, end);
       }
     }
+    for (uint32_t i = low; i < len; i++) a[i] &= 0x7fffffffu;
   }
-  for (uint32_t i = low; i < len; i++) a[i] &= 0x7fffffffu;
+  if (HALVES) cell_mid[cidx] = s + low;
 }
 
 /* Sorted payload; with apply_gravity also add_ExtForce (src/flip3D.cpp:
@@ -479,10 +483,11 @@ cudaError_t launch_sort(FlipGpu *h, int apply_gravity, int fields) {
     k_sort_scatter<<<grid_for(h->np, 256), 256, 0, h->stream>>>(h->np, h->key, h->rank,
                                                                 h->cell_start, h->perm);
     if (h->prm.arith == FLIPGPU_ARITH_FAST)
-      k_sort_fixup_halves<<<grid_for(h->nc, 256), 256, 0, h->stream>>>(
+      k_sort_fixup<true><<<grid_for(h->nc, 256), 256, 0, h->stream>>>(
           h->nc, h->cell_start, h->perm, h->cell_mid);
     else
-      k_sort_fixup<<<grid_for(h->nc, 256), 256, 0, h->stream>>>(h->nc, h->cell_start, h->perm);
+      k_sort_fixup<false><<<grid_for(h->nc, 256), 256, 0, h->stream>>>(
+          h->nc, h->cell_start, h->perm, h->cell_mid);
     FG_LAUNCHED(h, 2);
   }
   e = cudaGetLastError();
