@@ -96,13 +96,21 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
 /* Y[s][v][co] = (relu)(sum_{tap, ci} X[s][v + off(tap)][ci] W[tap][ci][co] + bias[co])
  * over the block's output channels [blockIdx.y*NB, +NB). Cells outside the
  * grid read as zero. frag holds W as B fragments: for (tap, 16-channel chunk
- * c, 8-column tile nt) 32 lanes x {W[2t..2t+1][g], W[2t+8..2t+9][g]}. */
-template <int NB>
-__global__ void __launch_bounds__(CTHREADS, 1)
-    k_conv3(int n, int cin, int cout, const bf16 *__restrict__ X, const uint2 *__restrict__ frag,
+ * c, 8-column tile nt) 32 lanes x {W[2t..2t+1][g], W[2t+8..2t+9][g]}.
+ *
+ * NCH: the 16-channel chunks of the input, 0 for any number. A warp has four to
+ * eighteen MMAs a tap against its index arithmetic and the latency of its
+ * fragments: with the channels known, the address a constant off one register and
+ * the next fragments requested ahead, 16 to 16 channels on 16 samples of 32^3 take
+ * 33 us instead of 84 (2,500 instructions a warp, two blocks an SM before), 16 to
+ * 48 61 instead of 155 (one block an SM before). */
+template <int NB, int NCH>
+__global__ void __launch_bounds__(CTHREADS, NB == 16 ? 4 : 2)
+    k_conv3(int n, int cin_, int cout, const bf16 *__restrict__ X, const uint2 *__restrict__ frag,
             const float *__restrict__ bias, bf16 *__restrict__ Y, int relu) {
   extern __shared__ __align__(16) unsigned char smraw[];
   bf16 *sm = reinterpret_cast<bf16 *>(smraw);
+  const int cin = NCH ? 16 * NCH : cin_;
   const int stride = cin + 8; /* bf16 per staged cell (padded against bank conflicts) */
   const int tj_n = tiles_of(n, TJ), tk_n = tiles_of(n, TK);
   const int tile = blockIdx.x;
@@ -110,17 +118,19 @@ __global__ void __launch_bounds__(CTHREADS, 1)
             k0 = (tile % tk_n) * TK;
   const size_t n3 = (size_t)n * n * n;
   const bf16 *Xs = X + (size_t)blockIdx.z * n3 * cin;
-  /* stage the halo */
-  const int q8 = cin / 8;
-  for (int idx = threadIdx.x; idx < HV * q8; idx += CTHREADS) {
-    const int hv = idx / q8, q = idx % q8;
-    const int hi = hv / (HJ * HK), hj = (hv / HK) % HJ, hk = hv % HK;
-    const int gi = i0 - 1 + hi, gj = j0 - 1 + hj, gk = k0 - 1 + hk;
-    uint4 val = make_uint4(0, 0, 0, 0);
-    if (gi >= 0 && gi < n && gj >= 0 && gj < n && gk >= 0 && gk < n)
-      val = *reinterpret_cast<const uint4 *>(Xs + (((size_t)gi * n + gj) * n + gk) * cin + q * 8);
-    *reinterpret_cast<uint4 *>(sm + hv * stride + q * 8) = val;
-  }
+  /* stage the halo: a thread takes 8 channels of every step-th cell */
+  const int q8 = cin / 8, step = CTHREADS / q8, first = (int)threadIdx.x / q8,
+            q = ((int)threadIdx.x - first * q8) * 8;
+  if (first < step)
+    for (int hv = first; hv < HV; hv += step) {
+      const int hi = hv / (HJ * HK), hj = (hv / HK) % HJ, hk = hv % HK;
+      const int gi = i0 - 1 + hi, gj = j0 - 1 + hj, gk = k0 - 1 + hk;
+      uint4 val = make_uint4(0, 0, 0, 0);
+      if ((unsigned)gi < (unsigned)n && (unsigned)gj < (unsigned)n && (unsigned)gk < (unsigned)n)
+        val = __ldg(reinterpret_cast<const uint4 *>(
+            Xs + (size_t)(unsigned)((gi * n + gj) * n + gk) * cin + q));
+      *reinterpret_cast<uint4 *>(sm + hv * stride + q) = val;
+    }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -138,26 +148,33 @@ __global__ void __launch_bounds__(CTHREADS, 1)
     const int ei = e / (TJ * TK), ej = (e / TK) % TJ, ek = e % TK;
     base_row[m] = (ei * HJ + ej) * HK + ek;
   }
-  const uint32_t sbase = smem_u32(sm) + (uint32_t)((lane >> 4) * 16);
-  const int nchunk = cin / 16, ntile_all = cout / 8;
+  const int nchunk = NCH ? NCH : cin / 16, ntile_all = cout / 8;
   const int nt0 = blockIdx.y * NT;
-  for (int tap = 0; tap < 27; tap++) {
-    const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
-    const int toff = (dz * HJ + dy) * HK + dx;
-    for (int c = 0; c < nchunk; c++) {
-      uint32_t a[2][4];
+  uint32_t row[2]; /* shared-memory address of the tap's row, per m-tile */
 #pragma unroll
-      for (int m = 0; m < 2; m++)
-        ldsm_x4(sbase + (uint32_t)(((base_row[m] + toff) * stride + c * 16) * 2), a[m][0], a[m][1],
-                a[m][2], a[m][3]);
-      const uint2 *fb = frag + ((size_t)(tap * nchunk + c) * ntile_all + nt0) * 32 + lane;
+  for (int m = 0; m < 2; m++)
+    row[m] = smem_u32(sm) + (uint32_t)((lane >> 4) * 16 + base_row[m] * stride * 2);
+  /* fragments lie in the order of the loops */
+  const uint2 *fb = frag + (size_t)nt0 * 32 + lane;
+  for (int line = 0; line < 9; line++) {
+    const uint32_t loff = (uint32_t)(((line / 3) * HJ + line % 3) * HK * stride * 2);
 #pragma unroll
-      for (int j = 0; j < NT; j++) {
-        const uint2 b = __ldg(fb + j * 32);
-        mma_bf16(acc[0][j], a[0][0], a[0][1], a[0][2], a[0][3], b.x, b.y);
-        mma_bf16(acc[1][j], a[1][0], a[1][1], a[1][2], a[1][3], b.x, b.y);
+    for (int dx = 0; dx < 3; dx++)
+#pragma unroll(NCH > 0 ? NCH : 1)
+      for (int c = 0; c < nchunk; c++) {
+        const uint32_t off = loff + (uint32_t)(dx * stride * 2 + c * 32);
+        uint32_t a[2][4];
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+          ldsm_x4(row[m] + off, a[m][0], a[m][1], a[m][2], a[m][3]);
+#pragma unroll
+        for (int j = 0; j < NT; j++) {
+          const uint2 b = __ldg(fb + j * 32);
+          mma_bf16(acc[0][j], a[0][0], a[0][1], a[0][2], a[0][3], b.x, b.y);
+          mma_bf16(acc[1][j], a[1][0], a[1][1], a[1][2], a[1][3], b.x, b.y);
+        }
+        fb += ntile_all * 32;
       }
-    }
   }
   bf16 *Ys = Y + (size_t)blockIdx.z * n3 * cout;
 #pragma unroll
@@ -884,6 +901,27 @@ template <class T> cudaError_t ualloc(T *&p, size_t n) {
 
 size_t conv_smem(int cin) { return (size_t)HV * (cin + 8) * sizeof(bf16); }
 
+/* f(the k_conv3 of nb output channels a block and cin input channels) */
+template <int NB, class F>
+void conv3_of(int cin, F f) {
+  switch (cin) {
+  case 16: f(k_conv3<NB, 1>); break;
+  case 32: f(k_conv3<NB, 2>); break;
+  case 48: f(k_conv3<NB, 3>); break;
+  case 64: f(k_conv3<NB, 4>); break;
+  default: f(k_conv3<NB, 0>); break;
+  }
+}
+template <class F>
+void conv3_kernels(int nb, int cin, F f) {
+  switch (nb) {
+  case 64: conv3_of<64>(cin, f); break;
+  case 48: conv3_of<48>(cin, f); break;
+  case 32: conv3_of<32>(cin, f); break;
+  default: conv3_of<16>(cin, f); break;
+  }
+}
+
 /* k_wgrad for the channel counts of one layer: f(kernel, threads, shared bytes) */
 template <class F> bool with_wgrad(int cin, int cout, F f) {
   bool hit = false;
@@ -908,12 +946,14 @@ int unet_init_device() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
   if (done[dev]) return 0;
   const int big = (int)conv_smem(112);
-  if (cudaFuncSetAttribute(k_conv3<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) ||
-      cudaFuncSetAttribute(k_conv3<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) ||
-      cudaFuncSetAttribute(k_conv3<48>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) ||
-      cudaFuncSetAttribute(k_conv3<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) ||
-      conv_tc_init_device() != 0)
-    return -1;
+  bool set = conv_tc_init_device() == 0;
+  for (int nb = 16; nb <= 64; nb += 16)
+    for (int cin = 16; cin <= 80; cin += 16)
+      conv3_kernels(nb, cin, [&](auto kernel) {
+        set = set && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          big) == cudaSuccess;
+      });
+  if (!set) return -1;
   for (int l = 0; l < NCONV; l++) {
     bool ok = true;
     if (!with_wgrad(kConv[l].cin, kConv[l].cout, [&](auto kern, int, int smem) {
@@ -934,12 +974,9 @@ cudaError_t conv(FlipUNet *u, int n, int batch, int cin, int cout, const bf16 *X
   const size_t smem = conv_smem(cin);
   const int nb = (cout % 64 == 0) ? 64 : (cout % 48 == 0) ? 48 : (cout % 32 == 0) ? 32 : 16;
   dim3 grid(tiles, cout / nb, batch);
-  switch (nb) {
-  case 64: k_conv3<64><<<grid, CTHREADS, smem, u->stream>>>(n, cin, cout, X, frag, bias, Y, relu); break;
-  case 48: k_conv3<48><<<grid, CTHREADS, smem, u->stream>>>(n, cin, cout, X, frag, bias, Y, relu); break;
-  case 32: k_conv3<32><<<grid, CTHREADS, smem, u->stream>>>(n, cin, cout, X, frag, bias, Y, relu); break;
-  default: k_conv3<16><<<grid, CTHREADS, smem, u->stream>>>(n, cin, cout, X, frag, bias, Y, relu); break;
-  }
+  conv3_kernels(nb, cin, [&](auto kernel) {
+    kernel<<<grid, CTHREADS, smem, u->stream>>>(n, cin, cout, X, frag, bias, Y, relu);
+  });
   return cudaGetLastError();
 }
 
