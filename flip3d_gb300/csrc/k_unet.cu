@@ -61,6 +61,7 @@ constexpr int HI = TI + 2, HJ = TJ + 2, HK = TK + 2, HV = HI * HJ * HK;
 constexpr int CTHREADS = 256;
 constexpr int EBLK = 256;
 constexpr int RB = 256; /* reduction blocks per sample */
+constexpr unsigned HEAD_BLOCKS = 304; /* of k_loss_head_bwd: two an SM */
 constexpr int WG_SUB = 64; /* cells staged per weight-gradient step */
 
 __host__ __device__ inline int tiles_of(int n, int t) { return (n + t - 1) / t; }
@@ -567,9 +568,19 @@ __global__ void k_head(size_t cells, const bf16 *__restrict__ D, const float *__
   O[v] = a;
 }
 
+/* A bf16 as a double by its bits: a conversion costs FP64 issue like the arithmetic. */
+__device__ __forceinline__ double bf16_to_double(bf16 b) {
+  const unsigned u = __bfloat16_as_ushort(b), e = (u >> 7) & 255u;
+  if (e - 1u >= 254u && (u & 0x7fffu)) return (double)__bfloat162float(b); /* denormal, Inf, NaN */
+  return __hiloint2double((int)((u & 0x8000u) << 16 |
+                                (e ? ((e + 896u) << 20 | (u & 127u) << 13) : 0u)), 0);
+}
+
 /* loss = sum over liquid cells of (O - T)^2 / count, T = (x - x0)/scale;
  * dO = 2 (O - T) / count on liquid cells; dD[v][c] = dO wh[c]; partial
- * sums of the loss and of the head's gradients per block */
+ * sums of the loss and of the head's gradients per block. Bound by FP64 issue: one
+ * cell a thread left 18 sums of 256 values to every block's tree (83 us for 16
+ * samples of 32^3); two blocks an SM that sum their cells first take 40 us. */
 __global__ void k_loss_head_bwd(size_t n3, int batch, const uint8_t *__restrict__ A,
                                 const float *__restrict__ x, const float *__restrict__ x0,
                                 const float *__restrict__ scale, double inv_count,
@@ -577,27 +588,29 @@ __global__ void k_loss_head_bwd(size_t n3, int batch, const uint8_t *__restrict_
                                 const float *__restrict__ wh, bf16 *__restrict__ dD,
                                 double *__restrict__ part) {
   __shared__ double sh[EBLK][18];
-  const size_t v = (size_t)blockIdx.x * EBLK + threadIdx.x;
   double l = 0.0, gw[17];
 #pragma unroll
   for (int c = 0; c < 17; c++) gw[c] = 0.0;
-  if (v < n3 * batch) {
+  for (size_t v = (size_t)blockIdx.x * EBLK + threadIdx.x; v < n3 * batch;
+       v += (size_t)gridDim.x * EBLK) {
     const size_t s = v / n3;
     float g = 0.0f;
     if (A[v] == CELL_FLUID) {
       const float T = (x[v] - x0[v]) / scale[4 * s + 3];
       const float e = O[v] - T;
-      l = (double)e * e * inv_count;
+      l += (double)e * e * inv_count;
       g = (float)(2.0 * e * inv_count);
     }
-    const bf16 *d = D + v * 16;
-    __align__(16) bf16 row[16];
+    __align__(16) bf16 d[16], row[16];
+    reinterpret_cast<uint4 *>(d)[0] = __ldg(reinterpret_cast<const uint4 *>(D + v * 16));
+    reinterpret_cast<uint4 *>(d)[1] = __ldg(reinterpret_cast<const uint4 *>(D + v * 16) + 1);
+    const double gd = g;
 #pragma unroll
     for (int c = 0; c < 16; c++) {
       row[c] = __float2bfloat16(g * wh[c]);
-      gw[c] = (double)g * __bfloat162float(d[c]);
+      gw[c] = fma(gd, bf16_to_double(d[c]), gw[c]); /* the product is exact */
     }
-    gw[16] = g;
+    gw[16] += gd;
     uint4 *dst = reinterpret_cast<uint4 *>(dD + v * 16);
     dst[0] = reinterpret_cast<uint4 *>(row)[0];
     dst[1] = reinterpret_cast<uint4 *>(row)[1];
@@ -1196,7 +1209,7 @@ int backward(FlipUNet *u, int n, int batch, const uint8_t *A, const float *x, co
   double total = 0.0;
   for (int s = 0; s < B; s++) total += cnt_host[s];
   const double inv = total > 0.0 ? 1.0 / total : 0.0;
-  const unsigned hb = eg(V0 * B);
+  const unsigned hb = std::min(eg(V0 * B), HEAD_BLOCKS);
   k_loss_head_bwd<<<hb, EBLK, 0, u->stream>>>(V0, B, A, x, x0, u->scale, inv, u->O, u->D0,
                                               u->P + u->hoff, u->G1, u->hpart);
   k_head_reduce<<<1, 18 * 32, 0, u->stream>>>((int)hb, u->hpart, u->G + u->hoff, u->loss);
