@@ -30,6 +30,11 @@
  * descriptors formed by one 64-bit add each, and two warps issue them, each
  * for its own tiles and accumulators.
  *
+ * Bound on 128-cell segments: the copies' 16-byte rows (about 0.6 a cycle), R + 2
+ * lines for R, so the time follows (R + 2) / R: 16 to 16 channels at n = 128 take
+ * 137, 103 and 90 us at R = 2, 4 and 8 (60 would be the tensor core's); R = 16
+ * leaves no room for a third stage.
+ *
  * Pipeline, one CTA of 7 warps per SM, persistent over units, a ring of up
  * to 6 stages (di, 16-channel chunk):
  *   warp 0     producer (one thread): two TMA tile copies (one per 8-channel
@@ -427,13 +432,13 @@ bool tc_plan(int n, int cin, int cout, int batch, TcShape &sh, size_t &smem, int
   auto tiles = [&](int r) { return sh.lk == 128 ? r : (r * sh.P - 2 + 127) / 128; };
   auto fits = [&](int r) {
     const int t = tiles(r);
-    return r >= 1 && r <= n && n % r == 0 && t <= 5 && 2 * t * cout <= 512;
+    return r >= 1 && r <= n && n % r == 0 && (t <= 5 || t == 8) && 2 * t * cout <= 512;
   };
   if (R_req > 0) {
     if (!fits(R_req)) return false;
     R = R_req;
   } else if (sh.lk == 128) {
-    R = 4;
+    R = fits(8) ? 8 : 4;
   } else {
     for (int r = 16; r >= 1; r >>= 1)
       if (fits(r)) {
@@ -503,7 +508,7 @@ int conv_tc_init_device() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
   if (done[dev]) return 0;
   if (set_smem_limit<1>() || set_smem_limit<2>() || set_smem_limit<3>() || set_smem_limit<4>() ||
-      set_smem_limit<5>())
+      set_smem_limit<5>() || set_smem_limit<8>())
     return -1;
   done[dev] = true;
   return 0;
@@ -561,6 +566,7 @@ cudaError_t tc_launch_one(cudaStream_t st, int n, int batch, int cin, int cout, 
   case 2: k_conv_tc<2><<<grid, TC_THREADS, smem, st>>>(map, sh, Wtc, bias, Y, relu, err); break;
   case 3: k_conv_tc<3><<<grid, TC_THREADS, smem, st>>>(map, sh, Wtc, bias, Y, relu, err); break;
   case 4: k_conv_tc<4><<<grid, TC_THREADS, smem, st>>>(map, sh, Wtc, bias, Y, relu, err); break;
+  case 8: k_conv_tc<8><<<grid, TC_THREADS, smem, st>>>(map, sh, Wtc, bias, Y, relu, err); break;
   default: k_conv_tc<5><<<grid, TC_THREADS, smem, st>>>(map, sh, Wtc, bias, Y, relu, err); break;
   }
   return cudaGetLastError();
