@@ -1107,10 +1107,12 @@ int refresh_frags(FlipUNet *u) {
 /* features and per-sample scales of a batch of systems */
 unsigned eg(size_t count) { return (unsigned)((count + EBLK - 1) / EBLK); }
 
-/* k_up_cat with three vectors a thread, or one line a block */
+/* k_up_cat with three vectors a thread, or fewer lines a block where that would
+ * leave less than eight blocks an SM */
 template <int C1, int C2>
 void up_cat(FlipUNet *u, int n, int batch, const bf16 *coarse, const bf16 *skip, bf16 *U) {
-  const int total = batch * n * n, lines = std::max(1, 3 * EBLK / (n * ((C1 + C2) / 8)));
+  const int total = batch * n * n, most = 3 * EBLK / (n * ((C1 + C2) / 8)),
+            lines = std::max(1, std::min(most, total / (8 * 152)));
   k_up_cat<C1, C2><<<(unsigned)((total + lines - 1) / lines), EBLK, 0, u->stream>>>(
       n, lines, total, coarse, skip, U);
 }
