@@ -248,21 +248,36 @@ void ktime_flush(FlipGpu *h) {
   cudaGetLastError();
 }
 
+/* x, y, z, final on the step's stream, through the transfer stream to the host. */
+static cudaError_t xfer_out(FlipGpu *h, const float *x, const float *y, const float *z,
+                            float4 *buffer, float *dst) {
+  cudaError_t e = cudaEventRecord(h->xev[2], h->stream);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(h->xstream, h->xev[2], 0);
+  if (e != cudaSuccess) return e;
+  float *stage = reinterpret_cast<float *>(buffer);
+  k_interleave<<<grid_for(h->np, BLK), BLK, 0, h->xstream>>>(h->np, x, y, z, stage);
+  FG_LAUNCHED(h, 1);
+  e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(dst, stage, (size_t)h->np * 3 * sizeof(float), cudaMemcpyDeviceToHost,
+                        h->xstream);
+  return e;
+}
+
 /* After the corrector's spring: the positions are final, so the transfer
  * stream interleaves them into the sorted grid-position buffer (unused by
  * the resample) and copies them to the host while the resample runs. */
 cudaError_t xfer_positions_out(FlipGpu *h) {
-  cudaError_t e = cudaEventRecord(h->xev[2], h->stream);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(h->xstream, h->xev[2], 0);
-  if (e != cudaSuccess) return e;
-  float *stage = reinterpret_cast<float *>(h->spg);
-  k_interleave<<<grid_for(h->np, BLK), BLK, 0, h->xstream>>>(h->np, h->px, h->py, h->pz, stage);
-  FG_LAUNCHED(h, 1);
-  e = cudaGetLastError();
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(h->xfer_pos_out, stage, (size_t)h->np * 3 * sizeof(float),
-                        cudaMemcpyDeviceToHost, h->xstream);
-  return e;
+  return xfer_out(h, h->px, h->py, h->pz, h->spg, h->xfer_pos_out);
+}
+
+/* Before the spring of a corrector that does not resample: the velocities are
+ * final and their sorted copy is not read again, so their copy runs beside the
+ * spring. */
+cudaError_t xfer_velocities_out(FlipGpu *h) {
+  float *dst = h->xfer_vel_out;
+  h->xfer_vel_out = nullptr;
+  return xfer_out(h, h->vx, h->vy, h->vz, h->svel, dst);
 }
 
 
@@ -992,8 +1007,11 @@ int flipgpu_step_host(FlipGpu *h, const float *pos_in, const float *vel_in, floa
   }
   h->cells_valid = false;
   h->xfer_pos_out = h->np > 0 ? pos_out : nullptr;
+  h->xfer_vel_out = h->np > 0 ? vel_out : nullptr;
   r = step_body(h, st);
   h->xfer_pos_out = nullptr;
+  if (!h->xfer_vel_out) vel_out = nullptr; /* on their way */
+  h->xfer_vel_out = nullptr;
   if (h->defer_vel) { /* the step stopped before the payload */
     cudaStreamWaitEvent(h->stream, h->xev[1], 0);
     h->defer_vel = 0;

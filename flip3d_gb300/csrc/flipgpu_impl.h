@@ -126,6 +126,7 @@ struct FlipGpu {
   cudaEvent_t xev[3];
   int defer_vel, defer_gravity;   /* payload velocities after the upload */
   float *xfer_pos_out;            /* host destination of the positions, or null */
+  float *xfer_vel_out;            /* of the velocities, or null (xfer_velocities_out) */
   /* MG preconditioner (k_pcg.cu mg_alloc): levels 1.. and level-0 scratch */
   int mg_nlev, mg_lb, mg_m[10];
   uint8_t *mg_flags[10];
@@ -261,6 +262,7 @@ cudaError_t launch_payload_vel(FlipGpu *h, int apply_gravity);
 /* flipgpu_step_host: download the corrected positions on the transfer
  * stream while the velocity resample runs (called between the two) */
 cudaError_t xfer_positions_out(FlipGpu *h);
+cudaError_t xfer_velocities_out(FlipGpu *h);
 cudaError_t launch_density(FlipGpu *h);
 cudaError_t launch_mark_water(FlipGpu *h);
 cudaError_t launch_add_force(FlipGpu *h);

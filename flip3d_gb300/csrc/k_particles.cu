@@ -1710,6 +1710,10 @@ cudaError_t launch_correct(FlipGpu *h) {
   SimConst c = make_const(h);
   const unsigned g = grid_for(h->np, BLK);
   const bool fast = h->prm.arith == FLIPGPU_ARITH_FAST;
+  if (h->xfer_vel_out && resample_is_identity(c)) {
+    const cudaError_t x = xfer_velocities_out(h);
+    if (x != cudaSuccess) return x;
+  }
   if (cell_gathers(h)) {
     cudaError_t e = tuned_gather(h, "k_spring_inline", h->np, [&](auto B) {
       constexpr int b = decltype(B)::value;
