@@ -218,11 +218,29 @@ __global__ void __launch_bounds__(CTHREADS, NB == 16 ? 4 : 2)
  * stages). One block per tap that staged synchronously, with the tiles dealt
  * to eight warps (two of which had work in the 16 x 16 layers), was bound by
  * the staging latency: the 14 layers of 16 systems of 32^3 cells took 7.33 ms
- * of a training step's 9.12 ms; with this the step takes 2.53 ms. */
+ * of a training step's 9.12 ms; with this 0.78 ms, and 0.66 ms with the copies'
+ * divisions by n as multiplications (half of a 16 x 16 layer's instructions were the
+ * index arithmetic of its copies). */
 __device__ __forceinline__ void wg_copy(uint32_t dst, const void *src, bool ok) {
   const int bytes = ok ? 16 : 0; /* 0: the 16 bytes are zero-filled */
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes)
                : "memory");
+}
+
+/* v / n for v < 2^31 by a multiplication (Granlund and Montgomery, 1994): with
+ * 2^(l-1) < n <= 2^l and m = ceil(2^(31+l) / n), m n exceeds 2^(31+l) by less than
+ * n <= 2^l, so v m / 2^(31+l) has the quotient's integer part. */
+struct DivBy {
+  unsigned m, shift; /* m 0: n = 1 */
+  __device__ __forceinline__ unsigned operator()(unsigned v) const {
+    return m ? __umulhi(v, m) >> shift : v;
+  }
+};
+DivBy div_by(int n) {
+  if (n == 1) return {0u, 0u};
+  int l = 1;
+  while ((1 << l) < n) l++;
+  return {(unsigned)(((1ull << (31 + l)) + n - 1) / n), (unsigned)l - 1};
 }
 
 constexpr int WG_ROWS = WG_SUB + 2, WG_STAGES = 3;
@@ -237,8 +255,8 @@ template <int CIN, int COUT> struct WgShape {
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(WgShape<CIN, COUT>::THREADS)
-    k_wgrad(int n, int cps, int ch, const bf16 *__restrict__ X, const bf16 *__restrict__ dZ,
-            float *__restrict__ part, float *__restrict__ part_b) {
+    k_wgrad(int n, DivBy by_n, int cps, int ch, const bf16 *__restrict__ X,
+            const bf16 *__restrict__ dZ, float *__restrict__ part, float *__restrict__ part_b) {
   typedef WgShape<CIN, COUT> S;
   constexpr int NT = COUT / 8;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -261,8 +279,8 @@ __global__ void __launch_bounds__(WgShape<CIN, COUT>::THREADS)
       for (int idx = threadIdx.x; idx < WG_ROWS * (CIN / 8); idx += S::THREADS) {
         const int slot = idx / (CIN / 8), q = idx % (CIN / 8);
         const int v = cb + sub + slot - 1; /* the cell whose (dz, dy) neighbour the slot holds */
-        const unsigned row = (unsigned)v / (unsigned)n;
-        const int i = (int)(row / (unsigned)n) + dz, j = (int)(row % (unsigned)n) + dy;
+        const unsigned row = by_n((unsigned)v), plane = by_n(row);
+        const int i = (int)plane + dz, j = (int)(row - plane * (unsigned)n) + dy;
         const bool ok = v >= 0 && v < n3 && i >= 0 && i < n && j >= 0 && j < n;
         const int src = ok ? v + (dz * n + dy) * n : 0;
         wg_copy(sx + (slot * S::XS + q * 8) * 2, Xs + (size_t)src * CIN + q * 8, ok);
@@ -273,7 +291,7 @@ __global__ void __launch_bounds__(WgShape<CIN, COUT>::THREADS)
         wg_copy(sz + (r * S::ZS + q * 8) * 2, Zs + (size_t)(ok ? sub + r : 0) * COUT + q * 8, ok);
       }
       if (threadIdx.x < WG_SUB) {
-        const int r = threadIdx.x, k = (cb + sub + r) % n;
+        const int r = threadIdx.x, v = cb + sub + r, k = v - (int)by_n((unsigned)v) * n;
         const int f = (k > 0 ? 1 : 0) | 2 | (k < n - 1 ? 4 : 0);
         flags[st * WG_SUB + r] = (unsigned char)(sub + r < chunk_cells ? f : 0);
       }
@@ -1191,8 +1209,8 @@ int wgrad(FlipUNet *u, int l, int n, int batch, const bf16 *X, const bf16 *dZ) {
   const int ch = (int)((V + cps - 1) / cps);
   const size_t chunks = (size_t)cps * batch;
   with_wgrad(cin, cout, [&](auto kern, int threads, int smem) {
-    kern<<<dim3((unsigned)chunks, 9), threads, smem, u->stream>>>(n, cps, ch, X, dZ, u->part,
-                                                                  u->part_b);
+    kern<<<dim3((unsigned)chunks, 9), threads, smem, u->stream>>>(n, div_by(n), cps, ch, X, dZ,
+                                                                  u->part, u->part_b);
   });
   const int wc = 27 * cin * cout;
   k_wgrad_reduce<<<(wc + cout + EBLK - 1) / EBLK, EBLK, 0, u->stream>>>(
