@@ -398,21 +398,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   if (failed && threadIdx.x == 0) atomicExch(err, 1);
 }
 
-/* W[tap][ci][co] FP32 -> per stage (di, chunk c) and tap t9 = dj*3 + dk a
- * block of cout*32 bytes: two K-halves of cout/8 core matrices (8 output
- * channels x 8 input channels, 16-byte rows). */
-__global__ void k_conv_tc_pack(int cin, int cout, const float *__restrict__ W,
-                               bf16 *__restrict__ out) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= 27 * cin * cout) return;
-  const int co = idx % cout, ci = (idx / cout) % cin, tap = idx / (cout * cin);
-  const int di = tap / 9, t9 = tap % 9;
-  const int c = ci / 16, kk = ci % 16, h = kk / 8, col = kk % 8, g = co / 8, r = co % 8;
-  const size_t byte = (size_t)((di * (cin / 16) + c) * 9 + t9) * cout * 32 +
-                      (size_t)(h * (cout / 8) + g) * 128 + r * 16 + col * 2;
-  out[byte / 2] = __float2bfloat16(W[idx]);
-}
-
 /* R_req / S_req > 0 ask for that many lines per unit / pipeline stages
  * (false if they do not fit); 0 takes the default */
 bool tc_plan(int n, int cin, int cout, int batch, TcShape &sh, size_t &smem, int R_req = 0,
@@ -494,12 +479,6 @@ bool conv_tc_supported(int n, int cin, int cout) {
   TcShape sh;
   size_t smem;
   return tc_plan(n, cin, cout, 1, sh, smem);
-}
-
-cudaError_t conv_tc_pack(cudaStream_t st, int cin, int cout, const float *W, bf16 *out) {
-  const int total = 27 * cin * cout;
-  k_conv_tc_pack<<<(total + 255) / 256, 256, 0, st>>>(cin, cout, W, out);
-  return cudaGetLastError();
 }
 
 int conv_tc_init_device() {

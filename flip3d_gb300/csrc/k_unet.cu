@@ -755,9 +755,23 @@ __global__ void k_prolong(int nc_, int f, int batch, const float *__restrict__ O
   Of[idx] = acc;
 }
 
-/* BF16 fragments of W (fwd) and of the flipped, transposed W (bwd-data). */
-__global__ void k_pack(int cin, int cout, const float *__restrict__ W, uint2 *__restrict__ ffwd,
-                       uint2 *__restrict__ fbwd) {
+/* Every layer's weights in the operand layouts, one launch for the network
+ * (blockIdx.y: the layer): BF16 fragments of W (f) and of the flipped, transposed
+ * W (b: backward-data) for mma.sync and, where t is not null, the tcgen05
+ * operand. A launch or two a layer took 84 us of a training step of 1.95 ms. */
+struct PackLayers {
+  struct {
+    int cin, cout;
+    const float *W;
+    uint2 *f, *b;
+    bf16 *t;
+  } l[NCONV];
+};
+__global__ void k_pack(const __grid_constant__ PackLayers layers) {
+  const int cin = layers.l[blockIdx.y].cin, cout = layers.l[blockIdx.y].cout;
+  const float *__restrict__ W = layers.l[blockIdx.y].W;
+  uint2 *__restrict__ ffwd = layers.l[blockIdx.y].f, *__restrict__ fbwd = layers.l[blockIdx.y].b;
+  bf16 *__restrict__ ftc = layers.l[blockIdx.y].t;
   const int nfw = 27 * (cin / 16) * (cout / 8) * 32;
   const int nbw = 27 * (cout / 16) * (cin / 8) * 32;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -773,7 +787,7 @@ __global__ void k_pack(int cin, int cout, const float *__restrict__ W, uint2 *__
     const int co = nt * 8 + g, ci = c * 16 + 2 * t;
     auto w = [&](int ci_) { return W[((size_t)tap * cin + ci_) * cout + co]; };
     ffwd[idx] = make_uint2(pack2(w(ci), w(ci + 1)), pack2(w(ci + 8), w(ci + 9)));
-  } else if (fbwd && idx < nfw + nbw) {
+  } else if (idx < nfw + nbw) {
     const int j = idx - nfw;
     const int lane = j % 32, rest = j / 32;
     /* convolution with Cin' = cout, Cout' = cin, tap' = 26 - tap */
@@ -784,6 +798,9 @@ __global__ void k_pack(int cin, int cout, const float *__restrict__ W, uint2 *__
     const int ci = nt * 8 + g, co = c * 16 + 2 * t;
     auto w = [&](int co_) { return W[((size_t)tap * cin + ci) * cout + co_]; };
     fbwd[j] = make_uint2(pack2(w(co), w(co + 1)), pack2(w(co + 8), w(co + 9)));
+  } else if (ftc && idx < nfw + nbw + 27 * cin * cout) {
+    const int e = idx - nfw - nbw;
+    ftc[conv_tc_weight(cin, cout, e)] = __float2bfloat16(W[e]);
   }
 }
 
@@ -1110,13 +1127,15 @@ int ensure_workspace(FlipUNet *u, int n, int batch) {
 
 int refresh_frags(FlipUNet *u) {
   if (u->frags_fresh) return FLIPGPU_OK;
+  PackLayers p;
+  int most = 0;
   for (int l = 0; l < NCONV; l++) {
-    const int cin = kConv[l].cin, cout = kConv[l].cout;
-    const int nf = 27 * (cin / 16) * (cout / 8) * 32, nb = 27 * (cout / 16) * (cin / 8) * 32;
-    k_pack<<<(nf + nb + EBLK - 1) / EBLK, EBLK, 0, u->stream>>>(cin, cout, u->P + u->woff[l],
-                                                               u->ffrag[l], u->bfrag[l]);
-    if (u->tc) UCK(conv_tc_pack(u->stream, cin, cout, u->P + u->woff[l], u->tcw[l]));
+    const int cin = kConv[l].cin, cout = kConv[l].cout, weights = 27 * cin * cout;
+    p.l[l] = {cin, cout, u->P + u->woff[l], u->ffrag[l], u->bfrag[l], u->tc ? u->tcw[l] : nullptr};
+    /* four weights a fragment element, twice, and one an operand element */
+    most = std::max(most, weights / 2 + (u->tc ? weights : 0));
   }
+  k_pack<<<dim3((most + EBLK - 1) / EBLK, NCONV), EBLK, 0, u->stream>>>(p);
   UCK(cudaGetLastError());
   u->frags_fresh = true;
   return FLIPGPU_OK;
