@@ -462,7 +462,7 @@ int flipgpu_create(const FlipGpuParams *p, FlipGpu **out) {
       return r;
     }
   }
-  if (particles_init_device() != 0) {
+  if (particles_init_device(h) != 0) {
     free_all(h);
     cudaStreamDestroy(h->own_stream);
     delete h;
@@ -1351,6 +1351,12 @@ int flipgpu_get_ic_tag_counter(FlipGpu *h, unsigned *value) {
   if (r != FLIPGPU_OK) return fail(h, r, "get_ic_tag_counter: wavefront buffers");
   CK(h, cudaMemcpyAsync(value, h->ic_ctr, sizeof *value, cudaMemcpyDeviceToHost, h->stream));
   CK(h, cudaStreamSynchronize(h->stream));
+  return FLIPGPU_OK;
+}
+
+int flipgpu_set_reposition_wait(FlipGpu *h, double seconds) {
+  if (!h || !(seconds >= 0.0 && seconds <= 60.0)) return FLIPGPU_EINVAL;
+  h->repo_wait_ns = (unsigned long long)(seconds * 1e9);
   return FLIPGPU_OK;
 }
 

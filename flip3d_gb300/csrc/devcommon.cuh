@@ -143,16 +143,19 @@ template <int BLOCK> __device__ __forceinline__ FF block_sum_ff(FF v) {
  * (zeroed before it), so the epoch-th barrier is complete when it reaches
  * epoch x gridDim.x. Thread 0 arrives with an acquire-release add after the
  * block's __syncthreads (the last block to arrive reads no more) and polls
- * with acquire loads: two L2 round trips, no reset and no generation word. The wait gives up after 2 s of %globaltimer,
- * flags FLIPGPU_ETIMEOUT and returns false in that block (the others give up
- * at their next barrier). */
+ * with acquire loads: two L2 round trips, no reset and no generation word. The
+ * wait gives up after limit_ns of %globaltimer (0: at once), sets *expired and
+ * returns false in that block (the others give up at their next barrier). */
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
 
-__device__ __forceinline__ bool count_barrier(unsigned *bar, unsigned &epoch, int *iflags) {
+constexpr unsigned long long BARRIER_NS = 2000000000ull;
+
+__device__ __forceinline__ bool count_barrier_for(unsigned *bar, unsigned &epoch, int *expired,
+                                                  unsigned long long limit_ns) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -164,13 +167,14 @@ __device__ __forceinline__ bool count_barrier(unsigned *bar, unsigned &epoch, in
     bool good = true;
     unsigned long long t0 = 0;
     unsigned spins = 0;
+    const unsigned mask = limit_ns < BARRIER_NS ? 0u : 1023u; /* polls between looks at the time */
     while ((int)(v - target) < 0) {
-      if ((++spins & 1023u) == 0) {
+      if ((++spins & mask) == 0) {
         const unsigned long long t = global_ns();
-        if (t0 == 0) {
+        if (t0 == 0 && limit_ns != 0) {
           t0 = t;
-        } else if (t - t0 > 2000000000ull) {
-          atomicExch(iflags + IF_TIMEOUT, 1);
+        } else if (t - t0 > limit_ns) {
+          atomicExch(expired, 1);
           good = false;
           break;
         }
@@ -181,6 +185,11 @@ __device__ __forceinline__ bool count_barrier(unsigned *bar, unsigned &epoch, in
   }
   __syncthreads();
   return ok != 0;
+}
+
+/* the solvers' barrier: an expired wait is the solve's FLIPGPU_ETIMEOUT */
+__device__ __forceinline__ bool count_barrier(unsigned *bar, unsigned &epoch, int *iflags) {
+  return count_barrier_for(bar, epoch, iflags + IF_TIMEOUT, BARRIER_NS);
 }
 
 __device__ __forceinline__ double ff_to_double(FF v) { return (double)v.hi + (double)v.lo; }

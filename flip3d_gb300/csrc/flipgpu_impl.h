@@ -169,6 +169,7 @@ struct FlipGpu {
   uint32_t *repo_cnt, *repo_start, *repo_list; /* shuffle steps listed by position */
   float4 *repo_res, *repo_old; /* per stuck particle: resampled / previous velocity */
   uint8_t *repo_state;       /* per stuck particle: resample round state */
+  unsigned long long repo_wait_ns; /* limit of a wait in k_repo_resample */
   size_t scan_cap;
 
   float *stage;       /* AoS staging for downloads */
@@ -236,7 +237,9 @@ enum {
   IF_NAN,
   IF_TIMEOUT,
   IF_REPO_LEFT,  /* reposition: stuck particles not yet resampled */
-  IF_REPO_BAR,   /* ... and the barrier of the kernel that resamples them */
+  IF_REPO_BAR,   /* the barrier of the kernel that resamples them, */
+  IF_REPO_TICKET,  /* its blocks that have left the rounds, */
+  IF_REPO_EXPIRED, /* and whether one left because a wait expired */
   IF_IR_DONE,    /* refinement: 0 running, 1 converged, 2 non-finite, 3 no
                     convergence, 4 zero right-hand side (x = 0) */
   IF_IR_ITERS,   /* refinement: inner CG iterations of all passes */
@@ -298,7 +301,7 @@ int mg_alloc(FlipGpu *h);  /* MG preconditioner buffers (idempotent) */
 void mg_free(FlipGpu *h);
 int ic_alloc(FlipGpu *h);
 void ic_free(FlipGpu *h);
-int particles_init_device();
+int particles_init_device(FlipGpu *h);
 
 /* device-wide exclusive scan of n uint32 (in may equal out) */
 cudaError_t scan_exclusive(FlipGpu *h, const uint32_t *in, uint32_t *out,

@@ -930,14 +930,20 @@ enum { RP_PENDING = 0, RP_DONE = 1, RP_READY = 2 };
  * rounds. Whatever is PENDING after the rounds runs in increasing q on one
  * warp: every earlier stuck particle is final by then. Nearly always round 0
  * leaves nothing, and the rest is two grid barriers; as 34 launches, one
- * particle a thread, the chain took 0.25 ms at n = 24. */
+ * particle a thread, the chain took 0.25 ms at n = 24.
+ *
+ * A block that waits longer than wait_ns leaves the rounds, and so do the others
+ * at their next barrier. No result depends on that: round 0 is whole by then, a
+ * READY value holds for every order of the others, and the last block to leave
+ * commits what is READY and then runs what is PENDING. */
 __global__ void __launch_bounds__(BLK)
 k_repo_resample(SimConst c, int *__restrict__ flags, const uint32_t *__restrict__ stuck_idx,
                 const uint32_t *__restrict__ cs, const uint32_t *__restrict__ perm,
                 const float4 *__restrict__ spos, const uint8_t *__restrict__ stuck,
                 const uint32_t *__restrict__ rank, const float *__restrict__ px,
                 const float *__restrict__ py, const float *__restrict__ pz, float *vx, float *vy,
-                float *vz, float4 *res, float4 *old, volatile uint8_t *state) {
+                float *vz, float4 *res, float4 *old, volatile uint8_t *state,
+                unsigned long long wait_ns) {
   const int m = flags[IF_NSTUCK], w = flags[IF_NWATER];
   if (w == 0 || m == 0) return;
   volatile int *left = flags + IF_REPO_LEFT;
@@ -946,6 +952,17 @@ k_repo_resample(SimConst c, int *__restrict__ flags, const uint32_t *__restrict_
   const int gw = blockIdx.x * (BLK / 32) + (threadIdx.x >> 5);
   auto at = [&](uint32_t p) { return make_float3(px[p], py[p], pz[p]); };
   auto now = [&](uint32_t o) { return make_float3(vx[o], vy[o], vz[o]); };
+  auto barrier = [&]() {
+    return count_barrier_for(bar, epoch, flags + IF_REPO_EXPIRED, wait_ns);
+  };
+  auto commit = [&](int q) {
+    const float4 r = res[q];
+    const uint32_t p = stuck_idx[q];
+    vx[p] = r.x;
+    vy[p] = r.y;
+    vz[p] = r.z;
+    state[q] = RP_DONE;
+  };
   for (int round = 0; round <= REPO_ROUNDS; round++) {
     for (int q = gw; q < m; q += warps) {
       if (round > 0 && state[q] != RP_PENDING) continue;
@@ -973,22 +990,33 @@ k_repo_resample(SimConst c, int *__restrict__ flags, const uint32_t *__restrict_
         if (round == 0 || !wait) state[q] = wait ? RP_PENDING : RP_READY;
       }
     }
-    if (!count_barrier(bar, epoch, flags)) return;
+    if (!barrier()) break;
     for (int q = blockIdx.x * BLK + threadIdx.x; q < m; q += gridDim.x * BLK) {
       if (state[q] != RP_READY) continue;
-      const float4 r = res[q];
-      const uint32_t p = stuck_idx[q];
-      vx[p] = r.x;
-      vy[p] = r.y;
-      vz[p] = r.z;
-      state[q] = RP_DONE;
+      commit(q);
       if (round > 0) atomicSub((int *)left, 1);
     }
-    if (round == 0 && *left == 0) return; /* nothing adds to it after the barrier */
-    if (!count_barrier(bar, epoch, flags)) return;
-    if (*left == 0) return;
+    if (round == 0 && *left == 0) break; /* nothing adds to it after the barrier */
+    if (!barrier()) break;
+    if (*left == 0) break;
   }
-  if (gw != 0) return;
+  __shared__ int last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(flags + IF_REPO_TICKET, 1) == (int)gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  if (*(volatile int *)(flags + IF_REPO_EXPIRED)) {
+    for (int q = threadIdx.x; q < m; q += BLK)
+      if (state[q] == RP_READY) commit(q);
+    __syncthreads();
+  } else if (*left == 0) {
+    return;
+  }
+  if (threadIdx.x >= 32) return;
   for (int q = 0; q < m; q++) {
     if (state[q] == RP_DONE) continue;
     const uint32_t p = stuck_idx[q];
@@ -1671,8 +1699,8 @@ cudaError_t launch_reposition(FlipGpu *h, int *stuck_host, bool in_step) {
   /* sorter::sort (src/flip3D.cpp:443), shared with the corrector's sort. */
   if ((e = launch_sort(h, 0, in_step ? 0 : PL_ALL)) != cudaSuccess) return e;
   /* corrector::resample of each stuck particle in order (src/flip3D.cpp:445-450) */
-  static_assert(IF_REPO_BAR == IF_REPO_LEFT + 1, "cleared together");
-  if ((e = cudaMemsetAsync(h->iflags + IF_REPO_LEFT, 0, 2 * sizeof(int), h->stream)) !=
+  static_assert(IF_REPO_EXPIRED == IF_REPO_LEFT + 3, "cleared together");
+  if ((e = cudaMemsetAsync(h->iflags + IF_REPO_LEFT, 0, 4 * sizeof(int), h->stream)) !=
       cudaSuccess)
     return e;
   {
@@ -1681,7 +1709,7 @@ cudaError_t launch_reposition(FlipGpu *h, int *stuck_host, bool in_step) {
     uint8_t *state = h->repo_state;
     void *args[] = {&c,     &flags, &h->stuck_idx, &h->cell_start, &h->perm, &h->spos,
                     &h->flag, &h->scan_a, &h->px, &h->py, &h->pz, &h->vx, &h->vy, &h->vz,
-                    &res,   &old,   &state};
+                    &res,   &old,   &state, &h->repo_wait_ns};
     /* a warp for about every 512 particles, at most two blocks an SM */
     const unsigned want = grid_for(h->np, 512 * (BLK / 32));
     const unsigned g = want < 2 * 152 ? want : 2 * 152;
@@ -1753,4 +1781,7 @@ cudaError_t launch_correct(FlipGpu *h) {
   return cudaGetLastError();
 }
 
-int particles_init_device() { return 0; }
+int particles_init_device(FlipGpu *h) {
+  h->repo_wait_ns = BARRIER_NS;
+  return 0;
+}

@@ -121,6 +121,7 @@ SIGNATURES = {
     "flipgpu_set_profiling": (C.c_int, [C.c_void_p, C.c_int]),
     "flipgpu_set_ic_tag_counter": (C.c_int, [C.c_void_p, C.c_uint]),
     "flipgpu_get_ic_tag_counter": (C.c_int, [C.c_void_p, C.POINTER(C.c_uint)]),
+    "flipgpu_set_reposition_wait": (C.c_int, [C.c_void_p, C.c_double]),
     "flipgpu_get_profile": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int]),
     "flipgpu_get_kernel_profile": (C.c_int, [C.c_void_p, C.c_char_p, C.c_int]),
     "flipgpu_sort_cells_noalloc": (C.c_int, [C.c_int, C.c_int, C.c_void_p, C.c_void_p,
@@ -482,6 +483,11 @@ class Simulation:
         out = C.c_uint(0)
         self._ck(self.lib.flipgpu_get_ic_tag_counter(self.h, C.byref(out)), "get_ic_tag_counter")
         return out.value
+
+    def reposition_wait(self, seconds):
+        """Limit of a wait in the reposition's resample (a testing aid)."""
+        self._ck(self.lib.flipgpu_set_reposition_wait(self.h, float(seconds)),
+                 "set_reposition_wait")
 
     def set_profiling(self, on=True):
         self._ck(self.lib.flipgpu_set_profiling(self.h, int(on)), "set_profiling")

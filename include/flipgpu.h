@@ -416,6 +416,11 @@ int flipgpu_set_ic_tag_counter(FlipGpu *h, unsigned value);
 /* its current value (synchronises) */
 int flipgpu_get_ic_tag_counter(FlipGpu *h, unsigned *value);
 
+/* Testing aid (no reference counterpart): how long a block of the reposition's
+ * resample waits for the others before it leaves the rest to the last one, in
+ * seconds (2 by default; 0: not at all). The results do not depend on it. */
+int flipgpu_set_reposition_wait(FlipGpu *h, double seconds);
+
 /* Cell sort that allocates no device memory. It has no counterpart in the
  * reference. It is for callers that may not allocate on the GPU, such as a
  * plugin inside a host application that owns all device memory, or a frame
