@@ -1360,6 +1360,12 @@ int flipgpu_set_reposition_wait(FlipGpu *h, double seconds) {
   return FLIPGPU_OK;
 }
 
+int flipgpu_set_reposition_blocks(FlipGpu *h, int blocks) {
+  if (!h || blocks < 0) return FLIPGPU_EINVAL;
+  h->repo_blocks = blocks;
+  return FLIPGPU_OK;
+}
+
 int flipgpu_get_profile(FlipGpu *h, double *ms, int64_t *calls, int max) {
   if (!h || max < 0) return FLIPGPU_EINVAL;
   for (int i = 0; i < FLIPGPU_NSTAGES && i < max; i++) {

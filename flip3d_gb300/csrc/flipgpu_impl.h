@@ -170,6 +170,8 @@ struct FlipGpu {
   float4 *repo_res, *repo_old; /* per stuck particle: resampled / previous velocity */
   uint8_t *repo_state;       /* per stuck particle: resample round state */
   unsigned long long repo_wait_ns; /* limit of a wait in k_repo_resample */
+  int repo_capacity;         /* its co-resident blocks (1: an ordinary launch) */
+  int repo_blocks;           /* cap on them (0: none) */
   size_t scan_cap;
 
   float *stage;       /* AoS staging for downloads */

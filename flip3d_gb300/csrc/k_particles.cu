@@ -15,6 +15,7 @@
  * evaluates the same formulas in native FP32 with fused multiply-adds and
  * the fast division intrinsic (FLIPGPU_ARITH_FAST).
  */
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -1710,11 +1711,14 @@ cudaError_t launch_reposition(FlipGpu *h, int *stuck_host, bool in_step) {
     void *args[] = {&c,     &flags, &h->stuck_idx, &h->cell_start, &h->perm, &h->spos,
                     &h->flag, &h->scan_a, &h->px, &h->py, &h->pz, &h->vx, &h->vy, &h->vz,
                     &res,   &old,   &state, &h->repo_wait_ns};
-    /* a warp for about every 512 particles, at most two blocks an SM */
-    const unsigned want = grid_for(h->np, 512 * (BLK / 32));
-    const unsigned g = want < 2 * 152 ? want : 2 * 152;
-    e = cudaLaunchCooperativeKernel((const void *)k_repo_resample, dim3(g), dim3(BLK), args, 0,
-                                    h->stream);
+    /* a warp for about every 512 particles, as far as the blocks fit on the device;
+     * a single block waits for nobody and needs no cooperative launch */
+    unsigned g = grid_for(h->np, 512 * (BLK / 32));
+    g = std::min(g, (unsigned)h->repo_capacity);
+    if (h->repo_blocks > 0) g = std::min(g, (unsigned)h->repo_blocks);
+    const void *kernel = (const void *)k_repo_resample;
+    e = g > 1 ? cudaLaunchCooperativeKernel(kernel, dim3(g), dim3(BLK), args, 0, h->stream)
+              : cudaLaunchKernel(kernel, dim3(1), dim3(BLK), args, 0, h->stream);
     FG_LAUNCHED(h, 1);
     if (e != cudaSuccess) return e;
   }
@@ -1782,6 +1786,14 @@ cudaError_t launch_correct(FlipGpu *h) {
 }
 
 int particles_init_device(FlipGpu *h) {
+  int dev = 0, sms = 0, coop = 0, per_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_repo_resample, BLK, 0) !=
+          cudaSuccess)
+    return -1;
   h->repo_wait_ns = BARRIER_NS;
+  h->repo_capacity = coop && per_sm > 0 ? sms * std::min(per_sm, 2) : 1;
   return 0;
 }

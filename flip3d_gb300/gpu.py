@@ -122,6 +122,7 @@ SIGNATURES = {
     "flipgpu_set_ic_tag_counter": (C.c_int, [C.c_void_p, C.c_uint]),
     "flipgpu_get_ic_tag_counter": (C.c_int, [C.c_void_p, C.POINTER(C.c_uint)]),
     "flipgpu_set_reposition_wait": (C.c_int, [C.c_void_p, C.c_double]),
+    "flipgpu_set_reposition_blocks": (C.c_int, [C.c_void_p, C.c_int]),
     "flipgpu_get_profile": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int]),
     "flipgpu_get_kernel_profile": (C.c_int, [C.c_void_p, C.c_char_p, C.c_int]),
     "flipgpu_sort_cells_noalloc": (C.c_int, [C.c_int, C.c_int, C.c_void_p, C.c_void_p,
@@ -488,6 +489,11 @@ class Simulation:
         """Limit of a wait in the reposition's resample (a testing aid)."""
         self._ck(self.lib.flipgpu_set_reposition_wait(self.h, float(seconds)),
                  "set_reposition_wait")
+
+    def reposition_blocks(self, blocks):
+        """Cap on the blocks of the reposition's resample (a testing aid; 0: none)."""
+        self._ck(self.lib.flipgpu_set_reposition_blocks(self.h, int(blocks)),
+                 "set_reposition_blocks")
 
     def set_profiling(self, on=True):
         self._ck(self.lib.flipgpu_set_profiling(self.h, int(on)), "set_profiling")

@@ -420,6 +420,10 @@ int flipgpu_get_ic_tag_counter(FlipGpu *h, unsigned *value);
  * resample waits for the others before it leaves the rest to the last one, in
  * seconds (2 by default; 0: not at all). The results do not depend on it. */
 int flipgpu_set_reposition_wait(FlipGpu *h, double seconds);
+/* Testing aid: at most this many blocks run it (0: as many as the device holds
+ * at once). One block is launched as on a device without cooperative launches.
+ * The results do not depend on it. */
+int flipgpu_set_reposition_blocks(FlipGpu *h, int blocks);
 
 /* Cell sort that allocates no device memory. It has no counterpart in the
  * reference. It is for callers that may not allocate on the GPU, such as a
