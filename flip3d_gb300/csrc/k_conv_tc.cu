@@ -33,7 +33,11 @@
  * Bound on 128-cell segments: the copies' 16-byte rows (about 0.6 a cycle), R + 2
  * lines for R, so the time follows (R + 2) / R: 16 to 16 channels at n = 128 take
  * 137, 103 and 90 us at R = 2, 4 and 8 (60 would be the tensor core's); R = 16
- * leaves no room for a third stage.
+ * leaves no room for a third stage. Levels of 112 and 120 cells take the same eight
+ * tiles, across line ends (R = 8; 107, 82 and 72 us at n = 112, 121, 93 and 80 at
+ * n = 120): the last one reads up to 1,824 bytes past a slab, into what follows it
+ * in shared memory (the other plane, the weights or the guard), for rows that are
+ * dropped. No other level below 128 cells has a power of two of lines with eight tiles.
  *
  * Pipeline, one CTA of 7 warps per SM, persistent over units, a ring of up
  * to 6 stages (di, 16-channel chunk):
@@ -74,7 +78,7 @@ namespace {
 constexpr int TC_THREADS = 224;
 constexpr int TC_STAGES = 6;
 constexpr unsigned TC_SPIN = 1u << 22;
-constexpr uint32_t TC_GUARD = 2304;       /* slots read past a slab by dropped rows */
+constexpr uint32_t TC_GUARD = 2304;       /* bytes read past a slab by dropped rows */
 constexpr size_t TC_SMEM_MAX = 225 * 1024;
 constexpr size_t TC_SMEM_MIN = 120 * 1024; /* keeps one CTA per SM: its TMEM is never contended */
 
@@ -398,7 +402,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   if (failed && threadIdx.x == 0) atomicExch(err, 1);
 }
 
-/* R_req / S_req > 0 ask for that many lines per unit / pipeline stages
+/* Tiles a unit: up to 5, or 8 (128-cell segments and levels of 112 and 120 cells);
+ * R_req / S_req > 0 ask for that many lines per unit / pipeline stages
  * (false if they do not fit); 0 takes the default */
 bool tc_plan(int n, int cin, int cout, int batch, TcShape &sh, size_t &smem, int R_req = 0,
              int S_req = 0) {
