@@ -149,7 +149,7 @@ struct FlipGpu {
                                FAST MG, cells in registers */
   int solve_blocks;   /* cap on the persistent solve's grid (0 = none; not the IC
                          wavefront), so that concurrent simulations' solves share the GPU */
-  int solve_capacity; /* co-resident grid of the last solve's kernel */
+  int solve_capacity; /* co-resident grid of the last solve's kernel (the one without a cap) */
   unsigned *ticket;   /* task ticket of the IC wavefront */
   /* IC(0)/MIC(0) line wavefront (k_pcg.cu ic_alloc) */
   int ic_njb, ic_tasks;              /* 32-j line blocks; tasks */

@@ -4311,9 +4311,11 @@ int run_solve(FlipGpu *h, FlipGpuSolveStats *st) {
     /* small grids: the cells in registers, as few to a thread as the blocks
      * allow */
     int reg_cells = 0;
+    bool reg_fits = false; /* without a cap */
     if (mode == FLIPGPU_SOLVE_REF ||
         (precond == FLIPGPU_PRECOND_JACOBI && kern == (const void *)k_cg<FLIPGPU_SOLVE_FAST>)) {
       int most = h->cg_grid[6];
+      reg_fits = nc <= (size_t)most * CGR_BLOCK * CGR_CELLS;
       if (h->solve_blocks > 0 && h->solve_blocks < most) most = h->solve_blocks;
       for (int e = 1; e <= CGR_CELLS && reg_cells == 0; e *= 2)
         if (nc <= (size_t)most * CGR_BLOCK * e) reg_cells = e;
@@ -4377,7 +4379,9 @@ int run_solve(FlipGpu *h, FlipGpuSolveStats *st) {
      * cells per thread): small grids keep short barriers and leave the rest
      * of the GPU to other simulations */
     if (precond != FLIPGPU_PRECOND_IC) {
-      h->solve_capacity = grid;
+      /* a cap is a share of the capacity: that of the kernel without a cap, so
+       * that it does not move with the cap */
+      h->solve_capacity = reg_fits ? h->cg_grid[6] : grid;
       const size_t per_block = (size_t)cg_block_of(kern) * (reg_cells > 0 ? reg_cells : 8);
       const size_t want = (nc + per_block - 1) / per_block;
       if (want < (size_t)grid) grid = want > 0 ? (int)want : 1;
