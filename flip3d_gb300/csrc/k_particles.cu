@@ -1004,9 +1004,12 @@ k_repo_resample(SimConst c, int *__restrict__ flags, const uint32_t *__restrict_
   __shared__ int last;
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(flags + IF_REPO_TICKET, 1) == (int)gridDim.x - 1;
-    __threadfence();
+    int ticket;
+    asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;"
+                 : "=r"(ticket)
+                 : "l"(flags + IF_REPO_TICKET)
+                 : "memory");
+    last = ticket == (int)gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return;
