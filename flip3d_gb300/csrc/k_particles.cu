@@ -1493,14 +1493,18 @@ static bool cell_gathers(const FlipGpu *h) {
   return !(e && strcmp(e, "particle") == 0);
 }
 
-/* The FAST gathers' block size, tuned per kernel and problem size (key: the
+/* The block size of the FAST gathers that have no better fixed one (the corrector,
+ * density below DENSITY_TILE_N and P2G from P2G_CELLS_N on; the tiles of
+ * k_density_tile and the small grids' k_p2g have one size), tuned per kernel and
+ * problem size (key: the
  * kernel, N and the power of two at or above its thread count) over 256
  * (the default, and the choice while a stream is being captured or an
  * asynchronous step runs), 128 and 512 threads. Every thread computes one
  * particle's or face cell's sums on its own, so the results do not depend
  * on the choice; each kernel only writes outputs that it does not read, so
  * the tuner's repeated launches leave the same state. FLIPGPU_GATHER_BLOCK
- * = 128, 256 or 512 in the environment (read at each launch) fixes it. */
+ * = 128, 256 or 512 in the environment (read at each launch) fixes it for these
+ * kernels; it chooses no kernel. */
 template <class L>
 static cudaError_t tuned_gather(FlipGpu *h, const char *kernel, size_t threads, L launch) {
   auto run = [&](int i) -> cudaError_t {
@@ -1532,13 +1536,18 @@ static cudaError_t tuned_gather(FlipGpu *h, const char *kernel, size_t threads, 
   return err;
 }
 
+/* From which grid the tile kernel pays (both give the same bits). us a call at n =
+ * 32, 40, 48, 56, 64, 72, 80, 96, 128:
+ *   pool, tile         46   63   65   90   97  117  143  216  456
+ *   pool, a particle   32   37   47   73   95  128  164  261  594
+ *   dam, tile          49   50   62   78   94  122  148  235  522
+ *   dam, a particle    33   38   52   92  100  143  188  316  723
+ * Its tiles are too few blocks below. */
 constexpr int DENSITY_TILE_N = 64;
 
 cudaError_t launch_density(FlipGpu *h) {
   if (h->np == 0) return cudaSuccess;
   SimConst c = make_const(h);
-  /* the tile kernel pays from n = 64 (85 against 98 us; at n = 48 its blocks are
-   * too few, 56 against 49); both give the same bits */
   if (cell_gathers(h) && h->n >= DENSITY_TILE_N) {
     ktime_begin(h, "k_density");
     k_density_tile<<<cell_tiles(h->n), CT_BLOCK, 0, h->stream>>>(c, h->cell_start, h->perm, h->spos,
@@ -1566,7 +1575,13 @@ cudaError_t launch_density(FlipGpu *h) {
  * Small grids leave SMs idle and wait for each candidate's loads in turn, so
  * they take more threads and overlap the loads; larger ones are bound by the
  * instructions issued. REF takes a face a thread at every size, and requests ahead
- * below P2G_AHEAD_N. */
+ * below P2G_AHEAD_N (us at n = 16, 24, 32, 40, 48, 52, 56, 60, 64, 72, 80, 96, 128):
+ *   pool, ahead   66   76   85  113  125  148  183  203  227  298  378  597  1379
+ *   pool, not     78   93   96  106  140  146  169  207  233  290  368  581  1315
+ *   dam, ahead    72   79   80   90  113  124  166  198  213  292  372  625  1466
+ *   dam, not      86   97   97  104  121  135  146  193  236  274  373  607  1389
+ * From n = 52 to 68 either is up to 14 % faster by the scene; below it nearly
+ * always pays, above it does not. */
 constexpr int P2G_CELLS_N = 40, P2G_AHEAD_N = 64;
 
 cudaError_t launch_p2g(FlipGpu *h, int enforce) {
@@ -1666,8 +1681,8 @@ cudaError_t launch_advect(FlipGpu *h) {
  * 1e-5 keeps clear of the FAST division's rounding. */
 static bool resample_is_identity(const SimConst &c) { return c.re_corr_hh <= 0.999e-5f; }
 
-/* Compute stuck and deep-water lists, place the stuck particles. The sort
- * and the ordered resample follow in launch_reposition_resample. */
+/* Stuck and deep-water lists, the stuck particles' new places, the sort, and
+ * their resample in order (k_repo_resample). */
 cudaError_t launch_reposition(FlipGpu *h, int *stuck_host, bool in_step) {
   SimConst c = make_const(h);
   cudaError_t e;

@@ -2096,7 +2096,7 @@ __device__ __forceinline__ void mg_cells_up(const MgArgs &mg, const MgBlockLevel
  * back to global memory). Block 0 is alone with these levels while the grid
  * waits, so their latency counts whole. Cell by cell, with flags, tests and
  * index divisions, they took 35 to 45 us of a V-cycle of two sweeps at n =
- * 128; on lists of cells 17 us. A level has at most 512 segments; the threads
+ * 128; as segments and cells 11 us. A level has at most 512 segments; the threads
  * past its last warp skip it, and its barriers count the others alone. Not
  * inlined: among k_cg_mg's own values its registers would be spilled. */
 __device__ __noinline__ void mg_block_levels(const MgArgs &mg) {

@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(CTHREADS, NB == 16 ? 4 : 2)
  * stages). One block per tap that staged synchronously, with the tiles dealt
  * to eight warps (two of which had work in the 16 x 16 layers), was bound by
  * the staging latency: the 14 layers of 16 systems of 32^3 cells took 7.33 ms
- * of a training step's 9.12 ms; with this 0.78 ms, and 0.66 ms with the copies'
+ * of a training step's 9.12 ms; with this 0.78 ms, and 0.63 ms with the copies'
  * divisions by n as multiplications (half of a 16 x 16 layer's instructions were the
  * index arithmetic of its copies). */
 __device__ __forceinline__ void wg_copy(uint32_t dst, const void *src, bool ok) {
