@@ -261,7 +261,7 @@ def roofline_note(kernel, traffic, nbytes):
     notes = []
     if kernel in GATHER_KERNELS:
         notes.append("a particle gather: bound by the L1 data pipe (one 16-byte neighbour "
-                     "load per particle pair, 85-91 % of its peak in ncu), not by HBM")
+                     "load per particle pair, 78-95 % of its peak in ncu), not by HBM")
     if traffic is not None and nbytes:
         if traffic < 0.2 * nbytes:
             notes.append(f"ncu DRAM traffic {traffic} B per call against {nbytes} algorithmic "

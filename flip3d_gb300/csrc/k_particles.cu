@@ -1573,8 +1573,8 @@ cudaError_t launch_density(FlipGpu *h) {
  *   a face a thread, next candidate requested ahead    35   42   47   61   80  141  837
  *   a face cell a thread                               44   54   54   58   70   99  456
  * Small grids leave SMs idle and wait for each candidate's loads in turn, so
- * they take more threads and overlap the loads; larger ones are bound by the
- * instructions issued. REF takes a face a thread at every size, and requests ahead
+ * they take more threads and overlap the loads; larger ones are bound by the L1
+ * data pipe and the instructions issued. REF takes a face a thread at every size, and requests ahead
  * below P2G_AHEAD_N (us at n = 16, 24, 32, 40, 48, 52, 56, 60, 64, 72, 80, 96, 128):
  *   pool, ahead   66   76   85  113  125  148  183  203  227  298  378  597  1379
  *   pool, not     78   93   96  106  140  146  169  207  233  290  368  581  1315
